@@ -17,6 +17,30 @@ def _pack(seqs):
     return np.concatenate(seqs).astype(np.uint8), offsets, lengths
 
 
+@pytest.mark.parametrize("s", [1, 2, 31, 32, 33, 64, 100, 128, 129, 256, 500, 1000, 1861, 1862, 4096])
+@pytest.mark.parametrize("k,alphabet", [(5, 20), (3, 20), (7, 20), (11, 4), (32, 4)])
+def test_sketch_sizes(ck, s, k, alphabet):
+    """Sequences with as many k-mers as the threshold form's buffers hold, one
+    more and one fewer; repeats that leave no threshold between too few and
+    too many; codes outside the alphabet."""
+    rng = np.random.default_rng(s + k)
+    seqs = []
+    for c in (0, 1, s - 1, s, s + 1, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1025, 2047, 2048,
+              2049, 5000):
+        seqs.append(rng.integers(0, alphabet, max(0, c + k - 1)))
+    for n in (300, 3000, 6000):  # one value, two values, a few, and a repeat among others
+        seqs.append(np.zeros(n, np.int64))
+        seqs.append(rng.integers(0, 2, n))
+        seqs.append(np.tile(rng.integers(0, alphabet, 9), n // 9))
+        x = rng.integers(0, alphabet, n)
+        x[n // 4: n // 2] = 3
+        seqs.append(x)
+    seqs.append(rng.integers(0, 256, 2500))
+    flat, off, lens = _pack(seqs)
+    got = sketch_flat(flat, off, lens, k, s, alphabet)
+    assert np.array_equal(got, oracle.sketches(flat, off, lens, k, s, alphabet))
+
+
 @pytest.mark.parametrize("tables,bands,size", [(1, 1, 1), (40, 1, 8), (64, 2, 3), (200, 1, 128), (30, 3, 4)])
 def test_lsh_repeated_tables(ck, tables, bands, size):
     """Tables that read the same columns (most of them, here) add nothing; the
