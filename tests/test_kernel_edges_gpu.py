@@ -6,6 +6,7 @@ import pytest
 import oracle
 from clustkit_gb300 import synth
 from clustkit_gb300.lsh import band_parameters, lsh_candidates, lsh_candidates_device
+from clustkit_gb300.pairwise import batch_jaccard
 from clustkit_gb300.sketch import sketch_flat
 
 pytestmark = pytest.mark.gpu
@@ -39,6 +40,33 @@ def test_sketch_sizes(ck, s, k, alphabet):
     flat, off, lens = _pack(seqs)
     got = sketch_flat(flat, off, lens, k, s, alphabet)
     assert np.array_equal(got, oracle.sketches(flat, off, lens, k, s, alphabet))
+
+
+@pytest.mark.parametrize("s", [1, 2, 31, 32, 33, 63, 65, 100, 127, 128, 129, 255, 256, 257])
+@pytest.mark.parametrize("m", [1, 31, 33, 2431, 2433, 80000])
+def test_jaccard_runs(ck, s, m):
+    """Pair lists of every run length, sorted by the first sequence and not,
+    over sketches with repeats, padding and values that differ in the high
+    bits alone (the bitmap reads the low ones)."""
+    rng = np.random.default_rng(s * 7 + m)
+    mx = np.uint64(np.iinfo(np.uint64).max)
+    rows = []
+    for r in range(120):
+        n = int(rng.integers(0, s + 1)) if r % 3 else s
+        hi = [4, 3 * s, 2 ** 40, 2 ** 63][r % 4]
+        x = rng.integers(0, hi, n).astype(np.uint64)
+        if r % 5 == 0:
+            x <<= np.uint64(20)
+        rows.append(np.concatenate([np.sort(x), np.full(s - n, mx, np.uint64)]))
+    sk = np.stack(rows)
+    sk[60:90] = np.sort(np.where(rng.random((30, s)) < 0.5, sk[:30], sk[60:90]), 1)
+    pairs = rng.integers(0, 120, size=(m, 2)).astype(np.int32)
+    if m % 2 == 0:
+        pairs = pairs[np.argsort(pairs[:, 0], kind="stable")]
+    sims, mask = batch_jaccard(pairs, sk, 0.25)
+    ref = oracle.jaccard(pairs, sk)
+    assert np.array_equal(sims, ref)
+    assert np.array_equal(mask, ref >= np.float32(0.25))
 
 
 @pytest.mark.parametrize("tables,bands,size", [(1, 1, 1), (40, 1, 8), (64, 2, 3), (200, 1, 128), (30, 3, 4)])
