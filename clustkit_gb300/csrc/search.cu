@@ -666,21 +666,50 @@ __global__ void cap_unpack_kernel(const uint64_t *__restrict__ keys, const int32
 // (nbr_list_kernel) lists the (query, 5-mer, score) triples in one pass;
 // stage 2 (nbr_walk_kernel) walks their posting lists.
 //
-// Stage 1 work items are (query position p, first two residues a0 a1), 400
-// per position.  A warp tests 32 items against clustkit's pruning bound (the
-// score so far plus the best remaining row scores must reach T); then, one
-// surviving item at a time, its lanes split the 400 (a2, a3) continuations
-// and each lane tries the 20 last residues, so no thread walks a heavy prefix
-// alone.  Hits go to the warp's shared-memory stage as 4-byte entries (value
-// | score << 22; 20^5 < 2^22, a score is at most 5 x 127); a full stage is
-// flushed to the list with one global reservation, as 8-byte entries
-// (query << 48 | score << 32 | value).  Which warp lists a triple first
-// varies from run to run; the walk's integer sums do not depend on the order.
-constexpr int32_t NB_PREFIX = 400;
+// Stage 1 splits a 5-mer's first four residues into two pairs.  For a query
+// position, a warp orders the 400 residue pairs (a0, a1) and the 400 pairs
+// (a2, a3) by score, descending (a counting sort: a pair's score has a few
+// dozen values).  The (a0 a1, a2 a3) combinations that can still reach the
+// threshold with the best last residue are then, for each score of the first
+// pair, a prefix of the second list: a rectangle whose cells go to the lanes
+// 32 at a time, so no lane tests a combination that clustkit's bound would
+// prune.  A cell's last residues are one AND: the residues that reach the
+// threshold (a table by query residue and score needed) and the indexed 5-mers
+// of those four residues (one bit each, kmer_valid_kernel: 640 KB, so L2 and
+// largely L1 hold it; the frequencies themselves are 12.8 MB).  Hits go to the
+// warp's shared-memory stage as 4-byte entries (value | score << 22;
+// 20^5 < 2^22, a score is at most 5 x 127); a full stage is flushed to the
+// list with one global reservation, as 8-byte entries (query << 48 |
+// score << 32 | value).  Which warp lists a triple first varies from run to
+// run; the walk's integer sums do not depend on the order.
+// 64 queries against 200,000 sequences: 8.1 -> 0.4 ms, the whole search call
+// 25.0 -> 17.3 (before, a warp tested all 400
+// continuations of every surviving pair, a lane up to 20 frequencies each).
+constexpr int32_t NB_PAIRS = 400;
 constexpr int NB_WARPS = 8;              // warps per block
 constexpr int32_t NB_STAGE = 1024;       // staged entries per warp (a round adds at most 32 x 20)
 constexpr uint32_t NB_SCORE_SHIFT = 22;
 constexpr int64_t NB_BLOCKS_PER_QUERY = 512;
+
+// Bit a of valid[u]: the 5-mer of the four residues u and last residue a has a
+// frequency in 1 .. freq_thresh.  A warp turns 640 frequencies into 20 ballots,
+// whose bits are then 32 words of 20.
+__global__ void kmer_valid_kernel(const int32_t *__restrict__ freqs, int32_t freq_thresh, int32_t n_words,
+                                  uint32_t *__restrict__ valid) {
+    const int lane = threadIdx.x & 31;
+    const int32_t base = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
+    if (base >= n_words) return;  // n_words = 20^4 is a multiple of 32
+    const int32_t bit = 20 * lane, first = bit >> 5;
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int r = 0; r < 20; ++r) {
+        const int32_t f = __ldg(freqs + (int64_t)base * 20 + r * 32 + lane);
+        const uint32_t bal = __ballot_sync(0xffffffffu, f != 0 && f <= freq_thresh);
+        if (r == first) lo = bal;
+        if (r == first + 1) hi = bal;
+    }
+    valid[base + lane] = __funnelshift_r(lo, hi, bit & 31) & 0xfffffu;
+}
 
 __device__ __forceinline__ void nbr_flush(const uint32_t *stage, int32_t fill, int32_t q, uint64_t *list,
                                           int64_t cap, unsigned long long *cursor, int lane) {
@@ -697,17 +726,63 @@ __device__ __forceinline__ void nbr_flush(const uint32_t *stage, int32_t fill, i
     }
 }
 
+// Shared memory of the listing: the matrix, the table of last residues (20
+// rows of `range` + 1 words, range = largest - smallest matrix entry) and per
+// warp the two ordered pair lists, their starts by score (2 range + 2 each)
+// and the stage.
+__host__ __device__ constexpr size_t nbr_warp_words(int32_t range) {
+    return (size_t)(NB_PAIRS / 2 + NB_PAIRS + 2 * (2 * range + 2) + NB_STAGE);
+}
+__host__ __device__ constexpr size_t nbr_smem(int32_t range) {
+    return (400 + 20 * (size_t)(range + 1) + NB_WARPS * nbr_warp_words(range)) * 4;
+}
+
+// One residue-pair list of a position, ordered by score: bin b of `start`
+// becomes the number of pairs with a score above 2 smin + b, and put(at, pair,
+// bin) is called once for each pair.
+template <class Put>
+__device__ __forceinline__ void nbr_order_pairs(const int32_t *Sa, const int32_t *Sb, int32_t smin, int32_t bins,
+                                                int32_t *start, int lane, Put put) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    for (int32_t b = lane; b < bins; b += 32) start[b] = 0;
+    __syncwarp();
+    for (int32_t t = lane; t < NB_PAIRS; t += 32) {
+        const int32_t a = t / 20;
+        atomicAdd(&start[Sa[a] + Sb[t - a * 20] - 2 * smin], 1);
+    }
+    __syncwarp();
+    int32_t above = 0;  // pairs in the bins already passed (higher scores)
+    for (int32_t top = bins - 1; top >= 0; top -= 32) {
+        const int32_t b = top - lane;
+        const int32_t n = b >= 0 ? start[b] : 0;
+        int32_t incl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t x = __shfl_up_sync(FULL, incl, d);
+            if (lane >= d) incl += x;
+        }
+        if (b >= 0) start[b] = above + incl - n;
+        above += __shfl_sync(FULL, incl, 31);
+    }
+    __syncwarp();
+    for (int32_t t = lane; t < NB_PAIRS; t += 32) {
+        const int32_t a = t / 20, b = Sa[a] + Sb[t - a * 20] - 2 * smin;
+        put(atomicAdd(&start[b], 1), t, b);  // leaves start[b] = pairs with a score of bin b or above
+    }
+    __syncwarp();
+}
+
 // Lists every (query, 5-mer, score) triple; *cursor (zeroed by the caller)
 // ends as the number of triples, of which the first `cap` are written.
 __global__ void __launch_bounds__(NB_WARPS * 32)
 nbr_list_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int64_t *__restrict__ qoff,
-                const int32_t *__restrict__ qlen, const int8_t *__restrict__ sub, int32_t T,
-                const int32_t *__restrict__ kmer_freqs, int32_t freq_thresh, uint64_t *__restrict__ list, int64_t cap,
+                const int32_t *__restrict__ qlen, const int8_t *__restrict__ sub, int32_t smin, int32_t range,
+                int32_t T, const uint32_t *__restrict__ valid, uint64_t *__restrict__ list, int64_t cap,
                 unsigned long long *__restrict__ cursor, int32_t *err) {
     constexpr uint32_t FULL = 0xffffffffu;
-    __shared__ int32_t S[400];
-    __shared__ int32_t mx[20];
-    __shared__ uint32_t stage_all[NB_WARPS][NB_STAGE];
+    extern __shared__ int32_t nb_smem[];
+    int32_t *S = nb_smem;
+    uint32_t *reach = (uint32_t *)(nb_smem + 400);  // [query residue][score needed - smin]: last residues that give it
     const int32_t q = blockIdx.y;
     const int32_t L = qlen[q];
     const int64_t o = qoff[q];
@@ -716,74 +791,64 @@ nbr_list_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int6
         if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(err, ERRBIT_SEQ_EXTENT);
         return;
     }
-    const int64_t work = (int64_t)(L >= 5 ? L - 4 : 0) * NB_PREFIX;
-    if ((int64_t)blockIdx.x * NB_WARPS * 32 >= work) return;  // a shorter query than the batch's longest
+    const int32_t npos = L >= 5 ? L - 4 : 0;
+    if ((int32_t)blockIdx.x * NB_WARPS >= npos) return;  // a shorter query than the batch's longest
     for (int i = threadIdx.x; i < 400; i += blockDim.x) S[i] = sub[i];
     __syncthreads();
-    if (threadIdx.x < 20) {
-        int32_t m = -1000;
-        for (int j = 0; j < 20; ++j) m = max(m, S[threadIdx.x * 20 + j]);
-        mx[threadIdx.x] = m;
+    for (int i = threadIdx.x; i < 20 * (range + 1); i += blockDim.x) {
+        const int32_t a = i / (range + 1), need = i - a * (range + 1) + smin;
+        uint32_t m = 0;
+        for (int b = 0; b < 20; ++b) m |= S[a * 20 + b] >= need ? 1u << b : 0u;
+        reach[i] = m;
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t *stage = stage_all[warp];
+    const int32_t bins = 2 * range + 1;
+    uint32_t *pairs2 = (uint32_t *)(nb_smem + 400 + 20 * (range + 1) + (size_t)warp * nbr_warp_words(range));
+    uint16_t *pairs1 = (uint16_t *)(pairs2 + NB_PAIRS);
+    int32_t *n1 = (int32_t *)(pairs2 + NB_PAIRS + NB_PAIRS / 2), *n2 = n1 + 2 * range + 2;
+    uint32_t *stage = (uint32_t *)(n2 + 2 * range + 2);
     const uint8_t *sq = qflat + o;
-    const int64_t step = (int64_t)gridDim.x * NB_WARPS * 32;
     int32_t fill = 0;  // warp-uniform
-    for (int64_t t0 = ((int64_t)blockIdx.x * NB_WARPS + warp) * 32; t0 < work; t0 += step) {
-        const int64_t t = t0 + lane;
-        bool live = false;
-        int32_t p = 0, s1 = 0, v1 = 0;
-        if (t < work) {
-            p = (int32_t)(t / NB_PREFIX);
-            const int32_t pre = (int32_t)(t - (int64_t)p * NB_PREFIX);
-            const int32_t a0 = pre / 20, a1 = pre - a0 * 20;
-            const int32_t q0 = sq[p], q1 = sq[p + 1], q2 = sq[p + 2], q3 = sq[p + 3], q4 = sq[p + 4];
-            if (q0 < 20 && q1 < 20 && q2 < 20 && q3 < 20 && q4 < 20) {
-                const int32_t m234 = mx[q2] + mx[q3] + mx[q4];
-                const int32_t s0 = S[q0 * 20 + a0];
-                s1 = s0 + S[q1 * 20 + a1];
-                live = s0 + mx[q1] + m234 >= T && s1 + m234 >= T;
-                v1 = a0 * 160000 + a1 * 8000;
-            }
-        }
-        uint32_t lm = __ballot_sync(FULL, live);
-        while (lm) {
-            const int src = __ffs(lm) - 1;
-            lm &= lm - 1;
-            const int32_t P = __shfl_sync(FULL, p, src);
-            const int32_t S1 = __shfl_sync(FULL, s1, src);
-            const int32_t V1 = __shfl_sync(FULL, v1, src);
-            const int32_t q2 = sq[P + 2], q3 = sq[P + 3], q4 = sq[P + 4];
-            const int32_t m4 = mx[q4], m34 = mx[q3] + m4;
-            const int32_t *S4 = S + q4 * 20;
-            for (int32_t c0 = 0; c0 < 400; c0 += 32) {
-                const int32_t c = c0 + lane;
+    for (int32_t p = blockIdx.x * NB_WARPS + warp; p < npos; p += gridDim.x * NB_WARPS) {
+        const int32_t q0 = sq[p], q1 = sq[p + 1], q2 = sq[p + 2], q3 = sq[p + 3], q4 = sq[p + 4];
+        if (q0 >= 20 || q1 >= 20 || q2 >= 20 || q3 >= 20 || q4 >= 20) continue;  // the same for the whole warp
+        __syncwarp();
+        nbr_order_pairs(S + q0 * 20, S + q1 * 20, smin, bins, n1, lane,
+                        [&](int32_t at, int32_t t, int32_t) { pairs1[at] = (uint16_t)t; });
+        nbr_order_pairs(S + q2 * 20, S + q3 * 20, smin, bins, n2, lane,
+                        [&](int32_t at, int32_t t, int32_t b) { pairs2[at] = (uint32_t)t | ((uint32_t)b << 16); });
+        int32_t m4 = range;  // the best last residue's score, less smin
+        while (m4 > 0 && reach[q4 * (range + 1) + m4] == 0) --m4;
+        for (int32_t b1 = bins - 1; b1 >= 0; --b1) {
+            // second pairs must have bin >= T - (their last residue's best) - first pair's score
+            const int32_t need = T - (m4 + smin) - (b1 + 2 * smin) - 2 * smin;
+            if (need >= bins) break;  // and so for every lower first pair
+            const int32_t i1 = b1 + 1 < bins ? n1[b1 + 1] : 0, c1 = n1[b1] - i1, c2 = n2[need > 0 ? need : 0];
+            if (c2 == 0) break;
+            const int32_t cells = c1 * c2;
+            // cell / c2 by a multiplication: exact, as cell * c2 <= 160,000 * 400 < 2^32
+            const uint32_t inv = (uint32_t)(0x100000000ull / (uint32_t)c2) + 1u;
+            for (int32_t k0 = 0; k0 < cells; k0 += 32) {
+                const int32_t k = k0 + lane;
                 uint32_t bits = 0;
-                int32_t s3 = 0, v3 = 0;
-                if (c < 400) {
-                    const int32_t a2 = c / 20, a3 = c - a2 * 20;
-                    const int32_t s2 = S1 + S[q2 * 20 + a2];
-                    s3 = s2 + S[q3 * 20 + a3];
-                    if (s2 + m34 >= T && s3 + m4 >= T) {
-                        v3 = V1 + a2 * 400 + a3 * 20;
-#pragma unroll
-                        for (int a4 = 0; a4 < 20; ++a4) {
-                            if (s3 + S4[a4] >= T) {
-                                const int32_t f = __ldg(kmer_freqs + v3 + a4);
-                                if (f != 0 && f <= freq_thresh) bits |= 1u << a4;
-                            }
-                        }
-                    }
+                int32_t s4 = 0, v4 = 0;
+                if (k < cells) {
+                    const int32_t row = c2 == 1 ? k : (int32_t)__umulhi((uint32_t)k, inv);
+                    const uint32_t x = pairs2[k - row * c2];
+                    s4 = b1 + (int32_t)(x >> 16) + 4 * smin;
+                    v4 = (int32_t)pairs1[i1 + row] * NB_PAIRS + (int32_t)(x & 0xffffu);
+                    int32_t w = T - s4 - smin;
+                    w = w < 0 ? 0 : w;  // at most m4
+                    bits = reach[q4 * (range + 1) + w] & __ldg(valid + v4);
                 }
                 if (!__any_sync(FULL, bits != 0)) continue;
                 const int32_t n = __popc(bits);
                 int32_t incl = n;
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1) {
-                    const int32_t x = __shfl_up_sync(FULL, incl, d);
-                    if (lane >= d) incl += x;
+                    const int32_t y = __shfl_up_sync(FULL, incl, d);
+                    if (lane >= d) incl += y;
                 }
                 const int32_t tot = __shfl_sync(FULL, incl, 31);
                 if (fill + tot > NB_STAGE) {
@@ -796,7 +861,7 @@ nbr_list_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int6
                 while (bits) {
                     const int b = __ffs(bits) - 1;
                     bits &= bits - 1;
-                    stage[at++] = (uint32_t)(v3 + b) | ((uint32_t)(s3 + S4[b]) << NB_SCORE_SHIFT);
+                    stage[at++] = (uint32_t)(v4 * 20 + b) | ((uint32_t)(s4 + S[q4 * 20 + b]) << NB_SCORE_SHIFT);
                 }
                 fill += tot;
             }
@@ -1158,20 +1223,33 @@ static int32_t phase_a_impl(void *pv) {
             uint64_t *list = (uint64_t *)scratch(SLOT_SEARCH_TMP1, (size_t)std::max<int64_t>(cap, 1) * 8, &status);
             if (!list) return status;
             if (!bounded) cap = (int64_t)(scratch_capacity(SLOT_SEARCH_TMP1) / 8);
-            // one block per 256 items of the longest query, at most
+            // a block per 8 positions of the longest query, at most
             // NB_BLOCKS_PER_QUERY (longer queries loop; a graph captured for
-            // an arena-long query would otherwise launch ~10^5 empty blocks per
-            // query): blocks start in query order, so the list fills (and the
-            // walk later runs) about one query at a time -- the walk's
-            // count-row atomics then hit L2
-            const int64_t groups = ((int64_t)npos * NB_PREFIX + NB_WARPS * 32 - 1) / (NB_WARPS * 32);
+            // an arena-long query would otherwise launch mostly empty blocks):
+            // blocks start in query order, so the list fills (and the walk
+            // later runs) about one query at a time -- the walk's count-row
+            // atomics then hit L2
+            const int64_t groups = ((int64_t)npos + NB_WARPS - 1) / NB_WARPS;
             const dim3 grid((unsigned)std::min<int64_t>(groups, NB_BLOCKS_PER_QUERY), (unsigned)a.nq);
+            int32_t smin = a.sub_host[0], smax = a.sub_host[0];
+            for (int i = 1; i < 400; ++i) {
+                smin = std::min<int32_t>(smin, a.sub_host[i]);
+                smax = std::max<int32_t>(smax, a.sub_host[i]);
+            }
+            const int32_t range = smax - smin, n_words = 160000;  // 20^4
+            const size_t smem = nbr_smem(range);
+            CK_CUDA(cudaFuncSetAttribute(nbr_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            uint32_t *valid = (uint32_t *)scratch(SLOT_SEARCH_TMP2, (size_t)n_words * 4, &status);
+            if (!valid) return status;
+            kmer_valid_kernel<<<(n_words / 32 * 32 + 255) / 256, 256, 0, a.st>>>(a.kmer_freqs, a.freq_thresh, n_words,
+                                                                                 valid);
+            CK_CUDA(cudaGetLastError());
             int64_t listed = -1;
             for (int pass = 0; pass < 2; ++pass) {
                 CK_CUDA(cudaMemsetAsync(cursor, 0, 8, a.st));
-                nbr_list_kernel<<<grid, NB_WARPS * 32, 0, a.st>>>(a.qflat, a.qflat_len, a.qoff, a.qlen, d_sub,
-                                                                   a.score_thresh, a.kmer_freqs, a.freq_thresh, list,
-                                                                   cap, cursor, err);
+                nbr_list_kernel<<<grid, NB_WARPS * 32, smem, a.st>>>(a.qflat, a.qflat_len, a.qoff, a.qlen, d_sub, smin,
+                                                                      range, a.score_thresh, valid, list, cap, cursor,
+                                                                      err);
                 CK_CUDA(cudaGetLastError());
                 if (bounded) break;
                 unsigned long long h = 0;
