@@ -663,42 +663,45 @@ __global__ void cap_unpack_kernel(const uint64_t *__restrict__ keys, const int32
 // clustkit/kmer_index.py:1187-1291: with k = 5 every 5-mer whose BLOSUM62
 // column sum against a query 5-mer reaches the threshold T adds that sum to
 // each target of its posting list (frequency in (0, freq_thresh]).  Stage 1
-// (nbr_list_kernel) lists the (query, 5-mer, score) triples in one pass;
-// stage 2 (nbr_walk_kernel) walks their posting lists.
+// (nbr_weight_kernel) sums, per query, each 5-mer's scores over the query's
+// positions; stage 2 walks the posting lists of the 5-mers with a sum.
 //
-// Stage 1 splits a 5-mer's first four residues into two pairs.  For a query
-// position, a warp orders the 400 residue pairs (a0, a1) and the 400 pairs
-// (a2, a3) by score, descending (a counting sort: a pair's score has a few
-// dozen values).  The (a0 a1, a2 a3) combinations that can still reach the
-// threshold with the best last residue are then, for each score of the first
-// pair, a prefix of the second list: a rectangle whose cells go to the lanes
-// 32 at a time, so no lane tests a combination that clustkit's bound would
-// prune.  A cell's last residues are one AND: the residues that reach the
-// threshold (a table by query residue and score needed) and the indexed 5-mers
-// of those four residues (one bit each, kmer_valid_kernel: 640 KB, so L2 and
-// largely L1 hold it; the frequencies themselves are 12.8 MB).  Hits go to the
-// warp's shared-memory stage as 4-byte entries (value | score << 22;
-// 20^5 < 2^22, a score is at most 5 x 127); a full stage is flushed to the
-// list with one global reservation, as 8-byte entries (query << 48 |
-// score << 32 | value).  Which warp lists a triple first varies from run to
-// run; the walk's integer sums do not depend on the order.
-// 64 queries against 200,000 sequences: 8.1 -> 0.4 ms, the whole search call
-// 25.0 -> 17.3 (before, a warp tested all 400
-// continuations of every surviving pair, a lane up to 20 frequencies each).
+// Stage 1.  A block takes one query and NB_PREFIXES first residue pairs
+// (a0, a1) -- 56,000 5-mers, whose sums fit its shared memory -- and its warps
+// take the query's positions.  The pairs (a2, a3) ordered by score against two
+// query residues depend on these residues alone: nbr_tables_kernel orders them
+// for all 400 pairs of residues once a call (640 KB).  At a position the pairs
+// that can still reach the threshold after (a0, a1), with the best last
+// residue, are then a prefix of one such list: the lanes hold the prefix
+// lengths of the block's (a0, a1), and the concatenated prefixes go to the
+// lanes 32 at a time, so no lane tests a combination that clustkit's bound
+// would prune.  A combination's last residues are one AND: the residues that
+// reach the threshold (a table by query residue and score needed) and the
+// indexed 5-mers of those four residues (one bit each, kmer_valid_kernel: 640
+// KB, where the frequencies themselves are 12.8 MB).  The block then writes its
+// 5-mers with a sum, in order, to its region of the weights.
+// Summing first makes stage 2's work distinct 5-mers in index order (a 64-query
+// batch lists 144 M triples; many repeat a 5-mer of the same query), and leaves
+// nothing whose size the host would have to know.
+// 64 queries against 200,000 sequences: 1.1 ms (the first form listed triples,
+// a warp testing all 400 continuations of every surviving pair (a0,
+// a1) and a lane reading up to 20 frequencies for each: 8.1 ms).
 constexpr int32_t NB_PAIRS = 400;
-constexpr int NB_WARPS = 8;              // warps per block
-constexpr int32_t NB_STAGE = 1024;       // staged entries per warp (a round adds at most 32 x 20)
-constexpr uint32_t NB_SCORE_SHIFT = 22;
-constexpr int64_t NB_BLOCKS_PER_QUERY = 512;
+constexpr int32_t NB_KMERS = 3200000;    // 20^5
+constexpr int32_t NB_VALID = 160000;     // 20^4
+constexpr int32_t NB_PREFIXES = 7;       // (a0, a1) pairs of a block; 6 where the matrix's tables need the room
+constexpr int32_t NB_REGION = NB_PREFIXES * 8000;  // room for a block's 5-mers
+constexpr int NB_WARPS = 32;
+constexpr int32_t NB_QUERIES = 64;       // queries whose weights are held at a time (336,000 bytes a block of 5-mers)
 
 // Bit a of valid[u]: the 5-mer of the four residues u and last residue a has a
 // frequency in 1 .. freq_thresh.  A warp turns 640 frequencies into 20 ballots,
 // whose bits are then 32 words of 20.
-__global__ void kmer_valid_kernel(const int32_t *__restrict__ freqs, int32_t freq_thresh, int32_t n_words,
+__global__ void kmer_valid_kernel(const int32_t *__restrict__ freqs, int32_t freq_thresh,
                                   uint32_t *__restrict__ valid) {
     const int lane = threadIdx.x & 31;
-    const int32_t base = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-    if (base >= n_words) return;  // n_words = 20^4 is a multiple of 32
+    const int32_t base = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
+    if (base >= NB_VALID) return;  // a multiple of 32
     const int32_t bit = 20 * lane, first = bit >> 5;
     uint32_t lo = 0, hi = 0;
 #pragma unroll
@@ -711,91 +714,82 @@ __global__ void kmer_valid_kernel(const int32_t *__restrict__ freqs, int32_t fre
     valid[base + lane] = __funnelshift_r(lo, hi, bit & 31) & 0xfffffu;
 }
 
-__device__ __forceinline__ void nbr_flush(const uint32_t *stage, int32_t fill, int32_t q, uint64_t *list,
-                                          int64_t cap, unsigned long long *cursor, int lane) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(cursor, (unsigned long long)fill);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int32_t i = lane; i < fill; i += 32) {
-        const unsigned long long at = base + (unsigned long long)i;
-        if (at < (unsigned long long)cap) {
-            const uint32_t x = stage[i];
-            list[at] = ((uint64_t)(uint32_t)q << 48) | ((uint64_t)(x >> NB_SCORE_SHIFT) << 32) |
-                       (uint64_t)(x & ((1u << NB_SCORE_SHIFT) - 1u));
-        }
-    }
-}
-
-// Shared memory of the listing: the matrix, the table of last residues (20
-// rows of `range` + 1 words, range = largest - smallest matrix entry) and per
-// warp the two ordered pair lists, their starts by score (2 range + 2 each)
-// and the stage.
-__host__ __device__ constexpr size_t nbr_warp_words(int32_t range) {
-    return (size_t)(NB_PAIRS / 2 + NB_PAIRS + 2 * (2 * range + 2) + NB_STAGE);
-}
-__host__ __device__ constexpr size_t nbr_smem(int32_t range) {
-    return (400 + 20 * (size_t)(range + 1) + NB_WARPS * nbr_warp_words(range)) * 4;
-}
-
-// One residue-pair list of a position, ordered by score: bin b of `start`
-// becomes the number of pairs with a score above 2 smin + b, and put(at, pair,
-// bin) is called once for each pair.
-template <class Put>
-__device__ __forceinline__ void nbr_order_pairs(const int32_t *Sa, const int32_t *Sb, int32_t smin, int32_t bins,
-                                                int32_t *start, int lane, Put put) {
+// One warp per pair of query residues (q2, q3): the pairs (a2, a3) by score,
+// descending: ordered[at] = a2 * 20 + a3 | bin << 16 with bin = score - 2 smin,
+// and from[b] = the number of pairs of bin b or above.
+__global__ void __launch_bounds__(32)
+nbr_tables_kernel(const int8_t *__restrict__ sub, int32_t smin, int32_t bins, uint32_t *__restrict__ ordered_all,
+                  int32_t *__restrict__ from_all) {
     constexpr uint32_t FULL = 0xffffffffu;
-    for (int32_t b = lane; b < bins; b += 32) start[b] = 0;
+    __shared__ int32_t from[512];
+    const int lane = threadIdx.x;
+    const int8_t *Sa = sub + blockIdx.x / 20 * 20, *Sb = sub + blockIdx.x % 20 * 20;
+    uint32_t *ordered = ordered_all + (size_t)blockIdx.x * NB_PAIRS;
+    for (int32_t b = lane; b < bins; b += 32) from[b] = 0;
     __syncwarp();
-    for (int32_t t = lane; t < NB_PAIRS; t += 32) {
-        const int32_t a = t / 20;
-        atomicAdd(&start[Sa[a] + Sb[t - a * 20] - 2 * smin], 1);
-    }
+    for (int32_t t = lane; t < NB_PAIRS; t += 32) atomicAdd(&from[Sa[t / 20] + Sb[t % 20] - 2 * smin], 1);
     __syncwarp();
     int32_t above = 0;  // pairs in the bins already passed (higher scores)
     for (int32_t top = bins - 1; top >= 0; top -= 32) {
         const int32_t b = top - lane;
-        const int32_t n = b >= 0 ? start[b] : 0;
+        const int32_t n = b >= 0 ? from[b] : 0;
         int32_t incl = n;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int32_t x = __shfl_up_sync(FULL, incl, d);
             if (lane >= d) incl += x;
         }
-        if (b >= 0) start[b] = above + incl - n;
+        if (b >= 0) from[b] = above + incl - n;
         above += __shfl_sync(FULL, incl, 31);
     }
     __syncwarp();
     for (int32_t t = lane; t < NB_PAIRS; t += 32) {
-        const int32_t a = t / 20, b = Sa[a] + Sb[t - a * 20] - 2 * smin;
-        put(atomicAdd(&start[b], 1), t, b);  // leaves start[b] = pairs with a score of bin b or above
+        const int32_t b = Sa[t / 20] + Sb[t % 20] - 2 * smin;
+        ordered[atomicAdd(&from[b], 1)] = (uint32_t)t | ((uint32_t)b << 16);  // each bin's count goes on top
     }
     __syncwarp();
+    for (int32_t b = lane; b < bins; b += 32) from_all[(size_t)blockIdx.x * bins + b] = from[b];
 }
 
-// Lists every (query, 5-mer, score) triple; *cursor (zeroed by the caller)
-// ends as the number of triples, of which the first `cap` are written.
-__global__ void __launch_bounds__(NB_WARPS * 32)
-nbr_list_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int64_t *__restrict__ qoff,
-                const int32_t *__restrict__ qlen, const int8_t *__restrict__ sub, int32_t smin, int32_t range,
-                int32_t T, const uint32_t *__restrict__ valid, uint64_t *__restrict__ list, int64_t cap,
-                unsigned long long *__restrict__ cursor, int32_t *err) {
+// Shared memory of stage 1: the sums, the matrix, the table of last residues
+// (20 rows of `range` + 1 words, range = largest - smallest matrix entry).
+__host__ __device__ constexpr size_t nbr_smem(int32_t prefixes, int32_t range) {
+    return ((size_t)prefixes * 8000 + 400 + 20 * (size_t)(range + 1)) * 4;
+}
+
+// Grid (blocks of 5-mers, queries).  Region q * gridDim.x + block of the
+// weights gets n[region] 5-mers: kmer (counted from the block's first) and
+// weight, in 5-mer order.  *listed grows by the (query position, 5-mer) pairs
+// that reached the threshold.
+__global__ void __launch_bounds__(NB_WARPS * 32, 1)
+nbr_weight_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int64_t *__restrict__ qoff,
+                  const int32_t *__restrict__ qlen, const int8_t *__restrict__ sub, int32_t smin, int32_t range,
+                  int32_t T, const uint32_t *__restrict__ valid, const uint32_t *__restrict__ ordered_all,
+                  const int32_t *__restrict__ from_all, int32_t prefixes, int32_t *__restrict__ n,
+                  uint16_t *__restrict__ kmer, int32_t *__restrict__ weight, unsigned long long *__restrict__ listed,
+                  int32_t *err) {
     constexpr uint32_t FULL = 0xffffffffu;
     extern __shared__ int32_t nb_smem[];
-    int32_t *S = nb_smem;
-    uint32_t *reach = (uint32_t *)(nb_smem + 400);  // [query residue][score needed - smin]: last residues that give it
-    const int32_t q = blockIdx.y;
+    __shared__ int32_t warp_n[NB_WARPS];
+    const int32_t size = prefixes * 8000;
+    int32_t *W = nb_smem, *S = nb_smem + size;
+    uint32_t *reach = (uint32_t *)(S + 400);  // [query residue][score needed - smin]: last residues that give it
+    const int32_t q = blockIdx.y, region = q * gridDim.x + blockIdx.x;
     const int32_t L = qlen[q];
     const int64_t o = qoff[q];
     // both exits are the same for the whole block (before its first barrier)
-    if (L < 0 || o < 0 || o + L > qflat_len) {
-        if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(err, ERRBIT_SEQ_EXTENT);
+    const bool bad = L < 0 || o < 0 || o + L > qflat_len;
+    if (bad || L < 5) {
+        if (threadIdx.x == 0) {
+            n[region] = 0;
+            if (bad && blockIdx.x == 0) atomicOr(err, ERRBIT_SEQ_EXTENT);
+        }
         return;
     }
-    const int32_t npos = L >= 5 ? L - 4 : 0;
-    if ((int32_t)blockIdx.x * NB_WARPS >= npos) return;  // a shorter query than the batch's longest
-    for (int i = threadIdx.x; i < 400; i += blockDim.x) S[i] = sub[i];
+    for (int i = threadIdx.x; i < size / 4; i += NB_WARPS * 32) ((int4 *)W)[i] = make_int4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < 400; i += NB_WARPS * 32) S[i] = sub[i];
     __syncthreads();
-    for (int i = threadIdx.x; i < 20 * (range + 1); i += blockDim.x) {
+    for (int i = threadIdx.x; i < 20 * (range + 1); i += NB_WARPS * 32) {
         const int32_t a = i / (range + 1), need = i - a * (range + 1) + smin;
         uint32_t m = 0;
         for (int b = 0; b < 20; ++b) m |= S[a * 20 + b] >= need ? 1u << b : 0u;
@@ -804,179 +798,367 @@ nbr_list_kernel(const uint8_t *__restrict__ qflat, int64_t qflat_len, const int6
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int32_t bins = 2 * range + 1;
-    uint32_t *pairs2 = (uint32_t *)(nb_smem + 400 + 20 * (range + 1) + (size_t)warp * nbr_warp_words(range));
-    uint16_t *pairs1 = (uint16_t *)(pairs2 + NB_PAIRS);
-    int32_t *n1 = (int32_t *)(pairs2 + NB_PAIRS + NB_PAIRS / 2), *n2 = n1 + 2 * range + 2;
-    uint32_t *stage = (uint32_t *)(n2 + 2 * range + 2);
     const uint8_t *sq = qflat + o;
-    int32_t fill = 0;  // warp-uniform
-    for (int32_t p = blockIdx.x * NB_WARPS + warp; p < npos; p += gridDim.x * NB_WARPS) {
+    // this lane's first residues (the first `prefixes` lanes)
+    const int32_t a01 = blockIdx.x * prefixes + lane;
+    const bool has = lane < prefixes && a01 < NB_PAIRS;
+    const int32_t a0 = has ? a01 / 20 : 0, a1 = has ? a01 % 20 : 0;
+    uint32_t count = 0;
+    for (int32_t p = warp; p <= L - 5; p += NB_WARPS) {
         const int32_t q0 = sq[p], q1 = sq[p + 1], q2 = sq[p + 2], q3 = sq[p + 3], q4 = sq[p + 4];
         if (q0 >= 20 || q1 >= 20 || q2 >= 20 || q3 >= 20 || q4 >= 20) continue;  // the same for the whole warp
-        __syncwarp();
-        nbr_order_pairs(S + q0 * 20, S + q1 * 20, smin, bins, n1, lane,
-                        [&](int32_t at, int32_t t, int32_t) { pairs1[at] = (uint16_t)t; });
-        nbr_order_pairs(S + q2 * 20, S + q3 * 20, smin, bins, n2, lane,
-                        [&](int32_t at, int32_t t, int32_t b) { pairs2[at] = (uint32_t)t | ((uint32_t)b << 16); });
-        int32_t m4 = range;  // the best last residue's score, less smin
-        while (m4 > 0 && reach[q4 * (range + 1) + m4] == 0) --m4;
-        for (int32_t b1 = bins - 1; b1 >= 0; --b1) {
-            // second pairs must have bin >= T - (their last residue's best) - first pair's score
-            const int32_t need = T - (m4 + smin) - (b1 + 2 * smin) - 2 * smin;
-            if (need >= bins) break;  // and so for every lower first pair
-            const int32_t i1 = b1 + 1 < bins ? n1[b1 + 1] : 0, c1 = n1[b1] - i1, c2 = n2[need > 0 ? need : 0];
-            if (c2 == 0) break;
-            const int32_t cells = c1 * c2;
-            // cell / c2 by a multiplication: exact, as cell * c2 <= 160,000 * 400 < 2^32
-            const uint32_t inv = (uint32_t)(0x100000000ull / (uint32_t)c2) + 1u;
-            for (int32_t k0 = 0; k0 < cells; k0 += 32) {
-                const int32_t k = k0 + lane;
-                uint32_t bits = 0;
-                int32_t s4 = 0, v4 = 0;
-                if (k < cells) {
-                    const int32_t row = c2 == 1 ? k : (int32_t)__umulhi((uint32_t)k, inv);
-                    const uint32_t x = pairs2[k - row * c2];
-                    s4 = b1 + (int32_t)(x >> 16) + 4 * smin;
-                    v4 = (int32_t)pairs1[i1 + row] * NB_PAIRS + (int32_t)(x & 0xffffu);
-                    int32_t w = T - s4 - smin;
-                    w = w < 0 ? 0 : w;  // at most m4
-                    bits = reach[q4 * (range + 1) + w] & __ldg(valid + v4);
-                }
-                if (!__any_sync(FULL, bits != 0)) continue;
-                const int32_t n = __popc(bits);
-                int32_t incl = n;
+        const uint32_t *reach4 = reach + q4 * (range + 1);
+        int32_t m4 = S[q4 * 20 + (lane < 20 ? lane : 0)];  // the best last residue's score
+        m4 = __reduce_max_sync(FULL, m4);
+        const int32_t s01 = S[q0 * 20 + a0] + S[q1 * 20 + a1];
+        // how many (a2, a3) can reach T: those of bin `need` or above
+        const int32_t need = T - m4 - s01 - 2 * smin;
+        const int32_t pair = q2 * 20 + q3;
+        const int32_t mine = has && need < bins ? __ldg(from_all + pair * bins + (need > 0 ? need : 0)) : 0;
+        int32_t incl = mine;
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int32_t y = __shfl_up_sync(FULL, incl, d);
-                    if (lane >= d) incl += y;
-                }
-                const int32_t tot = __shfl_sync(FULL, incl, 31);
-                if (fill + tot > NB_STAGE) {
-                    __syncwarp();
-                    nbr_flush(stage, fill, q, list, cap, cursor, lane);
-                    __syncwarp();
-                    fill = 0;
-                }
-                int32_t at = fill + incl - n;
+        for (int d = 1; d < 8; d <<= 1) {  // prefixes <= 7
+            const int32_t x = __shfl_up_sync(FULL, incl, d);
+            if (lane >= d) incl += x;
+        }
+        const int32_t excl = incl - mine, cells = __shfl_sync(FULL, incl, 7);
+        const uint32_t *ordered = ordered_all + pair * NB_PAIRS;
+        for (int32_t k0 = 0; k0 < cells; k0 += 32) {
+            const int32_t k = k0 + lane;
+            int32_t a = 0;  // the last prefix that starts at or before k
+#pragma unroll
+            for (int step = 4; step; step >>= 1)
+                if (__shfl_sync(FULL, excl, a + step) <= k) a += step;
+            const int32_t at = k - __shfl_sync(FULL, excl, a);
+            const int32_t sa = __shfl_sync(FULL, s01, a);
+            if (k < cells) {
+                const uint32_t x = __ldg(ordered + at);
+                const int32_t s4 = sa + (int32_t)(x >> 16) + 2 * smin, v4 = a * NB_PAIRS + (int32_t)(x & 0xffffu);
+                const int32_t w = T - s4 - smin;  // at most m4 - smin
+                uint32_t bits = reach4[w < 0 ? 0 : w] & __ldg(valid + blockIdx.x * prefixes * NB_PAIRS + v4);
+                count += __popc(bits);
                 while (bits) {
                     const int b = __ffs(bits) - 1;
                     bits &= bits - 1;
-                    stage[at++] = (uint32_t)(v4 * 20 + b) | ((uint32_t)(s4 + S[q4 * 20 + b]) << NB_SCORE_SHIFT);
+                    atomicAdd(&W[v4 * 20 + b], s4 + S[q4 * 20 + b]);
                 }
-                fill += tot;
             }
         }
     }
-    if (fill > 0) {
-        __syncwarp();
-        nbr_flush(stage, fill, q, list, cap, cursor, lane);
+    count = __reduce_add_sync(FULL, count);
+    if (lane == 0 && count) atomicAdd(listed, (unsigned long long)count);
+    __syncthreads();
+    // the block's 5-mers with a sum (T >= 1, so a listed 5-mer's is positive):
+    // each warp a slice, counted, then written behind the slices before it
+    const int32_t slice = (size / 32 + NB_WARPS - 1) / NB_WARPS * 32;
+    const int32_t w0 = warp * slice, w1 = w0 + slice < size ? w0 + slice : size;
+    int32_t here = 0;
+    for (int32_t i = w0 + lane; i < w1; i += 32) here += W[i] != 0;
+    here = __reduce_add_sync(FULL, here);
+    if (lane == 0) warp_n[warp] = here;
+    __syncthreads();
+    const int32_t wn = warp_n[lane];
+    const int32_t total = __reduce_add_sync(FULL, wn);
+    int32_t at = __reduce_add_sync(FULL, lane < warp ? wn : 0);
+    uint16_t *ko = kmer + (size_t)region * NB_REGION;
+    int32_t *wo = weight + (size_t)region * NB_REGION;
+    for (int32_t i0 = w0; i0 < w1; i0 += 32) {
+        const int32_t x = i0 + lane < w1 ? W[i0 + lane] : 0;
+        const uint32_t bal = __ballot_sync(FULL, x != 0);
+        if (x != 0) {
+            const int32_t to = at + __popc(bal & ((1u << lane) - 1u));
+            ko[to] = (uint16_t)(i0 + lane);
+            wo[to] = x;
+        }
+        at += __popc(bal);
     }
+    if (threadIdx.x == 0) n[region] = total;
 }
 
 __global__ void fill_kernel(int32_t *a, int32_t n, int32_t v) {
     for (int32_t i = threadIdx.x; i < n; i += blockDim.x) a[i] = v;
 }
 
-// Stage 2.  A persistent grid; each block takes chunks of the list in order
-// (a ticket counter) and walks them.  The listing pass fills the list about
-// one query at a time, so the blocks in flight add into one or two queries'
-// count rows, which stay in L2 (a grid-stride walk, whose warps drift apart
-// over the whole list, kept every row of a 64-query batch live: 25.7 GB of
-// DRAM writes instead of 0.24, and 1.5x the time).  The chunk comes from the
-// count on the device (a multiple of 256, at most 2,048 triples): at least
-// two per block, and the blocks in flight within about two queries' triples;
-// so the launch needs no count from the host.
-// A warp takes 32 triples at once: each lane loads one and its posting-list
-// bounds -- 32 independent loads instead of 32 chains -- then the warp walks
-// the concatenated lists, lane k of each round taking entry k of the stream
-// (its list found by a binary search over the lanes' exclusive prefix sums
-// of list lengths) and adding the triple's score to the entry's target in
-// the triple's query row.  A list longer than `cap` (the listing pass
-// counted more triples than it could write) is reported.
-// Warps of the block take 32 triples of [c0, c1) at a time.
-__device__ __forceinline__ void walk_chunk(const uint64_t *__restrict__ list, int64_t c0, int64_t c1, int32_t nq,
-                                           const int64_t *__restrict__ kmer_offsets,
-                                           const int64_t *__restrict__ kmer_entries,
-                                           const int32_t *__restrict__ kmer_targets, int32_t num_db,
-                                           int32_t *__restrict__ counts, int32_t *err, int lane) {
+// Stage 2 on the count rows, for few queries.  A persistent grid; each block
+// takes runs of a region's 5-mers (a ticket counter; regions in query order, so
+// the blocks in flight add into one or two queries' count rows, which stay in
+// L2).  A warp takes 32 5-mers at once: each lane loads one and its
+// posting-list bounds -- 32 independent loads instead of 32 chains -- then the
+// warp walks the concatenated lists, lane k of each round taking entry k of
+// the stream (its list found by a binary search over the lanes' exclusive
+// prefix sums of list lengths) and adding the 5-mer's weight to the entry's
+// target in the query's row.  Bound by L2's atomic units (about 200 G adds/s).
+constexpr int32_t NB_RUN = 1024;  // 5-mers of a run
+
+// A region's first run: the runs before it (one block; regions in order).
+__global__ void __launch_bounds__(1024)
+nbr_runs_kernel(const int32_t *__restrict__ n, int32_t regions, int32_t *__restrict__ run0) {
+    using Scan = cub::BlockScan<int32_t, 1024>;
+    __shared__ typename Scan::TempStorage tmp;
+    int32_t run = 0, sum;
+    for (int32_t g0 = 0; g0 < regions; g0 += 1024) {
+        const int32_t g = g0 + threadIdx.x;
+        int32_t at;
+        Scan(tmp).ExclusiveSum(g < regions ? (n[g] + NB_RUN - 1) / NB_RUN : 0, at, sum);
+        if (g < regions) run0[g] = run + at;
+        run += sum;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) run0[regions] = run;
+}
+
+__global__ void __launch_bounds__(256)
+nbr_walk_kernel(const int32_t *__restrict__ n, const int32_t *__restrict__ run0, const uint16_t *__restrict__ kmer,
+                const int32_t *__restrict__ weight, int32_t regions, int32_t n_blocks, int32_t block_kmers,
+                const int64_t *__restrict__ kmer_offsets, const int64_t *__restrict__ kmer_entries,
+                const int32_t *__restrict__ kmer_targets, int32_t num_db, int32_t *__restrict__ counts,
+                unsigned long long *__restrict__ ticket, const unsigned long long *__restrict__ order, int32_t *err) {
     constexpr uint32_t FULL = 0xffffffffu;
-    for (int64_t base = c0 + (threadIdx.x >> 5) * 32; base < c1; base += blockDim.x) {
-        const int64_t e = base + lane;
-        int64_t b = 0;
-        int32_t len = 0, w = 0, qq = 0;
-        if (e < c1) {
-            const uint64_t x = list[e];
-            const int32_t v = (int32_t)(x & 0xffffffffu);
-            w = (int32_t)((x >> 32) & 0xffffu);
-            qq = (int32_t)(x >> 48);
-            if (qq < nq) {
+    __shared__ int32_t s_run;
+    if (order && order[0] == order[1] && order[2] == 0) return;  // the walk by target ranges has taken the call
+    const int lane = threadIdx.x & 31;
+    const int32_t runs = run0[regions];
+    for (;;) {
+        if (threadIdx.x == 0) {
+            const unsigned long long t = atomicAdd(ticket, 1ull);
+            s_run = t < (unsigned long long)runs ? (int32_t)t : -1;
+        }
+        __syncthreads();
+        const int32_t run = s_run;
+        __syncthreads();  // every thread has read s_run before it is written again
+        if (run < 0) break;  // the same for the whole block
+        int32_t g = 0, hi = regions;  // the last region whose first run is at or before this one
+        while (hi - g > 1) {
+            const int32_t mid = (g + hi) >> 1;
+            if (run0[mid] <= run) g = mid; else hi = mid;
+        }
+        const int32_t c0 = (run - run0[g]) * NB_RUN, c1 = c0 + NB_RUN < n[g] ? c0 + NB_RUN : n[g];
+        const int32_t v0 = g % n_blocks * block_kmers;
+        int32_t *row = counts + (int64_t)(g / n_blocks) * num_db;
+        for (int32_t base = c0 + (threadIdx.x >> 5) * 32; base < c1; base += 256) {
+            const int32_t e = base + lane;
+            int64_t b = 0;
+            int32_t len = 0, w = 0;
+            if (e < c1) {
+                const int32_t v = v0 + kmer[(size_t)g * NB_REGION + e];
+                w = weight[(size_t)g * NB_REGION + e];
                 b = kmer_offsets[v];
                 len = (int32_t)(kmer_offsets[v + 1] - b);
-            } else {
-                atomicOr(err, ERRBIT_PAIR_INDEX);
             }
-        }
-        int32_t incl = len;
+            int32_t incl = len;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t t = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int32_t excl = incl - len;
-        const int32_t total = __shfl_sync(FULL, incl, 31);
-        // rounds are warp-uniform so that every shuffle reads a live lane
-        for (int32_t k0 = 0; k0 < total; k0 += 32) {
-            const int32_t k = k0 + lane;
-            // the stream's entry k belongs to the last lane whose list starts
-            // at or before k (lanes with empty lists share their successor's
-            // start and lose to it)
-            int32_t o = 0;
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const int32_t cand = o + step;
-                if (__shfl_sync(FULL, excl, cand) <= k) o = cand;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += t;
             }
-            const int64_t h = __shfl_sync(FULL, b, o) + (k - __shfl_sync(FULL, excl, o));
-            const int32_t wo = __shfl_sync(FULL, w, o);
-            const int32_t qo = __shfl_sync(FULL, qq, o);
-            if (k < total) {
-                const int32_t t = entry_target(kmer_entries, kmer_targets, h);
-                if (t < 0 || t >= num_db) {
-                    atomicOr(err, ERRBIT_PAIR_INDEX);
-                } else {
-                    // no candidate list here (most of the database crosses
-                    // min_hits in this mode; the select scans the row): the
-                    // add's result is unused
-                    atomicAdd(&counts[(int64_t)qo * num_db + t], wo);
+            const int32_t excl = incl - len;
+            const int32_t total = __shfl_sync(FULL, incl, 31);
+            // rounds are warp-uniform so that every shuffle reads a live lane
+            for (int32_t k0 = 0; k0 < total; k0 += 32) {
+                const int32_t k = k0 + lane;
+                // the stream's entry k belongs to the last lane whose list starts
+                // at or before k (lanes with empty lists share their successor's
+                // start and lose to it)
+                int32_t o = 0;
+#pragma unroll
+                for (int step = 16; step; step >>= 1) {
+                    const int32_t cand = o + step;
+                    if (__shfl_sync(FULL, excl, cand) <= k) o = cand;
+                }
+                const int64_t h = __shfl_sync(FULL, b, o) + (k - __shfl_sync(FULL, excl, o));
+                const int32_t wo = __shfl_sync(FULL, w, o);
+                if (k < total) {
+                    const int32_t t = entry_target(kmer_entries, kmer_targets, h);
+                    if (t < 0 || t >= num_db) {
+                        atomicOr(err, ERRBIT_PAIR_INDEX);
+                    } else {
+                        // no candidate list here (most of the database crosses
+                        // min_hits in this mode; the select scans the row): the
+                        // add's result is unused
+                        atomicAdd(&row[t], wo);
+                    }
                 }
             }
         }
     }
 }
 
-__global__ void nbr_walk_kernel(const uint64_t *__restrict__ list, const unsigned long long *__restrict__ cursor,
-                                int64_t cap, int32_t nq, const int64_t *__restrict__ kmer_offsets,
-                                const int64_t *__restrict__ kmer_entries, const int32_t *__restrict__ kmer_targets,
-                                int32_t num_db, int32_t *__restrict__ counts, unsigned long long *__restrict__ ticket,
-                                int32_t *err) {
-    __shared__ int64_t s_c0;
-    const int lane = threadIdx.x & 31;
-    const unsigned long long listed = *cursor;
-    if (listed > (unsigned long long)cap && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, ERRBIT_LIST);
-    const int64_t n = (int64_t)(listed < (unsigned long long)cap ? listed : (unsigned long long)cap);
-    const int64_t G = gridDim.x;
-    int64_t chunk = 2 * n / ((int64_t)(nq > 0 ? nq : 1) * G);
-    if (n / (2 * G) < chunk) chunk = n / (2 * G);
-    chunk = chunk / 256 * 256;
-    chunk = chunk < 256 ? 256 : (chunk > 2048 ? 2048 : chunk);
+// Stage 2 by target ranges, for calls of several queries.  Here the targets
+// are cut into ranges of at most NB_RANGE, whose counters for one query fit a
+// block's shared memory: a work unit is (range, some blocks of 5-mers, query);
+// its block adds the postings that fall in the range into shared memory and
+// then adds the counters to the query's row, coalesced.  Every list is cut at
+// the range boundaries once per call (frag_kernel), so a block reads only its
+// range's part of a list.  Units are taken range by range, then 5-mers by
+// 5-mers, with all queries' units of these together, so that the cuts and
+// postings in use stay in L2 (in query order the same walk read 45 GB from
+// DRAM).  A lane walks its own 5-mer's part, eight postings (a sector) a load
+// and two loads in flight, with the next 5-mer's cut and the one after's
+// weight on their way: a part is a few postings long, sharing parts among
+// lanes cost more shuffles than the idle lanes do, and one load at a time left
+// the walk waiting for L2.
+// The cuts need lists in target order, as the index build leaves them;
+// order_kernel checks that (and that targets lie in the database), and a call
+// whose lists are not goes to the walk above.  Cutting and checking cost about
+// what a few queries save, so fewer than NB_RANGE_MIN_QUERIES keep that one.
+// 64 queries, 200,000 sequences: 5.3 ms, with 0.2 for the cuts and the check;
+// the walk on the count rows took 11.4 (listed triples, repeats and all).
+constexpr int32_t NB_RANGE = 56 * 1024;   // counters of a block: 224 KB of shared memory
+constexpr int32_t NB_MAX_RANGES = 16;     // 917,504 targets; 25.6 MB of cuts each
+constexpr int NB_RW_THREADS = 1024;
+constexpr int32_t NB_RANGE_MIN_QUERIES = 4;
+
+// Whether every list is in target order: the places where a target is below
+// the one before it, over the whole index, less those where a list starts
+// (order[0] - order[1], 0 when all are in order); order[2] counts targets
+// outside the database.
+__global__ void order_kernel(const int64_t *__restrict__ kmer_offsets, const int64_t *__restrict__ kmer_entries,
+                             const int32_t *__restrict__ kmer_targets, int32_t n_kmers, int32_t num_db,
+                             unsigned long long *__restrict__ order) {
+    const int64_t total = kmer_offsets[n_kmers], step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t me = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t falls = 0, starts = 0, outside = 0;
+    for (int64_t h = me * 4; h < total; h += step * 4) {
+        int32_t before = h > 0 ? entry_target(kmer_entries, kmer_targets, h - 1) : -1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (h + i >= total) break;
+            const int32_t t = entry_target(kmer_entries, kmer_targets, h + i);
+            falls += t < before;
+            outside += t < 0 || t >= num_db;
+            before = t;
+        }
+    }
+    for (int64_t v = me; v < n_kmers; v += step) {
+        const int64_t b = kmer_offsets[v], e = kmer_offsets[v + 1];
+        if (b > 0 && b < e)
+            starts += entry_target(kmer_entries, kmer_targets, b) < entry_target(kmer_entries, kmer_targets, b - 1);
+        outside += b < 0 || b > e || e > total || e > (int64_t)0xffffffff;
+    }
+    falls = __reduce_add_sync(0xffffffffu, falls);
+    starts = __reduce_add_sync(0xffffffffu, starts);
+    outside = __reduce_add_sync(0xffffffffu, outside);
+    if ((threadIdx.x & 31) == 0) {
+        if (falls) atomicAdd(order, (unsigned long long)falls);
+        if (starts) atomicAdd(order + 1, (unsigned long long)starts);
+        if (outside) atomicAdd(order + 2, (unsigned long long)outside);
+    }
+}
+__device__ __forceinline__ bool lists_in_order(const unsigned long long *order) {
+    return order[0] == order[1] && order[2] == 0;
+}
+
+// frag[r * n_kmers + v] = (first posting of v in range r, their number), by a
+// binary search for each boundary; the lists of a warp's 32 5-mers lie side by
+// side, so its searches share lines.  Lists that no walk reads stay empty.
+__global__ void frag_kernel(const int64_t *__restrict__ kmer_offsets, const int64_t *__restrict__ kmer_entries,
+                            const int32_t *__restrict__ kmer_targets, const int32_t *__restrict__ kmer_freqs,
+                            int32_t freq_thresh, int32_t n_kmers, int32_t range, int32_t n_ranges,
+                            const unsigned long long *__restrict__ order, uint2 *__restrict__ frag) {
+    if (!lists_in_order(order)) return;
+    const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n_kmers) return;
+    const int32_t f = kmer_freqs[v];
+    const int64_t b = kmer_offsets[v];
+    const bool walked = f != 0 && f <= freq_thresh;
+    const uint32_t end = (uint32_t)(walked ? kmer_offsets[v + 1] : b);
+    uint32_t at = (uint32_t)b;
+    for (int32_t r = 0; r < n_ranges; ++r) {
+        uint32_t lo = at, hi = end;
+        if (r + 1 == n_ranges) lo = hi;
+        const int32_t bound = (r + 1) * range;  // at most 16 x 57,344
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (entry_target(kmer_entries, kmer_targets, mid) < bound) lo = mid + 1; else hi = mid;
+        }
+        frag[(size_t)r * n_kmers + v] = make_uint2(at, lo - at);
+        at = lo;
+    }
+}
+
+// eight targets from a 32-byte boundary
+__device__ __forceinline__ void load_targets(const int32_t *p, int32_t (&t)[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+        : "l"(p));
+}
+
+__global__ void __launch_bounds__(NB_RW_THREADS, 1)
+nbr_range_walk_kernel(const int32_t *__restrict__ n, const uint16_t *__restrict__ kmer,
+                      const int32_t *__restrict__ weight, int32_t nq, int32_t n_blocks, int32_t block_kmers,
+                      int32_t set_blocks, const uint2 *__restrict__ frag, const int64_t *__restrict__ kmer_offsets,
+                      const int64_t *__restrict__ kmer_entries, const int32_t *__restrict__ kmer_targets,
+                      int32_t num_db, int32_t range, int32_t n_ranges, const unsigned long long *__restrict__ order,
+                      int32_t *__restrict__ counts, unsigned long long *__restrict__ ticket) {
+    extern __shared__ int32_t acc[];
+    __shared__ int32_t s_unit;
+    if (!lists_in_order(order)) return;
+    // eight targets a load where the compact index starts on a 32-byte boundary;
+    // a load that would pass the index's end is not made as one
+    const bool octets = kmer_targets && ((uintptr_t)kmer_targets & 31) == 0;
+    const uint32_t total = (uint32_t)kmer_offsets[NB_KMERS];
+    const int32_t sets = (n_blocks + set_blocks - 1) / set_blocks, units = n_ranges * sets * nq;
+    for (int32_t i = threadIdx.x; i < range; i += NB_RW_THREADS) acc[i] = 0;
     for (;;) {
-        if (threadIdx.x == 0) s_c0 = (int64_t)atomicAdd(ticket, 1ull) * chunk;
+        if (threadIdx.x == 0) {
+            const unsigned long long t = atomicAdd(ticket, 1ull);
+            s_unit = t < (unsigned long long)units ? (int32_t)t : -1;
+        }
         __syncthreads();
-        const int64_t c0 = s_c0;
-        __syncthreads();  // every thread has read s_c0 before it is written again
-        if (c0 >= n) break;  // the same for the whole block
-        const int64_t c1 = c0 + chunk < n ? c0 + chunk : n;
-        walk_chunk(list, c0, c1, nq, kmer_offsets, kmer_entries, kmer_targets, num_db, counts, err, lane);
+        const int32_t u = s_unit;
+        if (u < 0) break;  // the same for the whole block
+        const int32_t r = u / (sets * nq), set = u / nq % sets, q = u % nq;
+        const int32_t t0 = r * range, nt = num_db - t0 < range ? num_db - t0 : range;
+        int32_t *mine = acc - t0;  // only ever indexed by targets of the range
+        const int32_t b1 = (set + 1) * set_blocks < n_blocks ? (set + 1) * set_blocks : n_blocks;
+        for (int32_t b = set * set_blocks; b < b1; ++b) {
+            const int32_t region = q * n_blocks + b, size = n[region];
+            const uint16_t *ks = kmer + (size_t)region * NB_REGION;
+            const int32_t *ws = weight + (size_t)region * NB_REGION;
+            const uint2 *fr = frag + (size_t)r * NB_KMERS + b * block_kmers;
+            int32_t c = threadIdx.x;
+            uint32_t v_next = c + NB_RW_THREADS < size ? __ldg(ks + c + NB_RW_THREADS) : 0u;
+            uint2 f = c < size ? __ldg(fr + __ldg(ks + c)) : make_uint2(0u, 0u);
+            int32_t w = c < size ? __ldg(ws + c) : 0;
+            for (; c < size; c += NB_RW_THREADS) {
+                const uint2 part = f;
+                const int32_t score = w;
+                if (c + NB_RW_THREADS < size) {
+                    f = __ldg(fr + v_next);
+                    w = __ldg(ws + c + NB_RW_THREADS);
+                    if (c + 2 * NB_RW_THREADS < size) v_next = __ldg(ks + c + 2 * NB_RW_THREADS);
+                }
+                if (part.y == 0) continue;
+                const uint32_t end = part.x + part.y;
+                if (octets && ((end + 7) & ~7u) <= total) {
+                    for (uint32_t h = part.x & ~7u; h < end; h += 16) {
+                        int32_t t[8], t2[8];
+                        const bool two = h + 8 < end;
+                        load_targets(kmer_targets + h, t);
+                        if (two) load_targets(kmer_targets + h + 8, t2);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (h + i - part.x < part.y) atomicAdd(&mine[t[i]], score);
+                        if (two) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                if (h + 8 + i < end) atomicAdd(&mine[t2[i]], score);
+                        }
+                    }
+                } else {
+                    for (uint32_t h = part.x; h < end; ++h)
+                        atomicAdd(&mine[entry_target(kmer_entries, kmer_targets, h)], score);
+                }
+            }
+        }
+        __syncthreads();
+        // the counters go to the query's row and are zero again for the next unit
+        int32_t *row = counts + (int64_t)q * num_db + t0;
+        for (int32_t i = threadIdx.x; i < nt; i += NB_RW_THREADS) {
+            const int32_t x = acc[i];
+            if (x) { atomicAdd(&row[i], x); acc[i] = 0; }
+        }
+        __syncthreads();  // also: every thread has read s_unit before it is written again
     }
 }
 
@@ -1101,7 +1283,7 @@ struct PhaseAArgs {
     const int32_t *kmer_freqs; int32_t freq_thresh; int32_t num_db; int32_t min_hits; int32_t top_k;
     int32_t *out_targets; int32_t *out_scores; int32_t *out_n; cudaStream_t st;
     bool ordered = true;  // capped rows in (score desc, id asc) order, not only the set
-    int64_t list_capacity = -1;  // similar k-mers: caller's bound on listed triples, < 0 sized here
+    int64_t list_capacity = -1;  // similar k-mers: caller's bound on (position, 5-mer) pairs, < 0 none
 };
 
 // The select, then the order of rows capped above CAND_CAP.  `ordered`:
@@ -1176,6 +1358,99 @@ static int32_t select_rows(const int32_t *counts, int32_t nq, int32_t num_db, in
     return CK_OK;
 }
 
+// Error when a bounded call's pairs of query position and 5-mer pass its bound.
+__global__ void nbr_bound_kernel(const unsigned long long *__restrict__ listed, int64_t cap, int32_t *err) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && *listed > (unsigned long long)cap) atomicOr(err, ERRBIT_LIST);
+}
+
+// Similar k-mers: the weights of NB_QUERIES queries at a time, and their walk.
+static int32_t similar_weights_and_walk(const PhaseAArgs &a, const int8_t *d_sub, int32_t *counts, int32_t *err) {
+    int32_t status = CK_OK;
+    int32_t smin = a.sub_host[0], smax = a.sub_host[0];
+    for (int i = 1; i < 400; ++i) {
+        smin = std::min<int32_t>(smin, a.sub_host[i]);
+        smax = std::max<int32_t>(smax, a.sub_host[i]);
+    }
+    const int32_t srange = smax - smin, bins = 2 * srange + 1;
+    constexpr size_t SMEM = 227 * 1024 - 256;  // a block's most, less its static part
+    const int32_t prefixes = nbr_smem(NB_PREFIXES, srange) <= SMEM ? NB_PREFIXES : NB_PREFIXES - 1;
+    const size_t smem = nbr_smem(prefixes, srange);
+    const int32_t n_blocks = (NB_PAIRS + prefixes - 1) / prefixes, block_kmers = prefixes * 8000;
+    const int32_t chunk = std::min(a.nq, NB_QUERIES);
+    const size_t regions = (size_t)chunk * n_blocks;
+    // totals and tickets (8-byte words), then each region's count and first run
+    unsigned long long *words = (unsigned long long *)scratch(SLOT_SEARCH_TMP0, 8 * 8 + (2 * regions + 1) * 4, &status);
+    if (!words) return status;
+    unsigned long long *listed = words, *ticket = words + 1, *ticket2 = words + 2, *order = words + 4;
+    int32_t *n = (int32_t *)(words + 8), *run0 = n + regions;
+    // the bits of indexed 5-mers and the ordered residue pairs
+    uint32_t *valid = (uint32_t *)scratch(SLOT_SEARCH_TMP2, ((size_t)2 * NB_VALID + (size_t)NB_PAIRS * bins) * 4, &status);
+    if (!valid) return status;
+    uint32_t *ordered = valid + NB_VALID;
+    int32_t *from = (int32_t *)(ordered + NB_VALID);
+    int32_t *weight = (int32_t *)scratch(SLOT_SEARCH_TMP1, regions * NB_REGION * 6, &status);
+    if (!weight) return status;
+    uint16_t *kmer = (uint16_t *)(weight + regions * NB_REGION);
+    // by target ranges: several queries, on a database of at most NB_MAX_RANGES ranges
+    int32_t n_ranges = (int32_t)(((int64_t)a.num_db + NB_RANGE - 1) / NB_RANGE), range = 0;
+    uint2 *frag = nullptr;
+    if (a.nq >= NB_RANGE_MIN_QUERIES && n_ranges >= 1 && n_ranges <= NB_MAX_RANGES) {
+        range = (a.num_db + n_ranges - 1) / n_ranges;
+        frag = (uint2 *)scratch(SLOT_SEARCH_TMP4, (size_t)n_ranges * NB_KMERS * 8, &status);
+        if (!frag) return status;
+    } else {
+        n_ranges = 0;
+    }
+    CK_CUDA(cudaFuncSetAttribute(nbr_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK_CUDA(cudaMemsetAsync(words, 0, 8 * 8, a.st));
+    kmer_valid_kernel<<<NB_VALID / 256, 256, 0, a.st>>>(a.kmer_freqs, a.freq_thresh, valid);
+    CK_CUDA(cudaGetLastError());
+    nbr_tables_kernel<<<NB_PAIRS, 32, 0, a.st>>>(d_sub, smin, bins, ordered, from);
+    CK_CUDA(cudaGetLastError());
+    if (n_ranges > 0) {
+        order_kernel<<<sm_count() * 8, 256, 0, a.st>>>(a.kmer_offsets, a.kmer_entries, a.kmer_targets, NB_KMERS,
+                                                       a.num_db, order);
+        CK_CUDA(cudaGetLastError());
+        frag_kernel<<<(NB_KMERS + 255) / 256, 256, 0, a.st>>>(a.kmer_offsets, a.kmer_entries, a.kmer_targets,
+                                                              a.kmer_freqs, a.freq_thresh, NB_KMERS, range, n_ranges,
+                                                              order, frag);
+        CK_CUDA(cudaGetLastError());
+        CK_CUDA(cudaFuncSetAttribute(nbr_range_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NB_RANGE * 4));
+    }
+    for (int32_t q0 = 0; q0 < a.nq; q0 += chunk) {
+        const int32_t nq = std::min(chunk, a.nq - q0);
+        const int32_t nr = nq * n_blocks;
+        int32_t *rows = counts + (size_t)q0 * a.num_db;
+        if (q0 > 0) CK_CUDA(cudaMemsetAsync(ticket, 0, 16, a.st));
+        nbr_weight_kernel<<<dim3((unsigned)n_blocks, (unsigned)nq), NB_WARPS * 32, smem, a.st>>>(
+            a.qflat, a.qflat_len, a.qoff + q0, a.qlen + q0, d_sub, smin, srange, a.score_thresh, valid, ordered, from,
+            prefixes, n, kmer, weight, listed, err);
+        CK_CUDA(cudaGetLastError());
+        if (n_ranges > 0) {
+            // about 12 units an SM, of at least one block of 5-mers, at most an
+            // eighth of them (their cuts and postings have to stay in L2)
+            const int32_t want = std::max(8, std::min(n_blocks, 12 * sm_count() / (nq * n_ranges)));
+            const int32_t set_blocks = (n_blocks + want - 1) / want;
+            nbr_range_walk_kernel<<<sm_count(), NB_RW_THREADS, (size_t)range * 4, a.st>>>(
+                n, kmer, weight, nq, n_blocks, block_kmers, set_blocks, frag, a.kmer_offsets, a.kmer_entries,
+                a.kmer_targets, a.num_db, range, n_ranges, order, rows, ticket2);
+            CK_CUDA(cudaGetLastError());
+        }
+        nbr_runs_kernel<<<1, 1024, 0, a.st>>>(n, nr, run0);
+        CK_CUDA(cudaGetLastError());
+        // one resident block per slot (8 of 256 threads per SM)
+        nbr_walk_kernel<<<8 * sm_count(), 256, 0, a.st>>>(n, run0, kmer, weight, nr, n_blocks, block_kmers,
+                                                          a.kmer_offsets, a.kmer_entries, a.kmer_targets, a.num_db,
+                                                          rows, ticket, n_ranges > 0 ? order : nullptr, err);
+        CK_CUDA(cudaGetLastError());
+    }
+    if (a.list_capacity >= 0) {
+        nbr_bound_kernel<<<1, 32, 0, a.st>>>(listed, a.list_capacity, err);
+        CK_CUDA(cudaGetLastError());
+    }
+    return CK_OK;
+}
+
 static int32_t phase_a_impl(void *pv) {
     PhaseAArgs &a = *(PhaseAArgs *)pv;
     int32_t status = CK_OK;
@@ -1210,67 +1485,7 @@ static int32_t phase_a_impl(void *pv) {
         const int8_t *d_sub = device_sub_matrix(a.sub_host, &status);
         if (!d_sub) return status;
         if (npos > 0) {
-            // the listing's cursor and the walk's chunk ticket
-            unsigned long long *cursor = (unsigned long long *)scratch(SLOT_SEARCH_TMP0, 16, &status);
-            if (!cursor) return status;
-            unsigned long long *ticket = cursor + 1;
-            const bool bounded = a.list_capacity >= 0;
-            // unbounded: the list scratch as it stands (at least 1 Mi triples); a
-            // call that lists more reads the count, grows the list past it and
-            // lists again.  bounded: the caller's capacity, no host read
-            int64_t cap = bounded ? a.list_capacity
-                                  : std::max<int64_t>((int64_t)(scratch_capacity(SLOT_SEARCH_TMP1) / 8), 1 << 20);
-            uint64_t *list = (uint64_t *)scratch(SLOT_SEARCH_TMP1, (size_t)std::max<int64_t>(cap, 1) * 8, &status);
-            if (!list) return status;
-            if (!bounded) cap = (int64_t)(scratch_capacity(SLOT_SEARCH_TMP1) / 8);
-            // a block per 8 positions of the longest query, at most
-            // NB_BLOCKS_PER_QUERY (longer queries loop; a graph captured for
-            // an arena-long query would otherwise launch mostly empty blocks):
-            // blocks start in query order, so the list fills (and the walk
-            // later runs) about one query at a time -- the walk's count-row
-            // atomics then hit L2
-            const int64_t groups = ((int64_t)npos + NB_WARPS - 1) / NB_WARPS;
-            const dim3 grid((unsigned)std::min<int64_t>(groups, NB_BLOCKS_PER_QUERY), (unsigned)a.nq);
-            int32_t smin = a.sub_host[0], smax = a.sub_host[0];
-            for (int i = 1; i < 400; ++i) {
-                smin = std::min<int32_t>(smin, a.sub_host[i]);
-                smax = std::max<int32_t>(smax, a.sub_host[i]);
-            }
-            const int32_t range = smax - smin, n_words = 160000;  // 20^4
-            const size_t smem = nbr_smem(range);
-            CK_CUDA(cudaFuncSetAttribute(nbr_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            uint32_t *valid = (uint32_t *)scratch(SLOT_SEARCH_TMP2, (size_t)n_words * 4, &status);
-            if (!valid) return status;
-            kmer_valid_kernel<<<(n_words / 32 * 32 + 255) / 256, 256, 0, a.st>>>(a.kmer_freqs, a.freq_thresh, n_words,
-                                                                                 valid);
-            CK_CUDA(cudaGetLastError());
-            int64_t listed = -1;
-            for (int pass = 0; pass < 2; ++pass) {
-                CK_CUDA(cudaMemsetAsync(cursor, 0, 8, a.st));
-                nbr_list_kernel<<<grid, NB_WARPS * 32, smem, a.st>>>(a.qflat, a.qflat_len, a.qoff, a.qlen, d_sub, smin,
-                                                                      range, a.score_thresh, valid, list, cap, cursor,
-                                                                      err);
-                CK_CUDA(cudaGetLastError());
-                if (bounded) break;
-                unsigned long long h = 0;
-                CK_CUDA(cudaMemcpyAsync(&h, cursor, 8, cudaMemcpyDeviceToHost, a.st));
-                CK_CUDA(cudaStreamSynchronize(a.st));
-                listed = (int64_t)h;
-                if (listed <= cap) break;
-                // a quarter over the count, so that the next, slightly larger
-                // batch does not list twice as well
-                list = (uint64_t *)scratch(SLOT_SEARCH_TMP1, (size_t)(listed + listed / 4) * 8, &status);
-                if (!list) return status;
-                cap = (int64_t)(scratch_capacity(SLOT_SEARCH_TMP1) / 8);
-            }
-            // the walk: one resident block per slot (8 of 256 threads per
-            // SM), fewer when the count is known to be small
-            const int64_t n_walk = listed >= 0 ? listed : cap;
-            const int64_t bw = std::max<int64_t>(1, std::min<int64_t>((int64_t)8 * sm_count(), (n_walk + 255) / 256));
-            CK_CUDA(cudaMemsetAsync(ticket, 0, 8, a.st));
-            nbr_walk_kernel<<<(unsigned)bw, 256, 0, a.st>>>(list, cursor, cap, a.nq, a.kmer_offsets, a.kmer_entries,
-                                                            a.kmer_targets, a.num_db, counts, ticket, err);
-            CK_CUDA(cudaGetLastError());
+            CK_TRY(similar_weights_and_walk(a, d_sub, counts, err));
             // the select scans the whole count row (no candidate list in this mode)
             fill_kernel<<<1, 256, 0, a.st>>>(n_cand, a.nq, CAND_CAP + 1);
             CK_CUDA(cudaGetLastError());

@@ -94,21 +94,21 @@ class Scoring:
     def graphable(self) -> bool:
         """The pipeline can run without host synchronisation: every mode, under
         a caller bound where the library would otherwise read a device count
-        (the Phase-B bins, _Slot.bins_bound; the similar-k-mer neighbour list,
-        _Slot.list_bound)."""
+        (the Phase-B bins, _Slot.bins_bound)."""
         return True
 
 
 # largest Phase-B bin buffer a slot keeps resident (int32 counters); beyond it
 # the bins are sized per call from a device count (one host synchronisation)
 BINS_CAP = 1 << 29
-# Graph-replayed similar-k-mer batches list at most LIST_RATE neighbour triples
-# per arena residue (~5,000 per residue is typical at threshold 13 on a 500k
-# database, and arenas hold ~5x the residues of a typical batch); a batch that
-# lists more is run again call by call.  LIST_CAP bounds the list (8 bytes a
-# triple).
+# Graph-replayed similar-k-mer batches score at most LIST_RATE (query position,
+# 5-mer) pairs per arena residue (~5,000 per residue is typical at threshold 13
+# on a 500k database, and arenas hold ~5x the residues of a typical batch); a
+# batch that has more is run again call by call.  LIST_CAP bounds the product.
 LIST_RATE = 2048
 LIST_CAP = 1 << 28
+# targets per range of the similar-k-mer posting walk (csrc/search.cu: NB_RANGE)
+RANGE_TARGETS = 56 * 1024
 
 
 def _torch():
@@ -320,8 +320,8 @@ class _Slot:
         return bound if bound <= BINS_CAP else -1
 
     def list_bound(self, res_bytes: int) -> int:
-        """The caller bound on a similar-k-mer batch's neighbour triples
-        (LIST_RATE per residue of the slot arena); -1 when above LIST_CAP."""
+        """The caller bound on a similar-k-mer batch's (query position, 5-mer)
+        pairs (LIST_RATE per residue of the slot arena); -1 when above LIST_CAP."""
         bound = int(res_bytes) * LIST_RATE
         return bound if bound <= LIST_CAP else -1
 
@@ -337,9 +337,7 @@ class _Slot:
                  ctx: int | None = None):
         """The device pipeline of a batch of nq queries on this slot's stream:
         H2D, k-mer scoring, pair list, SW, D2H.  ``bounded``: the similar-k-mer
-        neighbour list under the slot's list bound, so that no step reads a
-        device count on the host and the pipeline can be captured in a CUDA
-        graph.  ``ctx``: a library context other than the slot's."""
+        pairs under the slot's list bound.  ``ctx``: a library context other than the slot's."""
         torch = _torch()
         db = self.db
         K = self.max_cands
@@ -454,8 +452,8 @@ class _Slot:
 
     def _rerun_unbounded(self):
         """The batch in flight again, call by call in the slot's spare context
-        (unfrozen, so its neighbour list can grow): a replayed batch whose
-        listing passed the slot's list bound.  The pinned inputs still hold
+        (without a bound): a replayed batch whose similar-k-mer pairs passed
+        the slot's list bound.  The pinned inputs still hold
         the batch; the outputs land in the same buffers."""
         torch = _torch()
         if not self.ctx_spare:
@@ -735,8 +733,10 @@ class SearchServer:
         sc = Scoring(int(min_total_hits), self.kmer_score_thresh, **scoring)
         if sc.diagonal:  # Phase B: target -> selection row, selection and bin offsets
             per_slot += db.arena_queries * (db.n * 4 + min(sc.phase_a_topk, db.n) * 16)
-        if sc.similar and use_graphs:  # the bounded neighbour list (8 bytes a triple)
-            per_slot += max(0, db.arena_residues * LIST_RATE) * 8
+        if sc.similar:
+            # the queries' summed 5-mer scores (6 bytes each, 64 queries at a time) and each 5-mer's list cut
+            # at the target ranges of the posting walk (8 bytes a cut)
+            per_slot += min(db.arena_queries, 64) * 58 * 56000 * 6 + -(-db.n // RANGE_TARGETS) * 20 ** 5 * 8
         n_slots = int(max(1, min(db.slots, (free // 2) // max(per_slot, 1))))
         self.slots = [_Slot(db, i, max_cands) for i in range(n_slots)]
         self.free = list(self.slots)

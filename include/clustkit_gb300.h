@@ -361,14 +361,13 @@ int32_t ck_lsh_candidates_device(int32_t ctx, const uint64_t *d_sketches, int64_
  * (k-mers with frequency 0 or above freq_thresh skipped); sums are int32, not
  * saturated; survivors and cap as above.  d_kmer_targets (may be NULL) as
  * in ck_search_phase_a_device.
- * The (query, 5-mer, score) triples are listed once into a device list that
- * the posting walk then reads.  list_capacity < 0: the library sizes that
- * list from its scratch, reads the count on the host (blocking) and, when it
- * was too small, grows it and lists again.  list_capacity >= 0: at most that
- * many triples (8 bytes each in the context's scratch), no host
- * synchronisation (the call can be captured in a CUDA graph); a call that
- * lists more walks only the first list_capacity and the next status check
- * reports CK_ERR_CAPACITY. */
+ * The scores are summed per query and 5-mer first; the posting walk then reads
+ * those sums (6 bytes a 5-mer in the context's scratch, for at most 64 queries
+ * at a time, and, for calls of several queries, 25.6 MB for every 57,344
+ * targets).  No host synchronisation (the call can be captured in a CUDA
+ * graph).  list_capacity >= 0 bounds the (query position, 5-mer) pairs at or
+ * above the threshold: a call with more reports CK_ERR_CAPACITY at the next
+ * status check; < 0: no bound. */
 int32_t ck_search_phase_a_similar_device(int32_t ctx, const uint8_t *d_qflat, int64_t qflat_len,
                                          const int64_t *d_qoffsets, const int32_t *d_qlengths, int32_t nq,
                                          int32_t max_qlen, const int8_t *sub_matrix_host,

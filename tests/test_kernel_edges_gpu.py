@@ -79,3 +79,100 @@ def test_lsh_repeated_tables(ck, tables, bands, size):
     assert tables == 1 or len(np.unique(idx, axis=0)) < tables
     got = lsh_candidates_device(sk, tables, bands, 5).cpu().numpy()
     assert np.array_equal(got, lsh_candidates(sk, tables, bands, 5))
+
+
+def _similar(db, qs, top_k, sub, thresh, entries=None, compact=True, list_capacity=-1):
+    """ck_search_phase_a_similar_device in the default context: rows of (ids, scores)."""
+    import torch
+    from clustkit_gb300 import _lib
+    lib, nq = db.lib, len(qs)
+    lens = np.array([len(q) for q in qs], np.int32)
+    offs = (np.cumsum(lens) - lens).astype(np.int64)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_q, d_off, d_len = dev(np.concatenate(qs).astype(np.uint8)), dev(offs), dev(lens)
+    d_ent = db.d_kmer_entries if entries is None else dev(entries)
+    d_tgt = dev((d_ent.cpu().numpy() >> 32).astype(np.int32)) if compact else None
+    out_t = torch.zeros(nq * top_k, dtype=torch.int32, device="cuda")
+    out_s, out_n = torch.zeros_like(out_t), torch.zeros(nq, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.ck_search_phase_a_similar_device(
+        0, d_q.data_ptr(), int(lens.sum()), d_off.data_ptr(), d_len.data_ptr(), nq, int(lens.max()), sub.ctypes.data,
+        thresh, db.d_kmer_offsets.data_ptr(), d_ent.data_ptr(), d_tgt.data_ptr() if compact else None,
+        db.d_kmer_freqs.data_ptr(), db.freq_thresh, db.n, 2, top_k, out_t.data_ptr(), out_s.data_ptr(),
+        out_n.data_ptr(), list_capacity, st))
+    _lib.check(lib.ck_ctx_status(0, st))
+    n, t, s = out_n.cpu().numpy(), out_t.cpu().numpy().reshape(nq, -1), out_s.cpu().numpy().reshape(nq, -1)
+    return [(t[q, :n[q]], s[q, :n[q]]) for q in range(nq)]
+
+
+def _matrix(kind):
+    from clustkit_gb300.blosum import BLOSUM62
+    if kind == "blosum":
+        return np.ascontiguousarray(BLOSUM62, np.int8)
+    if kind == "flat":  # one score: no bins between the least and the most
+        return np.full((20, 20), 3, np.int8)
+    return np.random.default_rng(3).integers(-128, 128, (20, 20)).astype(np.int8)  # every int8 score
+
+
+@pytest.fixture(scope="module")
+def small_db():
+    from clustkit_gb300.search import DeviceDatabase
+    ss = synth.generate_families(300, 4, median=120, lo=3, hi=300, seed=4)
+    return DeviceDatabase(ss.flat, ss.offsets, ss.lengths, arena_queries=8, arena_residues=8 * 400), ss
+
+
+@pytest.mark.parametrize("kind,thresh", [("blosum", 13), ("blosum", 3), ("blosum", 60), ("flat", 15), ("flat", 16),
+                                         ("wide", 330), ("wide", 636)])
+def test_similar_listing(ck, small_db, kind, thresh):
+    """Every 5-mer at or above the threshold, for matrices of the least and the
+    largest score range and thresholds that most, few and no 5-mers reach."""
+    db, ss = small_db
+    off, ent, fr = db.index_arrays()
+    sub = _matrix(kind)
+    rng = np.random.default_rng(9)
+    qs = [ss.seq(7)[:5].copy(), np.zeros(4, np.uint8), np.full(12, 18, np.uint8),  # 18: a large diagonal score
+          np.concatenate([ss.seq(40)[:20], [20], ss.seq(41)[:11]]).astype(np.uint8),
+          rng.integers(0, 20, 9).astype(np.uint8)]
+    if thresh > 10:
+        qs.append(ss.seq(100).copy())
+    for part in (qs, qs[:1]):
+        lens = np.array([len(q) for q in part], np.int32)
+        offs = (np.cumsum(lens) - lens).astype(np.int64)
+        want = oracle.similar_candidates_batch(np.concatenate(part), offs, lens, sub, thresh, off, ent, fr,
+                                               db.freq_thresh, db.n, 2, 50)
+        got = _similar(db, part, 50, sub, thresh)
+        for g, w in zip(got, want):
+            assert np.array_equal(g[0], w[0]) and np.array_equal(g[1], w[1])
+
+
+@pytest.mark.parametrize("n_db,shuffled,compact", [(57344, False, True), (57345, False, True), (57345, False, False),
+                                                   (120001, False, True), (120001, True, True), (1, False, True)])
+def test_similar_target_ranges(ck, n_db, shuffled, compact):
+    """The posting walk by target ranges: one range that is just full, two,
+    three, one target; and lists that are not in target order, which it leaves
+    to the walk on the count rows."""
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.search import DeviceDatabase
+    rng = np.random.default_rng(n_db)
+    lens = rng.integers(5, 14, n_db).astype(np.int32)
+    off = (np.cumsum(lens) - lens).astype(np.int64)
+    flat = rng.integers(0, 20, int(lens.sum())).astype(np.uint8)
+    db = DeviceDatabase(flat, off, lens, arena_queries=8, arena_residues=8 * 400)
+    koff, ent, fr = db.index_arrays()
+    if shuffled:  # each list's entries reversed
+        at = np.repeat(koff[:-1] + koff[1:] - 1, np.diff(koff)) - np.arange(len(ent))
+        ent = ent[at]
+    qs = [flat[off[i]:off[i] + lens[i]].copy() for i in (0, n_db // 2, n_db - 1)]
+    qs += [rng.integers(0, 20, 150).astype(np.uint8), np.zeros(3, np.uint8)]
+    sub = _matrix("blosum")
+    qlen = np.array([len(q) for q in qs], np.int32)
+    qoff = (np.cumsum(qlen) - qlen).astype(np.int64)
+    want = oracle.similar_candidates_batch(np.concatenate(qs), qoff, qlen, sub, 13, koff, ent, fr, db.freq_thresh,
+                                           n_db, 2, 300)
+    for cap in (-1, 4_000_000):
+        got = _similar(db, qs, 300, sub, 13, entries=ent, compact=compact, list_capacity=cap)
+        for g, w in zip(got, want):
+            assert np.array_equal(g[0], w[0]) and np.array_equal(g[1], w[1])
+    with pytest.raises(_lib.CkError) as e:
+        _similar(db, qs, 300, sub, 13, entries=ent, compact=compact, list_capacity=10)
+    assert e.value.status == _lib.CK_ERR_CAPACITY
