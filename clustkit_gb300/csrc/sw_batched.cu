@@ -352,31 +352,32 @@ __device__ __forceinline__ void strip_cells(uint32_t bcol, int32_t &hu, int32_t 
         const int32_t eR = __viaddmax_s32(hu, OPEN_E, fadd(eu, K::EXT, one));
         int32_t fTn = __viaddmax_s32(S.fT[r], K::EXT, fadd(S.hc[r], OPEN_F, one));
         if constexpr (!K::COMPACT) fTn |= TBIT;
-        const int32_t hn = __vimax3_s32(diagc, eR, fTn) & K::CLEAN;
+        int32_t hn = __vimax3_s32(diagc, eR, fTn) & K::CLEAN;
         int32_t en;
         if constexpr (K::COMPACT) en = (r % 6 == 5 || r == R - 1) ? (eR & ~K::CTR) : eR;
         else en = eR | TBIT;
         hdiag = S.hc[r];
         if constexpr (MASKED) {
             // A row outside its band at this column (bit r of rmask clear) is
-            // computed like the others and its results dropped by selects (no
-            // branch: the lanes of a warp are at different columns of their
-            // strips): a row that has not reached its band keeps H = 0 and its
-            // F; a row that has left it hands the out-of-band boundary (H = 0,
-            // E = -inf) to the row below and its last H as that row's diagonal
-            // input (hdiag above, as for a row inside its band).
-            const bool inb = (rmask >> r) & 1u;
-            const int32_t hs = inb ? hn : 0;
-            S.hc[r] = hs;
-            S.fT[r] = inb ? fTn : S.fT[r];
-            hu = hs;
-            eu = inb ? en : K::NEG_E;
-        } else {
-            S.hc[r] = hn;
-            S.fT[r] = fTn;
-            hu = hn;
-            eu = en;
+            // computed like the others and its results dropped (no branch: the
+            // lanes of a warp are at different columns of their strips) by an
+            // AND with its bit spread over the word, which the three-input
+            // logic op that clears H's low fields does on the way.  H = 0 is
+            // the boundary on every side.  E = 0 stands in for the boundary's
+            // -inf: the row below extends it to a negative E, which never
+            // reaches an H (zero wins ties) and is below any opening that
+            // does.  F needs nothing: over H = 0 it stays at a gap opening,
+            // which is what the first column in the band computes anyway.  A
+            // row that has left its band hands its last H on as the next row's
+            // diagonal input (hdiag above), as a row inside does.
+            const int32_t in = (int32_t)(rmask << (31 - r)) >> 31;
+            hn &= in;
+            en &= in;
         }
+        S.hc[r] = hn;
+        S.fT[r] = fTn;
+        hu = hn;
+        eu = en;
     }
 }
 
@@ -1230,7 +1231,7 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
         }
         __syncwarp();
         ++T;
-        if (__all_sync(FULL, exhausted && cur_slot < 0 && pend_slot < 0)) break;
+        if (exhausted && __all_sync(FULL, cur_slot < 0 && pend_slot < 0)) break;
     }
 }
 
