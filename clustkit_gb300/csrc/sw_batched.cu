@@ -359,20 +359,19 @@ __device__ __forceinline__ void strip_cells(uint32_t bcol, int32_t &hu, int32_t 
         hdiag = S.hc[r];
         if constexpr (MASKED) {
             // A row outside its band at this column (bit r of rmask clear) is
-            // computed like the others and its results dropped (no branch: the
-            // lanes of a warp are at different columns of their strips) by an
-            // AND with its bit spread over the word, which the three-input
-            // logic op that clears H's low fields does on the way.  H = 0 is
-            // the boundary on every side.  E = 0 stands in for the boundary's
-            // -inf: the row below extends it to a negative E, which never
-            // reaches an H (zero wins ties) and is below any opening that
-            // does.  F needs nothing: over H = 0 it stays at a gap opening,
-            // which is what the first column in the band computes anyway.  A
-            // row that has left its band hands its last H on as the next row's
-            // diagonal input (hdiag above), as a row inside does.
-            const int32_t in = (int32_t)(rmask << (31 - r)) >> 31;
-            hn &= in;
-            en &= in;
+            // computed like the others and its H dropped (no branch: the lanes
+            // of a warp are at different columns of their strips) by an AND
+            // with its bit spread over the word, which the three-input logic op
+            // that clears H's low fields does on the way.  H = 0 is the boundary
+            // on every side.  E and F need nothing.  Below rows that have left
+            // the band, E comes from H = 0 and, at the strip's top, from the
+            // boundary the caller passes, so it is negative and never reaches
+            // an H; below rows that have not reached it there are only such
+            // rows.  F over H = 0 stays at a gap opening, which is what the
+            // first column in the band computes anyway.  A row that has left
+            // its band hands its last H on as the next row's diagonal input
+            // (hdiag above), as a row inside does.
+            hn &= (int32_t)(rmask << (31 - r)) >> 31;
         }
         S.hc[r] = hn;
         S.fT[r] = fTn;
@@ -737,24 +736,27 @@ __device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &ou
                                                  int32_t *fallback, int32_t *fallback_count,
                                                  int32_t *err, int32_t one, int32_t wide_key);
 struct WaveSlot;
-__device__ __noinline__ void wave_stream_any(int32_t rows, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                             int32_t n_wave, int32_t *ticket, const char *s_inc, int32_t *s_best,
-                                             WaveSlot *slots, int32_t lane, int32_t *fallback,
-                                             int32_t *fallback_count, int32_t *err, int32_t one, int32_t compact);
+__device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
+                                             int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
+                                             int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
+                                             int32_t one, int32_t compact);
 
 // Persistent alignment kernel.  Its warps first take the leading
 // counters[6] sorted pairs one warp per pair (long pairs, or every pair of a
 // small call), then the rest 32 pairs per warp, one lane per pair, in
 // register strips of R rows.  Long pairs thus start first and the lane-per-
-// pair groups fill in around them.
+// pair groups fill in around them.  Each warp's (or group's) first warp-per-pair
+// pair is dealt to it, block by block, and a ticket gives the later ones: by
+// ticket alone the warps of the first block to start took the longest pairs
+// together, and a small call's pairs filled a fifth of the SMs (500 pairs: DEAL).
 template <int R, int V, int NT>
 __global__ void __launch_bounds__(NT, 1)
 sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
                 const int32_t *__restrict__ counters, const int32_t *__restrict__ inc_global,
                 int2 *__restrict__ window, int32_t W, int32_t *__restrict__ ticket,
                 int32_t *__restrict__ wave_ticket, int32_t *__restrict__ fallback,
-                int32_t *__restrict__ fallback_count, int32_t *err, int32_t one, int32_t wave_rows,
-                int32_t wave_rows_force, int32_t wide_key) {
+                int32_t *__restrict__ fallback_count, int32_t *err, int32_t one, int32_t wave_shape,
+                int32_t wave_force, int32_t wide_key) {
     extern __shared__ int32_t s_inc[];
     if (counters[0] <= 0) return;
     for (int t = threadIdx.x; t < INC_ENTRIES * 32; t += blockDim.x) s_inc[t] = inc_global[t >> 5];
@@ -766,7 +768,7 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
     // warps (each warp then sees several); with fewer, one pair per warp at the
     // rows per strip each pair allows has the shorter wavefronts
     const int32_t n_warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
-    if (wave_rows > 0 && (wave_rows_force || n_wave > n_warps)) {
+    if (wave_shape > 0 && (wave_force || n_wave > n_warps)) {
         // slots behind the increment table and the per-row trackers
         char *slot_base = (char *)(s_inc + INC_ENTRIES * 32 + track_rows<R>() * NT);
         WaveSlot *slots = (WaveSlot *)(slot_base + (size_t)(threadIdx.x >> 5) * WAVE_SLOTS_PER_WARP *
@@ -774,18 +776,16 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
         // the compact key when every pair of the call (so every warp-per-pair
         // pair) has at most 2047 rows
         if (n_wave > 0)
-            wave_stream_any(wave_rows, in, out, order, n_wave, wave_ticket, (const char *)s_inc, s_best, slots,
-                            lane, fallback, fallback_count, err, one,
-                            !wide_key && counters[8] <= KeyCompact::ROWS_MAX);
+            wave_stream_any(wave_shape, in, out, order, n_wave, wave_ticket, (const char *)s_inc, slots, lane,
+                            fallback, fallback_count, err, one, !wide_key && counters[8] <= KeyCompact::ROWS_MAX);
     } else {
-        for (;;) {
-            __syncwarp();
-            int32_t q = 0;
-            if (lane == 0) q = atomicAdd(wave_ticket, 1);
-            q = __shfl_sync(0xffffffffu, q, 0);
+        for (int32_t q = (int32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);;) {
             if (q >= n_wave) break;
             align_pair_wave_any(in, out, (int64_t)order[q], (const char *)s_inc, s_best, lane, fallback,
                                 fallback_count, err, one, wide_key);
+            __syncwarp();
+            if (lane == 0) q = n_warps + atomicAdd(wave_ticket, 1);
+            q = __shfl_sync(0xffffffffu, q, 0);
         }
     }
     const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -980,19 +980,27 @@ __device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &ou
 
 // ----------------------------------------------------------------- streamed warp-per-pair
 // The warp-per-pair phase with the strips of consecutive pairs streamed
-// through one warp, so that lanes freed by one pair's strips take the next
-// pair's instead of idling while the pair's wavefront fills and drains.  All
-// pairs of the call share R (chosen from the band width so every pair can
-// rotate).  Strips carry one global sequence number g; lane g mod 32 runs
-// strip g.  Strip s of a pair starting at T0 runs column j at step
-// T0 + s + j - J0(strip 0), i.e. exactly one step behind its upstream strip
-// s - 1 at every column, so the (H, E) hand-over by shuffle works as in the
-// single-pair schedule.  A pair is issued (one per step, once every strip
-// of the previous one has started) with the smallest T0 at which each of its
-// first 32 strips finds its lane free; its later strips rotate through the
-// same lanes as before.  A lane's strip whose upstream lane belongs to
+// through G lanes, so that lanes freed by one pair's strips take the next
+// pair's instead of idling while the pair's wavefront fills and drains.  A warp
+// holds 32 / G such groups, each with its own pairs; a step is one column of
+// every lane's strip.  Strips carry one sequence number g in their group; lane
+// g mod G of it runs strip g.  Strip s of a pair starting at T0 runs column j
+// at step T0 + s + j - J0(strip 0), i.e. exactly one step behind its upstream
+// strip s - 1 at every column, so the (H, E) hand-over by shuffle works as in
+// the single-pair schedule.  A pair is issued (one per group and step, once
+// every strip of the previous one has started) with the smallest T0 at which
+// each of its first G strips finds its lane free; its later strips rotate
+// through the same lanes.  A lane's strip whose upstream lane belongs to
 // another pair or strip reads the out-of-band boundary instead (overrides
 // below), so a lane never reads a neighbour's unrelated values.
+//
+// G and the strip height R are shared by all pairs of a call (wave_shape).  A
+// strip of a band of half-width w lives 2w + R steps and its pair's next starts
+// R + 1 steps later, so about (2w + R) / (R + 1) lanes of a group work on a
+// pair: at w = 50, 21 lanes of 32 with the 4 rows that 32 lanes need to rotate
+// there, but 7 lanes of 8 with 16 rows -- and what a step costs beside its
+// cells (about 100 instructions) is spread over 16 rows a lane instead of 4.
+// 12,000 pairs at band 50: SMALL_NOTE.
 //
 // Per pair, a slot in shared memory holds its geometry, the running best
 // score (first-maximum trigger; each lane compares with its own copy, taken
@@ -1000,8 +1008,11 @@ __device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &ou
 // the slot's, so a copy that lags only adds trigger steps) and the best cell
 // as one packed 64-bit value
 // (score, then lower row, then match count), merged by atomicMax at each
-// strip's end; the pair's last strip ends last and writes the result.
-constexpr int WS_SLOTS = 16;
+// strip's end; the pair's last strip ends last and writes the result.  Within
+// a strip a lane holds its best cell in registers: on a trigger, the column's
+// lowest row with its best score replaces it when it scores more, or as much
+// in a lower row (a later column of the same row does not).
+constexpr int WS_SLOTS = WAVE_SLOTS_PER_WARP;
 
 struct WaveSlot {
     unsigned long long acc;   // score << 27 | (16383 - row) << 13 | matches
@@ -1013,7 +1024,6 @@ struct WaveSlot {
 };
 
 static_assert(sizeof(WaveSlot) == WAVE_SLOT_BYTES, "slot layout");
-static_assert(WS_SLOTS == WAVE_SLOTS_PER_WARP, "slot count");
 
 template <int R>
 __device__ __forceinline__ void strip_bounds(const WaveSlot &sl, int32_t s, int32_t &i0, int32_t &lo,
@@ -1041,16 +1051,24 @@ __device__ __forceinline__ int32_t strip_te(const WaveSlot &sl, int32_t s) {
     return te > t0 ? te : t0;  // a strip whose band lies left of column 1 ends where it starts
 }
 
-template <int R, class K>
+template <int R, int G, class K>
 __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *order, int32_t n_wave,
-                            int32_t *ticket, const char *s_inc, int32_t *s_best, WaveSlot *slots, int32_t lane,
+                            int32_t *ticket, const char *s_inc, WaveSlot *warp_slots, int32_t lane,
                             int32_t *fallback, int32_t *fallback_count, int32_t *err, int32_t one) {
     using namespace key;
     constexpr uint32_t FULL = 0xffffffffu;
-    // warp-uniform schedule state
+    constexpr int SLOTS = WS_SLOTS * G / 32;  // of a group
+    const int32_t gl = lane & (G - 1), g0 = lane - gl;  // lane of its group, the group's first lane
+    const uint32_t gmask = G == 32 ? FULL : ((1u << (G & 31)) - 1u) << g0;
+    const int32_t up = g0 | ((gl + G - 1) & (G - 1));   // the upstream lane
+    WaveSlot *slots = warp_slots + lane / G * SLOTS;
+    // first pairs: dealt out over the blocks, then over a block's groups
+    const int32_t groups = (int32_t)(blockDim.x / G), n_first = groups * (int32_t)gridDim.x;
+    int32_t first_q = (int32_t)(threadIdx.x / G * gridDim.x + blockIdx.x);
+    // schedule state, the same for every lane of a group (T for the warp)
     int32_t T = 0, T_issue = -1, g_next = 0, seq = 0;
     bool exhausted = false;
-    for (int i = lane; i < WS_SLOTS; i += 32) slots[i].live = 0;
+    for (int i = lane; i < WS_SLOTS; i += 32) warp_slots[i].live = 0;
     __syncwarp();
     // per-lane strip state
     int32_t cur_slot = -1, cur_s = 0, i0 = 0, lo0 = 0, J0 = 1, J1 = 0, alive = 0, te = 0, top = 0;
@@ -1063,14 +1081,18 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
     // the held strip's pair's running best score as last seen by this lane: at
     // most the slot's, so its trigger fires at least whenever the slot's would
     int32_t gs_l = 1;
+    int32_t best = 0, best_r = 0;  // the strip's best cell so far: H, row of the strip
     const uint8_t *B = nullptr;
     StripRegs<R> S;
     for (;;) {
-        // ---- issue one pair (warp-uniform)
-        if (!exhausted && T > T_issue && !slots[seq % WS_SLOTS].live) {
-            int32_t q = 0;
-            if (lane == 0) q = atomicAdd(ticket, 1);
-            q = __shfl_sync(FULL, q, 0);
+        // ---- issue one pair (the same for every lane of the group)
+        if (!exhausted && T > T_issue && !slots[seq % SLOTS].live) {
+            int32_t q = first_q;
+            if (first_q < 0) {
+                if (gl == 0) q = n_first + atomicAdd(ticket, 1);
+                q = __shfl_sync(gmask, q, g0);
+            }
+            first_q = -1;
             if (q >= n_wave) {
                 exhausted = true;
             } else {
@@ -1083,21 +1105,21 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                     if (s_lim < n_strips) n_strips = (int32_t)s_lim;
                 }
                 if (n_strips <= 0) {
-                    if (lane == 0) write_result(out, in, p, 0, 0, g.la, g.la, g.lb);
+                    if (gl == 0) write_result(out, in, p, 0, 0, g.la, g.la, g.lb);
                 } else {
-                    WaveSlot &sl = slots[seq % WS_SLOTS];
+                    WaveSlot &sl = slots[seq % SLOTS];
                     const int32_t c0 = 1 + g.h - g.w;
                     const int32_t J00 = c0 > 1 ? c0 : 1;
-                    const int32_t m = (lane - g_next) & 31;
-                    const int32_t first = n_strips < 32 ? n_strips : 32;
+                    const int32_t m = (gl - g_next) & (G - 1);
+                    const int32_t first = n_strips < G ? n_strips : G;
                     int32_t req = T;
                     if (m < first) {
                         const int32_t lom = m * R + c0;
                         const int32_t r = F + 1 - m - ((lom > 1 ? lom : 1) - J00);
                         req = r > T ? r : T;
                     }
-                    const int32_t T0p = __reduce_max_sync(FULL, req);
-                    if (lane == 0) {
+                    const int32_t T0p = __reduce_max_sync(gmask, req);
+                    if (gl == 0) {
                         sl.acc = 0;
                         sl.a_off = in.offsets[g.a_idx];
                         sl.b_off = in.offsets[g.b_idx];
@@ -1105,12 +1127,12 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                         sl.la = g.la; sl.lb = g.lb; sl.w = g.w; sl.h = g.h; sl.c0 = c0;
                         sl.S = n_strips; sl.J00 = J00; sl.T0 = T0p; sl.gs = 1; sl.live = 1;
                     }
-                    __syncwarp();
+                    __syncwarp(gmask);
                     if (m < first) {
-                        pend_slot = seq % WS_SLOTS;
+                        pend_slot = seq % SLOTS;
                         pend_s = m;
                         pend_t0 = strip_t0<R>(sl, m);
-                        const int32_t last = m + 32 * ((n_strips - 1 - m) / 32);
+                        const int32_t last = m + G * ((n_strips - 1 - m) / G);
                         F = strip_te<R>(sl, last);
                     }
                     T_issue = strip_t0<R>(sl, n_strips - 1);
@@ -1120,8 +1142,8 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             }
         }
         // ---- start this lane's next strip.  Its start step is never in the past
-        // (the rotation bound on R); were it, the strip starts now and the call
-        // reports an internal error rather than the warp waiting forever.
+        // (the rotation bound, wave_shape); were it, the strip starts now and the
+        // call reports an internal error rather than the warp waiting forever.
         if (pend_slot >= 0 && T >= pend_t0) {
             if (T > pend_t0) atomicOr(err, ERRBIT_SCHEDULE);
             const WaveSlot &sl = slots[pend_slot];
@@ -1129,6 +1151,7 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             cur_s = pend_s;
             pend_slot = -1;
             gs_l = sl.gs;
+            best = 0;
             strip_bounds<R>(sl, cur_s, i0, lo0, J0, J1, alive);
             te = strip_te<R>(sl, cur_s);
             if (te < T) te = T;  // only after a late start: the strip still ends
@@ -1142,14 +1165,14 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             for (int r = 0; r < R; ++r) {
                 S.hc[r] = 0;
                 S.fT[r] = K::NEG_F;
-                s_best[r * 32] = 0;
                 const uint32_t code = r < alive ? (uint32_t)A[i0 + r - 1] : 0u;
                 S.arow[r] = (code * (uint32_t)N_CODES * 32u + (uint32_t)lane) * 4u;
             }
         }
+        __syncwarp();
         // ---- one column of this lane's strip
-        int32_t hin = __shfl_sync(FULL, hout, (lane + 31) & 31);
-        int32_t ein = __shfl_sync(FULL, eout, (lane + 31) & 31);
+        int32_t hin = __shfl_sync(FULL, hout, up);
+        int32_t ein = __shfl_sync(FULL, eout, up);
         int32_t cm = 0;
         const bool has = cur_slot >= 0;
         int32_t j = 0;
@@ -1184,31 +1207,36 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                 for (int r = 0; r < R; ++r) S.fT[r] &= ~K::CTR;
             }
         }
-        // ---- first-maximum trackers: per-pair running best score
-        const bool trig = has && (cm >> 16) >= gs_l;
-        if (__any_sync(FULL, trig)) {
-            if (has) {
+        // ---- first maximum: a column that reaches the pair's running best score
+        if (has && (cm >> 16) >= gs_l) {
+            const int32_t floor = cm & ~(KU - 1);
+            int32_t v = 0, vr = 0;
+            if constexpr (K::COMPACT) {
+                // the row rides in the four bits above the match count, clear
+                // in H: one maximum finds the lowest row with the best score
+                v = S.hc[0] + ((R - 1) << 12);
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int32_t b = s_best[r * 32];
-                    if (S.hc[r] > (b | (KU - 1))) s_best[r * 32] = S.hc[r];
+                for (int r = 1; r < R; r += 2) {
+                    const int32_t a = S.hc[r] + ((R - 1 - r) << 12);
+                    v = r + 1 < R ? __vimax3_s32(v, a, S.hc[r + 1] + ((R - 2 - r) << 12)) : max(v, a);
                 }
-                if (cm > 0) gs_l = max(atomicMax(&slots[cur_slot].gs, cm >> 16), cm >> 16);
-            }
-        }
-        // ---- strip end: merge its rows into the pair's best; the last strip writes
-        if (has && T == te) {
-            int32_t bk = 0, br = 0;
+                vr = R - 1 - ((v >> 12) & 15);
+                v &= ~(15 << 12);
+            } else {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int32_t b = s_best[r * 32];
-                if (r < alive && b > (bk | (KU - 1))) { bk = b; br = i0 + r; }
+                for (int r = R - 1; r >= 0; --r)
+                    if (S.hc[r] >= floor) { v = S.hc[r]; vr = r; }  // ends at the lowest such row
             }
+            if (floor > (best & ~(KU - 1)) || ((best >> 16) == (cm >> 16) && vr < best_r)) { best = v; best_r = vr; }
+            gs_l = max(atomicMax(&slots[cur_slot].gs, cm >> 16), cm >> 16);
+        }
+        // ---- strip end: its best cell into the pair's; the last strip writes
+        if (has && T == te) {
             WaveSlot &sl = slots[cur_slot];
-            if (bk > 0)
-                atomicMax(&sl.acc, ((unsigned long long)(uint32_t)(bk >> 16) << 27) |
-                                       ((unsigned long long)(uint32_t)(16383 - br) << 13) |
-                                       (unsigned long long)(uint32_t)(bk & K::MATCH_MASK));
+            if (best > 0)
+                atomicMax(&sl.acc, ((unsigned long long)(uint32_t)(best >> 16) << 27) |
+                                       ((unsigned long long)(uint32_t)(16383 - (i0 + best_r)) << 13) |
+                                       (unsigned long long)(uint32_t)(best & K::MATCH_MASK));
             if (cur_s == sl.S - 1) {
                 __threadfence_block();
                 const unsigned long long acc = atomicAdd(&sl.acc, 0ull);
@@ -1222,41 +1250,42 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                                  sl.lb);
                 }
                 sl.live = 0;
-            } else if (cur_s + 32 < sl.S) {
+            } else if (cur_s + G < sl.S) {
                 pend_slot = cur_slot;
-                pend_s = cur_s + 32;
+                pend_s = cur_s + G;
                 pend_t0 = strip_t0<R>(sl, pend_s);
             }
             cur_slot = -1;
         }
         __syncwarp();
         ++T;
-        if (exhausted && __all_sync(FULL, cur_slot < 0 && pend_slot < 0)) break;
+        if (__all_sync(FULL, exhausted && cur_slot < 0 && pend_slot < 0)) break;
     }
 }
 
 template <class K>
-__device__ __forceinline__ void wave_stream_k(int32_t rows, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                              int32_t n_wave, int32_t *ticket, const char *s_inc, int32_t *s_best,
-                                              WaveSlot *slots, int32_t lane, int32_t *fallback,
-                                              int32_t *fallback_count, int32_t *err, int32_t one) {
-    switch (rows) {
-        case 4: wave_stream<4, K>(in, out, order, n_wave, ticket, s_inc, s_best, slots, lane, fallback, fallback_count, err, one); break;
-        case 8: wave_stream<8, K>(in, out, order, n_wave, ticket, s_inc, s_best, slots, lane, fallback, fallback_count, err, one); break;
-        default: wave_stream<16, K>(in, out, order, n_wave, ticket, s_inc, s_best, slots, lane, fallback, fallback_count, err, one); break;
+__device__ __forceinline__ void wave_stream_k(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
+                                              int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
+                                              int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
+                                              int32_t one) {
+    switch (shape) {
+        case 8 << 8 | 8: wave_stream<8, 8, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 16 << 8 | 8: wave_stream<16, 8, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 16 << 8 | 16: wave_stream<16, 16, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        default: wave_stream<16, 32, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
     }
 }
 
-__device__ __noinline__ void wave_stream_any(int32_t rows, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                             int32_t n_wave, int32_t *ticket, const char *s_inc, int32_t *s_best,
-                                             WaveSlot *slots, int32_t lane, int32_t *fallback,
-                                             int32_t *fallback_count, int32_t *err, int32_t one, int32_t compact) {
+__device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
+                                             int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
+                                             int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
+                                             int32_t one, int32_t compact) {
     if (compact)
-        wave_stream_k<KeyCompact>(rows, in, out, order, n_wave, ticket, s_inc, s_best, slots, lane, fallback,
-                                  fallback_count, err, one);
+        wave_stream_k<KeyCompact>(shape, in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count,
+                                  err, one);
     else
-        wave_stream_k<KeyWide>(rows, in, out, order, n_wave, ticket, s_inc, s_best, slots, lane, fallback,
-                               fallback_count, err, one);
+        wave_stream_k<KeyWide>(shape, in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count,
+                               err, one);
 }
 
 // ----------------------------------------------------------------- driver
@@ -1285,19 +1314,25 @@ static int32_t g_wave_adaptive = 1;
 // stream the strips of consecutive pairs through a warp: 1 when the call has
 // more warp-per-pair pairs than warps, 2 always, 0 never
 static int32_t g_wave_stream = 1;
-// rows per strip of the streamed schedule: 0 = the smallest that rotates,
-// else 4, 8 or 16 when at least that (taller strips rotate a fortiori)
+// rows per strip of the streamed schedule: 0 = by band width, else at least
+// that many (4, 8 or 16)
 static int32_t g_wave_rows = 0;
 
-// Rows per strip shared by every warp-per-pair pair of a call: the smallest
-// that lets a strip of any of them rotate through 32 lanes (half-widths up to
-// max(band width, 50); with a wider band every pair has at most 512 rows, as
-// the routing guarantees, so 16 rows give at most 32 strips).  0: one pair
-// per warp at a time.
-static int32_t wave_rows_for(int32_t wmax) {
+// Rows per strip R and lanes per group G (as R << 8 | G) of the streamed
+// schedule, for band half-widths up to w.  A lane may start its next strip,
+// G strips on, once its last is done: that one ends R - 1 + 2w columns after its
+// first row's first, the other starts at least G R columns and G steps after it,
+// so 2w < G (R + 1) - R is enough (clipping at the matrix only shortens the
+// first).  Pairs of at most G strips never rotate: those with a longer side of
+// at most 50, whose band is the whole matrix, have at most 4 strips of 16 rows
+// or 7 of 8, and with a band too wide for 32 lanes every pair has at most 512
+// rows (wave_split_kernel), 32 strips.  0: one pair per warp at a time.
+static int32_t wave_shape(int32_t w) {
     if (!g_wave_stream) return 0;
-    const int32_t r = 2 * wmax < 31 * 4 + 32 ? 4 : 2 * wmax < 31 * 8 + 32 ? 8 : 16;
-    return g_wave_rows > r ? g_wave_rows : r;
+    if (w >= 1 && 2 * w < 8 * 9 - 8 && g_wave_rows <= 8) return 8 << 8 | 8;
+    if (w >= 1 && 2 * w < 8 * 17 - 16) return 16 << 8 | 8;
+    if (w >= 1 && 2 * w < 16 * 17 - 16) return 16 << 8 | 16;
+    return 16 << 8 | 32;
 }
 
 int32_t sw_set_wave(int32_t key, int32_t v) {
@@ -1306,7 +1341,7 @@ int32_t sw_set_wave(int32_t key, int32_t v) {
         return CK_ERR_INVALID_ARGUMENT;
     }
     if (key == 4 && v != 0 && v != 4 && v != 8 && v != 16) {
-        set_error(CK_ERR_UNSUPPORTED, "streamed strip rows must be 0 (smallest rotating), 4, 8 or 16");
+        set_error(CK_ERR_UNSUPPORTED, "streamed strip rows must be 0 (by band width), 4, 8 or 16");
         return CK_ERR_UNSUPPORTED;
     }
     if (key == 0) g_wave_min_rows = v;
@@ -1394,7 +1429,7 @@ static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *o
     int2 *window = (int2 *)scratch(SLOT_WINDOW, (size_t)blocks * per_block, &status);
     if (!window) return status;
     kern<<<blocks, NT, smem, st>>>(in, out, order, counters, inc, window, W, ticket,
-                                              ticket + 5, fallback, fb_count, err, 1, wave_rows_for(wmax),
+                                              ticket + 5, fallback, fb_count, err, 1, wave_shape(in.band_width),
                                               g_wave_stream == 2 ? 1 : 0, g_wide_key);
     CK_CUDA(cudaGetLastError());
     if (ctr) ctr->launches += 1;
@@ -1492,7 +1527,7 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
                                2 * in.band_width < 31 * 16 + 32;
         if (wave_only) rows = 8;
         int32_t nt = strip_threads(rows);
-        if (wave_only && !g_strip_threads && M <= 16 * (int64_t)sm_count()) nt = 512;
+        if (wave_only && !g_strip_threads) nt = 512;
         wave_split_kernel<<<1, 32, 0, st>>>(dk.Current(), cnt, in.band_width, g_wave_all_below,
                                             g_wave_min_rows, g_wave_adaptive, (int64_t)sm_count() * nt);
         CK_CUDA(cudaGetLastError());

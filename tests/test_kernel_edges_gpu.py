@@ -176,3 +176,41 @@ def test_similar_target_ranges(ck, n_db, shuffled, compact):
     with pytest.raises(_lib.CkError) as e:
         _similar(db, qs, 300, sub, 13, entries=ent, compact=compact, list_capacity=10)
     assert e.value.status == _lib.CK_ERR_CAPACITY
+
+
+@pytest.mark.parametrize("bw", [1, 8, 31, 32, 59, 60, 127, 128, 263])
+@pytest.mark.parametrize("hinted,long_rows", [(False, 0), (True, 0), (False, 2100)])
+def test_wave_group_shapes(ck, bw, hinted, long_rows):
+    """The streamed schedule at the band widths where its lanes per group and
+    rows per strip change: pairs of one strip, of just a group's lanes, and of
+    many rotations, with and without hints; rows above 2,047 take the wide key
+    for every pair."""
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.blosum import BLOSUM62
+    from clustkit_gb300.pairwise import batch_sw
+    rng = np.random.default_rng(bw + long_rows)
+    lens = [1, 2, 15, 16, 17, 49, 50, 51, 52, 64, 127, 128, 129, 130, 255, 256, 257, 258, 511, 513, 900, 1300]
+    if long_rows:
+        lens += [long_rows, long_rows + 40]
+    base = rng.integers(0, 20, max(lens) + 60)
+    seqs = []
+    for n in lens:
+        for v in range(3):  # related, shifted and unrelated
+            x = base[5 * v: 5 * v + n].copy() if v < 2 else rng.integers(0, 20, n)
+            x[rng.random(n) < 0.25] = rng.integers(0, 20)
+            seqs.append(x)
+    flat, off, length = _pack(seqs)
+    pairs = rng.integers(0, len(seqs), (2500, 2)).astype(np.int32)
+    pairs = np.concatenate([pairs, np.stack([np.arange(len(seqs) - 1), np.arange(1, len(seqs))], 1).astype(np.int32)])
+    hints = rng.integers(-80, 81, len(pairs)).astype(np.int32) if hinted else None
+    want = oracle.sw_batch(pairs, flat, off, length, bw, BLOSUM62, diag_hints=hints)
+    keep = _lib.get_config(_lib.CFG_WAVE_STREAM)
+    try:
+        for stream in (2, 0):
+            _lib.set_config(_lib.CFG_WAVE_STREAM, stream)
+            got = batch_sw(pairs, flat, off, length, bw, BLOSUM62, 0.3, diag_hints=hints)
+            for k in ("scores", "matches", "shorter", "sims"):
+                assert np.array_equal(got[k], want[k]), (k, stream)
+            assert _lib.sw_counters()["wave"] > 2000
+    finally:
+        _lib.set_config(_lib.CFG_WAVE_STREAM, keep)
