@@ -36,10 +36,9 @@
 //     H    = max(diag, E, F)                 (__vimax3_s32)
 // and H's priority/tie bits (or counter) are cleared before it feeds other
 // cells.
-// The first row-major cell holding the best score is tracked per row (strict
-// '>' along the row) and the rows are merged in row order after each strip;
-// a warp vote once per group of interior columns decides whether any lane's
-// cells reached its threshold, so most columns never touch the trackers.
+// The first row-major cell holding the best score is tracked per lane and strip
+// (StripBest); a warp vote once per group of interior columns decides whether
+// any lane's cells reached its threshold, so most columns need no more.
 // Rows of a pair's last strip below its last row read a pad code (their
 // diagonal always loses to zero), so every strip runs the same column code.
 // Scores use the key's top 16 bits; a pair whose best score comes within 24
@@ -103,9 +102,7 @@ struct KeyCompact {
 // up to 128 registers) for strips of 8 or 16 rows, 640 or 768 (20 or 24
 // warps at 96 or 80 registers) for 8-row strips, 256 (8 warps, up to 255
 // registers) for 24 or 32 rows.  One CTA per SM holds one increment table,
-// so the warps a CTA adds cost no table copy.  Each warp keeps its strip
-// rows' first-maximum trackers in a block of its own (row r of lane l at
-// r * 32 + l), so the layout does not depend on the CTA's size.
+// so the warps a CTA adds cost no table copy.
 // per warp, the streamed warp-per-pair phase's pair slots in shared memory
 constexpr size_t WAVE_SLOT_BYTES = 72;  // sizeof(WaveSlot), checked where it is defined
 constexpr int WAVE_SLOTS_PER_WARP = 16;
@@ -198,19 +195,6 @@ __host__ __device__ inline int64_t band_cells_closed(int32_t la, int32_t lb, int
     return sum_min(ilo, ihi, c2, lb) - sum_max(ilo, ihi, c1, 1) + (ihi - ilo + 1);
 }
 
-// Rows per lane strip for the warp-per-pair kernel, 0 when it cannot take
-// the pair.  Lane l runs strips l, l + 32, ... one column behind lane l - 1;
-// a lane may only start its next strip once its previous one (R + 2w - 1
-// steps) is done and its upstream lane has moved past the band, which holds
-// when 2w < 31 R + 32, or trivially when the pair has at most 32 strips.
-// The smallest such R keeps the most lanes busy.
-__host__ __device__ inline int32_t wave_rows_per_strip(int32_t la, int32_t w) {
-    if (la <= 128 || 2 * w < 31 * 4 + 32) return 4;
-    if (la <= 256 || 2 * w < 31 * 8 + 32) return 8;
-    if (la <= 512 || 2 * w < 31 * 16 + 32) return 16;
-    return 0;
-}
-
 // ----------------------------------------------------------------- prep
 __global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, uint8_t *__restrict__ seq_ok,
                                uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
@@ -254,8 +238,7 @@ __global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, uint8_t *__restric
 
 // Which sorted pairs (a prefix: rows descending) run one warp per pair,
 // decided on the device from the call's own counts.  Only when every
-// eligible pair can (wave_rows_per_strip > 0: band half-width <= 263, or at
-// most 512 rows).  A call with at most `all_below` eligible pairs: all of
+// eligible pair can (band half-width <= 263, or at most 512 rows: wave_shape).  A call with at most `all_below` eligible pairs: all of
 // them (too few to fill the GPU one per lane).  Otherwise, with a band width
 // > 0, the long pairs whose one-lane time would exceed the call's expected
 // run time: a pair of `rows` rows costs one lane about rows * (2w + 1) cell
@@ -479,35 +462,65 @@ __device__ __forceinline__ void strip_rows_masked(uint32_t bcol, int32_t &hu, in
     if (khi < R - 1) { hu = 0; eu = K::NEG_E; }  // the bottom row has not started
 }
 
-// First-max trackers (one per row, in shared memory) are touched only when
-// some lane holds a cell at or above its trigger threshold `tthr`: above the
-// pair's best when the strip began, and once this strip has set a best M, at
-// least M (an equal score in an earlier row still comes first in row-major
-// order; a lower one never can).  Only cells above the threshold read their
-// row's tracker; the strict '>' there keeps each row's first column.  The
-// check covers the U columns of `hs` (oldest first) at once, so that the
-// warp's vote and branch come once per U columns and the columns' row chains
-// can overlap in between.
-template <int R, int U>
-__device__ __forceinline__ void strip_track(const int32_t (&hs)[U][R], int32_t &tthr, int32_t *s_best) {
+// The best cell of a column of clean H keys: the lowest row with its best
+// score.  The row rides in the bits above the match count, clear in H (four in
+// the compact key, three in the wide one), so one maximum over 16 or 8 rows
+// finds it; taller strips compare those in row order.
+template <int R, class K>
+__device__ __forceinline__ void column_best(const int32_t (&hc)[R], int32_t &v, int32_t &row) {
+    constexpr int BITS = K::COMPACT ? 4 : 3, N = 1 << BITS, AT = 16 - BITS;
+    v = 0;
+    row = 0;
+#pragma unroll
+    for (int r0 = 0; r0 < R; r0 += N) {
+        int32_t x = hc[r0] + ((N - 1) << AT);
+#pragma unroll
+        for (int k = 1; k < N && r0 + k < R; k += 2) {
+            const int32_t a = hc[r0 + k] + ((N - 1 - k) << AT);
+            x = k + 1 < N && r0 + k + 1 < R ? __vimax3_s32(x, a, hc[r0 + k + 1] + ((N - 2 - k) << AT)) : max(x, a);
+        }
+        if (r0 == 0 || (x >> 16) > (v >> 16)) {
+            row = r0 + N - 1 - ((x >> AT) & (N - 1));
+            v = x & ~((N - 1) << AT);
+        }
+    }
+}
+
+// First maximum.  A lane holds its strip's best cell so far (`best`, its H, and
+// `best_r`, its row) and looks further only when some lane of the warp holds a
+// cell above its trigger threshold `tthr`: above the pair's best when the strip
+// began, and once this strip has set a best M, at least M (an equal score in an
+// earlier row still comes first in row-major order; a lower one never can).
+// Then each column's lowest row with its best score replaces the best cell when
+// it scores more, or as much in a lower row; a later column of the same row
+// does not.  The check covers the U columns of `hs` (oldest first) at once, so
+// that the warp's vote and branch come once per U columns and the columns' row
+// chains can overlap in between.  (A tracker per row in shared memory, the form
+// before, cost 32 accesses a strip to set up and merge and 32 KB of what is now
+// L1: 700,000 pairs at band 100 20.5 -> 19.5 ms.)
+struct StripBest {
+    int32_t best, best_r, tthr;
+};
+template <int R, int U, class K>
+__device__ __forceinline__ void strip_track(const int32_t (&hs)[U][R], StripBest &sb) {
     using namespace key;
     int32_t cm = hs[0][0];
 #pragma unroll
     for (int k = 1; k + 1 < U * R; k += 2) cm = __vimax3_s32(cm, hs[k / R][k % R], hs[(k + 1) / R][(k + 1) % R]);
     if (((U * R) & 1) == 0) cm = max(cm, hs[U - 1][R - 1]);
-    if (__any_sync(__activemask(), cm > tthr)) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
+    if (__any_sync(__activemask(), cm > sb.tthr)) {
+        if (cm > sb.tthr) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int32_t v = hs[u][r];
-                if (v > tthr) {
-                    const int32_t b = s_best[r * 32];
-                    if (v > (b | (KU - 1))) s_best[r * 32] = v;
+                int32_t v, vr;
+                column_best<R, K>(hs[u], v, vr);
+                if (v > sb.tthr && ((v >> 16) > (sb.best >> 16) || ((v >> 16) == (sb.best >> 16) && vr < sb.best_r))) {
+                    sb.best = v;
+                    sb.best_r = vr;
                 }
             }
+            sb.tthr = (cm & ~(KU - 1)) - 1;
         }
-        if (cm > tthr) tthr = (cm & ~(KU - 1)) - 1;
     }
 }
 
@@ -534,8 +547,8 @@ __device__ __forceinline__ void column_inputs(int32_t j, int32_t lb, StripRegs<R
 // over all of them.
 template <int R, int U, int P, class K>
 __device__ __forceinline__ void strip_group_percol(int32_t j, int32_t lb, StripRegs<R> &S, const char *s_inc,
-                                                   int2 *win, int32_t wmask, const uint8_t *B, int32_t &tthr,
-                                                   int32_t *s_best, int32_t one) {
+                                                   int2 *win, int32_t wmask, const uint8_t *B, StripBest &sb,
+                                                   int32_t one) {
     int32_t hs[U][R];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -550,7 +563,7 @@ __device__ __forceinline__ void strip_group_percol(int32_t j, int32_t lb, StripR
         for (int r = 0; r < R; ++r) hs[u][r] = S.hc[r];
     }
     strip_clear_f<R, K>(S);
-    strip_track<R, U>(hs, tthr, s_best);
+    strip_track<R, U, K>(hs, sb);
 }
 
 // U interior columns j .. j + U - 1 with j a multiple of U, inputs prefetched
@@ -561,8 +574,7 @@ __device__ __forceinline__ void strip_group_percol(int32_t j, int32_t lb, StripR
 // sequence.
 template <int R, int U, int P, class K>
 __device__ __forceinline__ void strip_group(int32_t j, StripRegs<R> &S, const char *s_inc, int2 *win,
-                                            int32_t wmask, const uint8_t *B, int32_t &tthr, int32_t *s_best,
-                                            int32_t one) {
+                                            int32_t wmask, const uint8_t *B, StripBest &sb, int32_t one) {
     int2 *cur = win + (size_t)(j & wmask) * 32;
     const uint8_t *pb = B + j + P - 1;  // residue of column j + P (columns are 1-based)
     int32_t hs[U][R];
@@ -587,7 +599,7 @@ __device__ __forceinline__ void strip_group(int32_t j, StripRegs<R> &S, const ch
         for (int r = 0; r < R; ++r) hs[u][r] = S.hc[r];
     }
     strip_clear_f<R, K>(S);
-    strip_track<R, U>(hs, tthr, s_best);
+    strip_track<R, U, K>(hs, sb);
 }
 
 // One column outside the aligned interior groups: a ramp or clipped column
@@ -595,7 +607,7 @@ __device__ __forceinline__ void strip_group(int32_t j, StripRegs<R> &S, const ch
 template <int R, int P, class K>
 __device__ __forceinline__ void strip_column(int32_t j, int32_t lb, StripRegs<R> &S, const char *s_inc,
                                              int2 *win, int32_t wmask, const uint8_t *B, int32_t lo0,
-                                             int32_t w2, int32_t &tthr, int32_t *s_best, int32_t one) {
+                                             int32_t w2, StripBest &sb, int32_t one) {
     int2 bnd;
     uint32_t bcol;
     column_inputs<R, P>(j, lb, S, win, wmask, B, bnd, bcol);
@@ -611,12 +623,12 @@ __device__ __forceinline__ void strip_column(int32_t j, int32_t lb, StripRegs<R>
     int32_t hs[1][R];
 #pragma unroll
     for (int r = 0; r < R; ++r) hs[0][r] = S.hc[r];
-    strip_track<R, 1>(hs, tthr, s_best);
+    strip_track<R, 1, K>(hs, sb);
 }
 
 template <int R, int V, class K>
 __device__ __forceinline__ void align_pair_strips_k(const SwIn &in, const SwOut &out, int64_t p,
-                                                    const PairGeom &g, const char *s_inc, int32_t *s_best,
+                                                    const PairGeom &g, const char *s_inc,
                                                     int2 *win, int32_t W, int32_t lane, int32_t *fallback,
                                                     int32_t *fallback_count, int32_t one) {
     using namespace key;
@@ -641,13 +653,12 @@ __device__ __forceinline__ void align_pair_strips_k(const SwIn &in, const SwOut 
         if (J0 > lb) break;
         if (J1 < J0) continue;
 
-        int32_t tthr = gbest | (KU - 1);
+        StripBest sb{0, 0, gbest | (KU - 1)};
         const int32_t alive = la - i0 + 1 < R ? la - i0 + 1 : R;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             S.hc[r] = 0;
             S.fT[r] = K::NEG_F;
-            s_best[r * 32] = gbest;
             // rows below the pair's last row (last strip only) read the pad code
             const uint32_t code = (r < alive) ? (uint32_t)A[i0 + r - 1] : PAD_CODE;
             S.arow[r] = (code * (uint32_t)N_CODES * 32u + (uint32_t)lane) * 4u;
@@ -672,23 +683,19 @@ __device__ __forceinline__ void align_pair_strips_k(const SwIn &in, const SwOut 
         constexpr bool ALIGNED = StripVariant<V>::ALIGNED;
         for (int32_t j = J0; j <= J1;) {
             if (ALIGNED && j >= I0 && (j & (U - 1)) == 0 && j + U - 1 <= I1 && j + U - 1 + P <= lb) {
-                strip_group<R, U, P, K>(j, S, s_inc, win, wmask, B, tthr, s_best, one);
+                strip_group<R, U, P, K>(j, S, s_inc, win, wmask, B, sb, one);
                 j += U;
             } else if (!ALIGNED && j >= I0 && j + U - 1 <= I1) {
-                strip_group_percol<R, U, P, K>(j, lb, S, s_inc, win, wmask, B, tthr, s_best, one);
+                strip_group_percol<R, U, P, K>(j, lb, S, s_inc, win, wmask, B, sb, one);
                 j += U;
             } else {
-                strip_column<R, P, K>(j, lb, S, s_inc, win, wmask, B, lo0, w2, tthr, s_best, one);
+                strip_column<R, P, K>(j, lb, S, s_inc, win, wmask, B, lo0, w2, sb, one);
                 j += 1;
             }
         }
-        // rows merge in row order: strict '>' keeps the earliest row on ties
-        // (pad rows never hold a new best: their values stay below a real cell's)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int32_t b = s_best[r * 32];
-            if (b > (gbest | (KU - 1))) gbest = b;
-        }
+        // strict '>': an equal score of an earlier strip comes first (pad rows
+        // never hold a new best: their values stay below a real cell's)
+        if (sb.best > (gbest | (KU - 1))) gbest = sb.best;
         // the columns right of this strip's band read as out-of-band for the next strip
         const int32_t fill_end = J1 + R < lb ? J1 + R : lb;
         for (int32_t j = J1 + 1; j <= fill_end; ++j)
@@ -709,37 +716,34 @@ __device__ __forceinline__ void align_pair_strips_k(const SwIn &in, const SwOut 
 // rows runs both forms.
 template <int R, int V>
 __device__ void align_pair_strips(const SwIn &in, const SwOut &out, int64_t p, const char *s_inc,
-                                  int32_t *s_best, int2 *win, int32_t W, int32_t lane,
+                                  int2 *win, int32_t W, int32_t lane,
                                   int32_t *fallback, int32_t *fallback_count, int32_t *err,
                                   int32_t one, int32_t wide_key) {
     const PairGeom g = pair_geometry(in, p, err);
     if (!wide_key && g.la <= KeyCompact::ROWS_MAX)
-        align_pair_strips_k<R, V, KeyCompact>(in, out, p, g, s_inc, s_best, win, W, lane, fallback,
+        align_pair_strips_k<R, V, KeyCompact>(in, out, p, g, s_inc, win, W, lane, fallback,
                                               fallback_count, one);
     else
-        align_pair_strips_k<R, V, KeyWide>(in, out, p, g, s_inc, s_best, win, W, lane, fallback,
+        align_pair_strips_k<R, V, KeyWide>(in, out, p, g, s_inc, win, W, lane, fallback,
                                            fallback_count, one);
 }
 
-// increment table + per-row first-max trackers (16 rows for the warp-per-pair
-// phase) + the warp-per-pair slots, for a CTA of NT threads
-template <int R>
-constexpr int track_rows() { return R > 16 ? R : 16; }
-template <int R, int NT>
+// increment table + the warp-per-pair slots, for a CTA of NT threads
+template <int NT>
 __host__ __device__ constexpr size_t strip_smem() {
-    return INC_SMEM + (size_t)track_rows<R>() * NT * sizeof(int32_t) +
-           (size_t)(NT / 32) * WAVE_SLOTS_PER_WARP * WAVE_SLOT_BYTES;
+    return INC_SMEM + (size_t)(NT / 32) * WAVE_SLOTS_PER_WARP * WAVE_SLOT_BYTES;
 }
 
-__device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &out, int64_t p,
-                                                 const char *s_inc, int32_t *s_best, int32_t lane,
-                                                 int32_t *fallback, int32_t *fallback_count,
-                                                 int32_t *err, int32_t one, int32_t wide_key);
 struct WaveSlot;
+// Shapes of the warp-per-pair phase, chosen in the kernel (wave_shapes).
+struct WaveShapes {
+    int32_t all, tail, few;  // R << 8 | G
+    int32_t force, serial;   // always `all`; a group's next pair only after its last
+};
 __device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                             int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
-                                             int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
-                                             int32_t one, int32_t compact);
+                                             int32_t n_wave, int32_t pack, int32_t serial, int32_t *ticket,
+                                             const char *s_inc, WaveSlot *slots, int32_t lane, int32_t *fallback,
+                                             int32_t *fallback_count, int32_t *err, int32_t one, int32_t compact);
 
 // Persistent alignment kernel.  Its warps first take the leading
 // counters[6] sorted pairs one warp per pair (long pairs, or every pair of a
@@ -748,45 +752,36 @@ __device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, cons
 // pair groups fill in around them.  Each warp's (or group's) first warp-per-pair
 // pair is dealt to it, block by block, and a ticket gives the later ones: by
 // ticket alone the warps of the first block to start took the longest pairs
-// together, and a small call's pairs filled a fifth of the SMs (500 pairs: DEAL).
+// together, and a small call's pairs filled a fifth of the SMs (500 pairs at the database
+// band, dealt out: 0.37 -> 0.24 ms the whole call).
 template <int R, int V, int NT>
 __global__ void __launch_bounds__(NT, 1)
 sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
                 const int32_t *__restrict__ counters, const int32_t *__restrict__ inc_global,
                 int2 *__restrict__ window, int32_t W, int32_t *__restrict__ ticket,
                 int32_t *__restrict__ wave_ticket, int32_t *__restrict__ fallback,
-                int32_t *__restrict__ fallback_count, int32_t *err, int32_t one, int32_t wave_shape,
-                int32_t wave_force, int32_t wide_key) {
+                int32_t *__restrict__ fallback_count, int32_t *err, int32_t one, WaveShapes wave,
+                int32_t wide_key) {
     extern __shared__ int32_t s_inc[];
     if (counters[0] <= 0) return;
     for (int t = threadIdx.x; t < INC_ENTRIES * 32; t += blockDim.x) s_inc[t] = inc_global[t >> 5];
     __syncthreads();
-    int32_t *s_best = s_inc + INC_ENTRIES * 32 + (threadIdx.x >> 5) * (track_rows<R>() * 32) + (threadIdx.x & 31);
     const int32_t lane = threadIdx.x & 31;
     const int32_t n_wave = counters[6];
-    // stream the pairs' strips through each warp when there are more pairs than
-    // warps (each warp then sees several); with fewer, one pair per warp at the
-    // rows per strip each pair allows has the shorter wavefronts
-    const int32_t n_warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
-    if (wave_shape > 0 && (wave_force || n_wave > n_warps)) {
-        // slots behind the increment table and the per-row trackers
-        char *slot_base = (char *)(s_inc + INC_ENTRIES * 32 + track_rows<R>() * NT);
+    if (n_wave > 0) {
+        char *slot_base = (char *)(s_inc + INC_ENTRIES * 32);  // behind the increment table
         WaveSlot *slots = (WaveSlot *)(slot_base + (size_t)(threadIdx.x >> 5) * WAVE_SLOTS_PER_WARP *
                                                        WAVE_SLOT_BYTES);
+        // the shape by what bounds the phase (wave_shapes)
+        const int32_t n_warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
+        const bool few = n_wave <= n_warps;
+        const int32_t shape = wave.force ? wave.all
+                              : few ? wave.few : counters[8] > KeyCompact::ROWS_MAX ? wave.tail : wave.all;
         // the compact key when every pair of the call (so every warp-per-pair
         // pair) has at most 2047 rows
-        if (n_wave > 0)
-            wave_stream_any(wave_shape, in, out, order, n_wave, wave_ticket, (const char *)s_inc, slots, lane,
-                            fallback, fallback_count, err, one, !wide_key && counters[8] <= KeyCompact::ROWS_MAX);
-    } else {
-        for (int32_t q = (int32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);;) {
-            if (q >= n_wave) break;
-            align_pair_wave_any(in, out, (int64_t)order[q], (const char *)s_inc, s_best, lane, fallback,
-                                fallback_count, err, one, wide_key);
-            __syncwarp();
-            if (lane == 0) q = n_warps + atomicAdd(wave_ticket, 1);
-            q = __shfl_sync(0xffffffffu, q, 0);
-        }
+        wave_stream_any(shape, in, out, order, n_wave, !few, wave.serial, wave_ticket,
+                        (const char *)s_inc, slots, lane, fallback, fallback_count, err, one,
+                        !wide_key && counters[8] <= KeyCompact::ROWS_MAX);
     }
     const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int2 *win = window + (size_t)gwarp * (size_t)W * 32 + lane;
@@ -801,206 +796,41 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
         if (grp >= n_groups) break;
         const int32_t q = grp * 32 + lane;
         if (q < n_elig)
-            align_pair_strips<R, V>(in, out, (int64_t)order[q], (const char *)s_inc, s_best, win, W, lane,
+            align_pair_strips<R, V>(in, out, (int64_t)order[q], (const char *)s_inc, win, W, lane,
                                  fallback, fallback_count, err, one, wide_key);
     }
 }
 
-// ----------------------------------------------------------------- wave kernel
-// One warp per pair, for pairs too few to fill the GPU one per lane and for
-// long pairs whose serial time would set the strip kernel's tail.  Rows are
-// cut into strips of R; lane l computes strips l, l + 32, l + 64, ..., and
-// at step T strip s works on column j = T - s + 1 + h - w, one column behind
-// strip s - 1.  Each step a lane receives by shuffle the (H, E) of the row
-// above its strip at column j, which the upstream lane produced the step
-// before, and the H it received the step before is its diagonal input.  A
-// lane outside its strip's columns sends the out-of-band boundary
-// (H = 0, E = -inf), and a lane whose upstream row has left its band
-// replaces what it receives by that boundary, so a lane that has moved on to
-// its next strip is never read.  Cells use the strip kernel's masked step.
+// ----------------------------------------------------------------- warp-per-pair phase
+// For pairs too few to fill the GPU one per lane, and for long pairs whose
+// serial time would set the strips' tail.  Rows are cut into strips of R; the
+// strips of consecutive pairs stream through G lanes, so that lanes freed by
+// one pair's strips take the next pair's instead of idling while the pair's
+// wavefront fills and drains.  A warp holds 32 / G such groups, each with its
+// own pairs; a step is U columns of every lane's strip, one block of columns
+// (blocks count from the pair's first band column c0, and R is a multiple of U,
+// so that all its strips share them).  Strips carry one sequence number g in
+// their group; lane g mod G of it runs strip g.  Strip s of a pair starting at
+// T0 runs block m at step T0 + s + m - m00, m00 being strip 0's first: exactly
+// one step behind its upstream strip s - 1 at every block, so each step a lane
+// receives by shuffle the (H, E) of the row above its strip at its columns,
+// which the upstream lane produced the step before; the last H received the
+// step before is its diagonal input.  A pair is issued (one per group and step,
+// once every strip of the previous one has started) with the smallest T0 at
+// which each of its first G strips finds its lane free; its later strips rotate
+// through the same lanes.  A lane whose upstream row has left its band (or that
+// has none) reads the out-of-band boundary (H = 0, E = -inf) instead, so a lane
+// never reads a neighbour's unrelated values.  Columns left and right of the
+// matrix, which a block may hold, are masked like rows outside their band.
 //
-// First maximum: a warp-wide running best score gs; when some lane's column
-// holds a score >= gs, every lane updates its per-row trackers (strict '>'
-// along a row) and gs rises.  A cell below gs cannot be the pair's maximum;
-// one equal to it may be, in an earlier row, so '>=' triggers.  At the end
-// of a strip its rows merge into the lane's best in row order (strict '>');
-// at the end of the pair the lanes agree on the best score, then on the
-// lowest row holding it -- clustkit's first cell in row-major order.
-template <int R, class K>
-__device__ void align_pair_wave(const SwIn &in, const SwOut &out, int64_t p, const PairGeom &g,
-                                const char *s_inc, int32_t *s_best, int32_t lane, int32_t *fallback,
-                                int32_t *fallback_count, int32_t one) {
-    using namespace key;
-    constexpr int32_t D = R + 1;
-    const int32_t la = g.la, lb = g.lb, w = g.w, h = g.h;
-    const uint8_t *A = in.flat + in.offsets[g.a_idx];
-    const uint8_t *B = in.flat + in.offsets[g.b_idx];
-    const uint32_t w2 = 2u * (uint32_t)w;
-    const int32_t c0 = 1 + h - w;  // j = T - s + c0
-
-    // strips that reach column <= lb (later ones lie right of the matrix)
-    int32_t n_strips = (la + R - 1) / R;
-    {
-        const int64_t lim = (int64_t)lb - 1 - h + w;  // s * R <= lim
-        const int64_t s_lim = lim < 0 ? 0 : lim / R + 1;
-        if (s_lim < n_strips) n_strips = (int32_t)s_lim;
-    }
-    int32_t lbest = 0, lrow = INT32_MAX;
-    if (n_strips > 0) {
-        const int32_t J0_0 = c0 > 1 ? c0 : 1;
-        const int32_t T_first = J0_0 - c0;
-        const int32_t sl = n_strips - 1;
-        const int32_t J1_l = sl * R + R + h + w < lb ? sl * R + R + h + w : lb;
-        const int32_t T_last = J1_l + sl - c0;
-
-        // this lane's strip at T_first; with at most 32 strips each lane has
-        // one and keeps it (its band may then be wider than the rotation allows)
-        const bool rotate = n_strips > 32;
-        int32_t s = lane;
-        if (rotate && T_first >= lane * D) s = lane + 32 * ((T_first - lane * D) / (32 * D));
-        int32_t next_switch = rotate ? (s + 32) * D : INT32_MAX;
-        int32_t i0 = 0, lo0 = 0, J0 = 0, J1 = -1, alive = 0;
-        uint32_t bcol_n = 0;  // residue offset of the strip's next column, loaded a step ahead
-        StripRegs<R> S;
-        auto setup = [&]() {
-            i0 = s * R + 1;
-            lo0 = i0 + h - w;
-            J0 = lo0 > 1 ? lo0 : 1;
-            J1 = i0 + R - 1 + h + w < lb ? i0 + R - 1 + h + w : lb;
-            if (s >= n_strips) { J0 = 1; J1 = 0; }
-            bcol_n = J0 <= J1 ? (uint32_t)__ldg(B + J0 - 1) * 128u : 0u;
-            alive = la - i0 + 1 < R ? la - i0 + 1 : R;
-            if (alive < 0) alive = 0;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                S.hc[r] = 0;
-                S.fT[r] = K::NEG_F;
-                s_best[r * 32] = 0;
-                const uint32_t code = (r < alive && s < n_strips) ? (uint32_t)A[i0 + r - 1] : 0u;
-                S.arow[r] = (code * (uint32_t)N_CODES * 32u + (uint32_t)lane) * 4u;
-            }
-        };
-        auto merge = [&]() {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int32_t b = s_best[r * 32];
-                if (r < alive && b > (lbest | (KU - 1))) { lbest = b; lrow = i0 + r; }
-            }
-        };
-        setup();
-        int32_t hout = 0, eout = K::NEG_E, hprev = 0, gs = 1;
-        for (int32_t T = T_first; T <= T_last; ++T) {
-            if (T == next_switch) {
-                merge();
-                s += 32;
-                next_switch += 32 * D;
-                setup();
-            }
-            const int32_t j = T - s + c0;
-            int32_t hin = __shfl_sync(0xffffffffu, hout, (lane + 31) & 31);
-            int32_t ein = __shfl_sync(0xffffffffu, eout, (lane + 31) & 31);
-            // H(row above, j - 1) arrived the step before; both it and this
-            // step's values are judged against the strip held now
-            const int32_t top = s * R + h + w;  // last in-band column of the row above
-            const int32_t hdiag = (s == 0 || j - 1 > top) ? 0 : hprev;
-            hprev = hin;
-            if (s == 0 || j > top) { hin = 0; ein = K::NEG_E; }
-            int32_t cm = 0;
-            if (j >= J0 && j <= J1) {
-                const uint32_t bcol = bcol_n;
-                if (j < J1) bcol_n = (uint32_t)__ldg(B + j) * 128u;  // column j + 1
-                int32_t hu = hin, eu = ein;
-                strip_cells<R, 0, R, true, K>(bcol, hu, eu, hdiag, S, s_inc, band_rows(j - lo0, w2, alive), one);
-                hout = hu;
-                eout = eu;
-                cm = S.hc[0];
-#pragma unroll
-                for (int r = 1; r + 1 < R; r += 2) cm = __vimax3_s32(cm, S.hc[r], S.hc[r + 1]);
-                if ((R & 1) == 0) cm = max(cm, S.hc[R - 1]);
-            } else {
-                hout = 0;
-                eout = K::NEG_E;
-            }
-            if constexpr (K::COMPACT) {
-                if ((T & 3) == 3) {  // at most 4 F extensions between clears (T is warp-uniform)
-#pragma unroll
-                    for (int r = 0; r < R; ++r) S.fT[r] &= ~K::CTR;
-                }
-            }
-            if (__any_sync(0xffffffffu, (cm >> 16) >= gs)) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int32_t b = s_best[r * 32];
-                    if (S.hc[r] > (b | (KU - 1))) s_best[r * 32] = S.hc[r];
-                }
-                const int32_t m = __reduce_max_sync(0xffffffffu, cm >> 16);
-                if (m > gs) gs = m;
-            }
-        }
-        merge();
-    }
-    // lanes agree on the best score, then on the lowest row holding it
-    const int32_t best = __reduce_max_sync(0xffffffffu, lbest >> 16);
-    const int32_t row = __reduce_min_sync(0xffffffffu, (best > 0 && (lbest >> 16) == best) ? lrow : INT32_MAX);
-    const bool writer = best > 0 ? ((lbest >> 16) == best && lrow == row) : lane == 0;
-    const uint32_t wmask = __ballot_sync(0xffffffffu, writer);
-    if (lane != __ffs(wmask) - 1) return;
-    if (best >= SCORE_LIMIT) {
-        const int32_t pos = atomicAdd(fallback_count, 1);
-        fallback[pos] = (int32_t)p;
-        atomicAdd(fallback_count + 2, 1);  // re-run counter
-        return;
-    }
-    write_result(out, in, p, best, best > 0 ? (lbest & K::MATCH_MASK) : 0, la, la, lb);
-}
-
-// One sorted wave pair, at the rows per strip its shape allows.
-template <class K>
-__device__ __forceinline__ void align_pair_wave_k(const SwIn &in, const SwOut &out, int64_t p, const PairGeom &g,
-                                                  const char *s_inc, int32_t *s_best, int32_t lane,
-                                                  int32_t *fallback, int32_t *fallback_count, int32_t one) {
-    switch (wave_rows_per_strip(g.la, g.w)) {
-        case 4: align_pair_wave<4, K>(in, out, p, g, s_inc, s_best, lane, fallback, fallback_count, one); break;
-        case 8: align_pair_wave<8, K>(in, out, p, g, s_inc, s_best, lane, fallback, fallback_count, one); break;
-        default: align_pair_wave<16, K>(in, out, p, g, s_inc, s_best, lane, fallback, fallback_count, one); break;
-    }
-}
-
-// the compact key for a pair of at most 2047 rows (unless wide_key)
-__device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &out, int64_t p,
-                                                 const char *s_inc, int32_t *s_best, int32_t lane,
-                                                 int32_t *fallback, int32_t *fallback_count,
-                                                 int32_t *err, int32_t one, int32_t wide_key) {
-    const PairGeom g = pair_geometry(in, p, err);
-    if (!wide_key && g.la <= KeyCompact::ROWS_MAX)
-        align_pair_wave_k<KeyCompact>(in, out, p, g, s_inc, s_best, lane, fallback, fallback_count, one);
-    else
-        align_pair_wave_k<KeyWide>(in, out, p, g, s_inc, s_best, lane, fallback, fallback_count, one);
-}
-
-// ----------------------------------------------------------------- streamed warp-per-pair
-// The warp-per-pair phase with the strips of consecutive pairs streamed
-// through G lanes, so that lanes freed by one pair's strips take the next
-// pair's instead of idling while the pair's wavefront fills and drains.  A warp
-// holds 32 / G such groups, each with its own pairs; a step is one column of
-// every lane's strip.  Strips carry one sequence number g in their group; lane
-// g mod G of it runs strip g.  Strip s of a pair starting at T0 runs column j
-// at step T0 + s + j - J0(strip 0), i.e. exactly one step behind its upstream
-// strip s - 1 at every column, so the (H, E) hand-over by shuffle works as in
-// the single-pair schedule.  A pair is issued (one per group and step, once
-// every strip of the previous one has started) with the smallest T0 at which
-// each of its first G strips finds its lane free; its later strips rotate
-// through the same lanes.  A lane's strip whose upstream lane belongs to
-// another pair or strip reads the out-of-band boundary instead (overrides
-// below), so a lane never reads a neighbour's unrelated values.
-//
-// G and the strip height R are shared by all pairs of a call (wave_shape).  A
-// strip of a band of half-width w lives 2w + R steps and its pair's next starts
-// R + 1 steps later, so about (2w + R) / (R + 1) lanes of a group work on a
-// pair: at w = 50, 21 lanes of 32 with the 4 rows that 32 lanes need to rotate
-// there, but 7 lanes of 8 with 16 rows -- and what a step costs beside its
-// cells (about 100 instructions) is spread over 16 rows a lane instead of 4.
-// 12,000 pairs at band 50: SMALL_NOTE.
+// R and G (wave_shapes): a strip of a band of half-width w lives (2w + R) / U
+// steps and its pair's next starts R / U + 1 later, so about (2w + R) / (R + U)
+// lanes of a group work on a pair, and G lanes suffice to rotate while
+// 2w <= (G - 1)(R + U) + 1.  What a step costs beside its cells, about 100
+// instructions, is spread over R U cells a lane.  Measured, 64 x 500 hinted
+// pairs at band 50: 1.93 ms with 32 lanes, strips of 4 rows and a column a
+// step, 0.92 with groups of 8 and 16 rows, 0.86 with two columns a step; 64 x 500
+// pairs at the database band (32 lanes, 16 rows): 3.47, 3.11 and 2.70.
 //
 // Per pair, a slot in shared memory holds its geometry, the running best
 // score (first-maximum trigger; each lane compares with its own copy, taken
@@ -1009,75 +839,73 @@ __device__ __noinline__ void align_pair_wave_any(const SwIn &in, const SwOut &ou
 // as one packed 64-bit value
 // (score, then lower row, then match count), merged by atomicMax at each
 // strip's end; the pair's last strip ends last and writes the result.  Within
-// a strip a lane holds its best cell in registers: on a trigger, the column's
+// a strip a lane holds its best cell in registers: on a trigger, each column's
 // lowest row with its best score replaces it when it scores more, or as much
 // in a lower row (a later column of the same row does not).
 constexpr int WS_SLOTS = WAVE_SLOTS_PER_WARP;
+constexpr int WS_U = 2;  // columns a step
 
 struct WaveSlot {
     unsigned long long acc;   // score << 27 | (16383 - row) << 13 | matches
     int64_t a_off, b_off;     // residues of the row and column sequences
     int64_t p;                // pair index
-    int32_t la, lb, w, h, c0, S, J00, T0;
+    int32_t la, lb, w, h, c0, S, m00, T0;
     int32_t gs;               // running best score of the pair (first-maximum trigger)
     int32_t live;
 };
 
 static_assert(sizeof(WaveSlot) == WAVE_SLOT_BYTES, "slot layout");
 
-template <int R>
-__device__ __forceinline__ void strip_bounds(const WaveSlot &sl, int32_t s, int32_t &i0, int32_t &lo,
-                                             int32_t &J0, int32_t &J1, int32_t &alive) {
-    i0 = s * R + 1;
-    lo = s * R + sl.c0;
-    J0 = lo > 1 ? lo : 1;
-    const int32_t hi = lo + R - 1 + 2 * sl.w;
-    J1 = hi < sl.lb ? hi : sl.lb;
-    alive = sl.la - i0 + 1 < R ? sl.la - i0 + 1 : R;
-    if (alive < 0) alive = 0;
-}
+// steps at which strip s starts (its first column's block) and ends (its last's)
 template <int R>
 __device__ __forceinline__ int32_t strip_t0(const WaveSlot &sl, int32_t s) {
     const int32_t lo = s * R + sl.c0;
-    return sl.T0 + s + (lo > 1 ? lo : 1) - sl.J00;
+    return sl.T0 + s + ((lo > 1 ? lo : 1) - sl.c0) / WS_U - sl.m00;
 }
 template <int R>
 __device__ __forceinline__ int32_t strip_te(const WaveSlot &sl, int32_t s) {
-    const int32_t lo = s * R + sl.c0;
-    const int32_t hi = lo + R - 1 + 2 * sl.w;
+    const int32_t hi = s * R + sl.c0 + R - 1 + 2 * sl.w;
     const int32_t J1 = hi < sl.lb ? hi : sl.lb;
-    const int32_t te = sl.T0 + s + J1 - sl.J00;
+    const int32_t te = sl.T0 + s + (J1 - sl.c0) / WS_U - sl.m00;
     const int32_t t0 = strip_t0<R>(sl, s);
     return te > t0 ? te : t0;  // a strip whose band lies left of column 1 ends where it starts
 }
 
 template <int R, int G, class K>
-__device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *order, int32_t n_wave,
-                            int32_t *ticket, const char *s_inc, WaveSlot *warp_slots, int32_t lane,
+__device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *order, int32_t n_wave, int32_t pack,
+                            int32_t serial, int32_t *ticket, const char *s_inc, WaveSlot *warp_slots, int32_t lane,
                             int32_t *fallback, int32_t *fallback_count, int32_t *err, int32_t one) {
     using namespace key;
     constexpr uint32_t FULL = 0xffffffffu;
+    constexpr int U = WS_U;
+    static_assert(R % U == 0 && R <= 16 && (U == 2 || U == 4), "blocks shared by a pair's strips; F counter clears");
     constexpr int SLOTS = WS_SLOTS * G / 32;  // of a group
     const int32_t gl = lane & (G - 1), g0 = lane - gl;  // lane of its group, the group's first lane
     const uint32_t gmask = G == 32 ? FULL : ((1u << (G & 31)) - 1u) << g0;
     const int32_t up = g0 | ((gl + G - 1) & (G - 1));   // the upstream lane
     WaveSlot *slots = warp_slots + lane / G * SLOTS;
-    // first pairs: dealt out over the blocks, then over a block's groups
+    // first pairs: dealt out over the blocks, then over a block's groups, warp
+    // by warp (a warp steps as long as its longest pair, so its groups take
+    // pairs of one length); over the warps first where there are fewer pairs
     const int32_t groups = (int32_t)(blockDim.x / G), n_first = groups * (int32_t)gridDim.x;
-    int32_t first_q = (int32_t)(threadIdx.x / G * gridDim.x + blockIdx.x);
+    const int32_t my_group = pack ? (int32_t)(threadIdx.x / G)
+                                  : lane / G * (int32_t)(blockDim.x >> 5) + (int32_t)(threadIdx.x >> 5);
+    int32_t first_q = my_group * (int32_t)gridDim.x + (int32_t)blockIdx.x;
     // schedule state, the same for every lane of a group (T for the warp)
     int32_t T = 0, T_issue = -1, g_next = 0, seq = 0;
     bool exhausted = false;
     for (int i = lane; i < WS_SLOTS; i += 32) warp_slots[i].live = 0;
     __syncwarp();
     // per-lane strip state
-    int32_t cur_slot = -1, cur_s = 0, i0 = 0, lo0 = 0, J0 = 1, J1 = 0, alive = 0, te = 0, top = 0;
-    int32_t jb = 0;    // j = T + jb for the strip held
-    uint32_t w2s = 0;  // 2w of its pair
-    uint32_t bcol_n = 0;  // residue offset of its next column, loaded a step ahead
+    int32_t cur_slot = -1, cur_s = 0, i0 = 0, lo0 = 0, alive = 0, te = 0, top = 0, lb = 0;
+    int32_t jb = 0;         // first column of the step's block: U * T + jb
+    uint32_t w2s = 0;       // 2w of its pair
+    uint32_t bcol[U] = {};  // residue offsets of the block's columns, loaded a step ahead
     int32_t pend_slot = -1, pend_s = 0, pend_t0 = 0;
     int32_t F = -1;
-    int32_t hout = 0, eout = K::NEG_E, hprev = 0;
+    int32_t hout[U], eout[U], hprev = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) { hout[u] = 0; eout[u] = K::NEG_E; }
     // the held strip's pair's running best score as last seen by this lane: at
     // most the slot's, so its trigger fires at least whenever the slot's would
     int32_t gs_l = 1;
@@ -1086,7 +914,8 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
     StripRegs<R> S;
     for (;;) {
         // ---- issue one pair (the same for every lane of the group)
-        if (!exhausted && T > T_issue && !slots[seq % SLOTS].live) {
+        if (!exhausted && T > T_issue && !slots[seq % SLOTS].live &&
+            (!serial || seq == 0 || !slots[(seq - 1) % SLOTS].live)) {
             int32_t q = first_q;
             if (first_q < 0) {
                 if (gl == 0) q = n_first + atomicAdd(ticket, 1);
@@ -1109,13 +938,13 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                 } else {
                     WaveSlot &sl = slots[seq % SLOTS];
                     const int32_t c0 = 1 + g.h - g.w;
-                    const int32_t J00 = c0 > 1 ? c0 : 1;
+                    const int32_t m00 = ((c0 > 1 ? c0 : 1) - c0) / U;
                     const int32_t m = (gl - g_next) & (G - 1);
                     const int32_t first = n_strips < G ? n_strips : G;
                     int32_t req = T;
                     if (m < first) {
                         const int32_t lom = m * R + c0;
-                        const int32_t r = F + 1 - m - ((lom > 1 ? lom : 1) - J00);
+                        const int32_t r = F + 1 - m - (((lom > 1 ? lom : 1) - c0) / U - m00);
                         req = r > T ? r : T;
                     }
                     const int32_t T0p = __reduce_max_sync(gmask, req);
@@ -1125,7 +954,7 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
                         sl.b_off = in.offsets[g.b_idx];
                         sl.p = p;
                         sl.la = g.la; sl.lb = g.lb; sl.w = g.w; sl.h = g.h; sl.c0 = c0;
-                        sl.S = n_strips; sl.J00 = J00; sl.T0 = T0p; sl.gs = 1; sl.live = 1;
+                        sl.S = n_strips; sl.m00 = m00; sl.T0 = T0p; sl.gs = 1; sl.live = 1;
                     }
                     __syncwarp(gmask);
                     if (m < first) {
@@ -1142,7 +971,7 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             }
         }
         // ---- start this lane's next strip.  Its start step is never in the past
-        // (the rotation bound, wave_shape); were it, the strip starts now and the
+        // (the rotation bound, wave_shapes); were it, the strip starts now and the
         // call reports an internal error rather than the warp waiting forever.
         if (pend_slot >= 0 && T >= pend_t0) {
             if (T > pend_t0) atomicOr(err, ERRBIT_SCHEDULE);
@@ -1152,14 +981,23 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             pend_slot = -1;
             gs_l = sl.gs;
             best = 0;
-            strip_bounds<R>(sl, cur_s, i0, lo0, J0, J1, alive);
+            best_r = 0;
+            lb = sl.lb;
+            i0 = cur_s * R + 1;
+            lo0 = cur_s * R + sl.c0;
+            alive = sl.la - i0 + 1 < R ? sl.la - i0 + 1 : R;
             te = strip_te<R>(sl, cur_s);
             if (te < T) te = T;  // only after a late start: the strip still ends
             top = cur_s * R + sl.h + sl.w;
-            jb = sl.J00 - sl.T0 - cur_s;
+            jb = sl.c0 + U * (sl.m00 - sl.T0 - cur_s);
             w2s = 2u * (uint32_t)sl.w;
             B = in.flat + sl.b_off;
-            bcol_n = J0 <= J1 ? (uint32_t)__ldg(B + J0 - 1) * 128u : 0u;
+            const int32_t j = U * T + jb;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t c = j + u < 1 ? 1 : j + u < lb ? j + u : lb;
+                bcol[u] = (uint32_t)__ldg(B + c - 1) * 128u;
+            }
             const uint8_t *A = in.flat + sl.a_off;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -1170,65 +1008,62 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             }
         }
         __syncwarp();
-        // ---- one column of this lane's strip
-        int32_t hin = __shfl_sync(FULL, hout, up);
-        int32_t ein = __shfl_sync(FULL, eout, up);
-        int32_t cm = 0;
-        const bool has = cur_slot >= 0;
-        int32_t j = 0;
-        if (has) {
-            j = T + jb;
-            const int32_t hdiag = (cur_s == 0 || j - 1 > top || j - 1 < 1) ? 0 : hprev;
-            hprev = hin;
-            if (cur_s == 0 || j > top) { hin = 0; ein = K::NEG_E; }
-            if (j >= J0 && j <= J1) {
-                const uint32_t bcol = bcol_n;
-                if (j < J1) bcol_n = (uint32_t)__ldg(B + j) * 128u;  // column j + 1
-                int32_t hu = hin, eu = ein;
-                strip_cells<R, 0, R, true, K>(bcol, hu, eu, hdiag, S, s_inc, band_rows(j - lo0, w2s, alive), one);
-                hout = hu;
-                eout = eu;
-                cm = S.hc[0];
+        // ---- one block of this lane's strip
+        int32_t hin[U], ein[U];
 #pragma unroll
-                for (int r = 1; r + 1 < R; r += 2) cm = __vimax3_s32(cm, S.hc[r], S.hc[r + 1]);
-                if ((R & 1) == 0) cm = max(cm, S.hc[R - 1]);
-            } else {
-                hout = 0;
-                eout = K::NEG_E;
+        for (int u = 0; u < U; ++u) {
+            hin[u] = __shfl_sync(FULL, hout[u], up);
+            ein[u] = __shfl_sync(FULL, eout[u], up);
+        }
+        const bool has = cur_slot >= 0;
+        if (has) {
+            const int32_t j = U * T + jb;
+            int32_t hdiag = (cur_s == 0 || j - 1 > top || j - 1 < 1) ? 0 : hprev;
+            hprev = hin[U - 1];
+            int32_t hs[U][R];
+            int32_t cm = 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t ju = j + u;
+                int32_t hu = hin[u], eu = ein[u];
+                if (cur_s == 0 || ju > top) { hu = 0; eu = K::NEG_E; }
+                const int32_t h_above = hu;
+                const uint32_t b = bcol[u];
+                const int32_t next = ju + U < lb ? ju + U : lb;  // at least 1: ju + U > J0 - 1
+                bcol[u] = (uint32_t)__ldg(B + (next > 1 ? next : 1) - 1) * 128u;
+                const uint32_t rows = ju >= 1 && ju <= lb ? band_rows(ju - lo0, w2s, alive) : 0u;
+                strip_cells<R, 0, R, true, K>(b, hu, eu, hdiag, S, s_inc, rows, one);
+                hdiag = h_above;
+                hout[u] = hu;
+                eout[u] = eu;
+#pragma unroll
+                for (int r = 0; r < R; ++r) hs[u][r] = S.hc[r];
+#pragma unroll
+                for (int r = 0; r < R; r += 2) cm = __vimax3_s32(cm, hs[u][r], hs[u][r + 1]);
+            }
+            // ---- first maximum: a column that reaches the pair's running best score
+            if ((cm >> 16) >= gs_l) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    int32_t v, vr;
+                    column_best<R, K>(hs[u], v, vr);
+                    if ((v >> 16) > (best >> 16) || ((v >> 16) == (best >> 16) && vr < best_r)) {
+                        best = v;
+                        best_r = vr;
+                    }
+                }
+                gs_l = max(atomicMax(&slots[cur_slot].gs, cm >> 16), cm >> 16);
             }
         } else {
-            hprev = hin;
-            hout = 0;
-            eout = K::NEG_E;
+            hprev = hin[U - 1];
+#pragma unroll
+            for (int u = 0; u < U; ++u) { hout[u] = 0; eout[u] = K::NEG_E; }
         }
         if constexpr (K::COMPACT) {
-            if ((T & 3) == 3) {  // at most 4 F extensions between clears (T is warp-uniform)
+            if (U == 4 || (T & 1)) {  // at most 4 F extensions between clears (T is warp-uniform)
 #pragma unroll
                 for (int r = 0; r < R; ++r) S.fT[r] &= ~K::CTR;
             }
-        }
-        // ---- first maximum: a column that reaches the pair's running best score
-        if (has && (cm >> 16) >= gs_l) {
-            const int32_t floor = cm & ~(KU - 1);
-            int32_t v = 0, vr = 0;
-            if constexpr (K::COMPACT) {
-                // the row rides in the four bits above the match count, clear
-                // in H: one maximum finds the lowest row with the best score
-                v = S.hc[0] + ((R - 1) << 12);
-#pragma unroll
-                for (int r = 1; r < R; r += 2) {
-                    const int32_t a = S.hc[r] + ((R - 1 - r) << 12);
-                    v = r + 1 < R ? __vimax3_s32(v, a, S.hc[r + 1] + ((R - 2 - r) << 12)) : max(v, a);
-                }
-                vr = R - 1 - ((v >> 12) & 15);
-                v &= ~(15 << 12);
-            } else {
-#pragma unroll
-                for (int r = R - 1; r >= 0; --r)
-                    if (S.hc[r] >= floor) { v = S.hc[r]; vr = r; }  // ends at the lowest such row
-            }
-            if (floor > (best & ~(KU - 1)) || ((best >> 16) == (cm >> 16) && vr < best_r)) { best = v; best_r = vr; }
-            gs_l = max(atomicMax(&slots[cur_slot].gs, cm >> 16), cm >> 16);
         }
         // ---- strip end: its best cell into the pair's; the last strip writes
         if (has && T == te) {
@@ -1265,27 +1100,29 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
 
 template <class K>
 __device__ __forceinline__ void wave_stream_k(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                              int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
-                                              int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
-                                              int32_t one) {
+                                              int32_t n_wave, int32_t pack, int32_t serial, int32_t *ticket,
+                                              const char *s_inc, WaveSlot *slots, int32_t lane, int32_t *fallback,
+                                              int32_t *fallback_count, int32_t *err, int32_t one) {
     switch (shape) {
-        case 8 << 8 | 8: wave_stream<8, 8, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
-        case 16 << 8 | 8: wave_stream<16, 8, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
-        case 16 << 8 | 16: wave_stream<16, 16, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
-        default: wave_stream<16, 32, K>(in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 8 << 8 | 8: wave_stream<8, 8, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 8 << 8 | 16: wave_stream<8, 16, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 8 << 8 | 32: wave_stream<8, 32, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 16 << 8 | 8: wave_stream<16, 8, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        case 16 << 8 | 16: wave_stream<16, 16, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
+        default: wave_stream<16, 32, K>(in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback, fallback_count, err, one); break;
     }
 }
 
 __device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, const SwOut &out, const uint32_t *order,
-                                             int32_t n_wave, int32_t *ticket, const char *s_inc, WaveSlot *slots,
-                                             int32_t lane, int32_t *fallback, int32_t *fallback_count, int32_t *err,
-                                             int32_t one, int32_t compact) {
+                                             int32_t n_wave, int32_t pack, int32_t serial, int32_t *ticket,
+                                             const char *s_inc, WaveSlot *slots, int32_t lane, int32_t *fallback,
+                                             int32_t *fallback_count, int32_t *err, int32_t one, int32_t compact) {
     if (compact)
-        wave_stream_k<KeyCompact>(shape, in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count,
-                                  err, one);
+        wave_stream_k<KeyCompact>(shape, in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback,
+                                  fallback_count, err, one);
     else
-        wave_stream_k<KeyWide>(shape, in, out, order, n_wave, ticket, s_inc, slots, lane, fallback, fallback_count,
-                               err, one);
+        wave_stream_k<KeyWide>(shape, in, out, order, n_wave, pack, serial, ticket, s_inc, slots, lane, fallback,
+                               fallback_count, err, one);
 }
 
 // ----------------------------------------------------------------- driver
@@ -1311,28 +1148,47 @@ static int32_t g_wide_key = 0;
 static int32_t g_wave_all_below = 40960;
 static int32_t g_wave_min_rows = 512;
 static int32_t g_wave_adaptive = 1;
-// stream the strips of consecutive pairs through a warp: 1 when the call has
-// more warp-per-pair pairs than warps, 2 always, 0 never
+// warp-per-pair schedule: 1 the shape by what bounds the phase, 2 always the
+// one of calls that run every pair this way, 0 a group's next pair only after
+// its last (one pair at a time)
 static int32_t g_wave_stream = 1;
-// rows per strip of the streamed schedule: 0 = by band width, else at least
+// rows per strip of the warp-per-pair schedule: 0 = by shape, else at least
 // that many (4, 8 or 16)
 static int32_t g_wave_rows = 0;
 
-// Rows per strip R and lanes per group G (as R << 8 | G) of the streamed
-// schedule, for band half-widths up to w.  A lane may start its next strip,
-// G strips on, once its last is done: that one ends R - 1 + 2w columns after its
-// first row's first, the other starts at least G R columns and G steps after it,
-// so 2w < G (R + 1) - R is enough (clipping at the matrix only shortens the
+// The smallest group that strips of R rows can rotate through in a band of
+// half-width w.  A lane may start its next strip, G strips on, once its last is
+// done: that one's last column is R - 1 + 2w after its first row's first, the
+// other's first at least G R after it and G steps later, so
+// 2w <= (G - 1)(R + U) + 1 is enough (clipping at the matrix only shortens the
 // first).  Pairs of at most G strips never rotate: those with a longer side of
-// at most 50, whose band is the whole matrix, have at most 4 strips of 16 rows
-// or 7 of 8, and with a band too wide for 32 lanes every pair has at most 512
-// rows (wave_split_kernel), 32 strips.  0: one pair per warp at a time.
-static int32_t wave_shape(int32_t w) {
-    if (!g_wave_stream) return 0;
-    if (w >= 1 && 2 * w < 8 * 9 - 8 && g_wave_rows <= 8) return 8 << 8 | 8;
-    if (w >= 1 && 2 * w < 8 * 17 - 16) return 16 << 8 | 8;
-    if (w >= 1 && 2 * w < 16 * 17 - 16) return 16 << 8 | 16;
-    return 16 << 8 | 32;
+// at most 50, whose band is the whole matrix, have at most 7 strips of 8 rows;
+// and where the band is too wide for 32 lanes of 16 rows, every pair has at most
+// 512 rows (wave_split_kernel), 32 strips.  0: none.
+static int32_t wave_group(int32_t R, int32_t w) {
+    if (w >= 1)
+        for (int32_t G = 8; G <= 32; G <<= 1)
+            if (2 * (int64_t)w <= (G - 1) * (R + WS_U) + 1) return G;
+    return R == 16 ? 32 : 0;
+}
+
+// The shapes of a call with band half-width w.  16 rows, for the cells a step's
+// own cost is spread over (8 where 8 lanes of them rotate: at narrow bands a
+// strip of 16 rows is largely ramps).  With a pair of more than 2,047 rows, whose
+// steps one after another set the phase's end: 8 rows, whose steps are shorter
+// (500,000 pairs of Pareto lengths to 8,000, band 32: 4.77 ms with 16 rows, 3.27
+// with 8; 100,000 pairs of at most 1,500 rows, band 100: 4.09 and 4.64).  Fewer
+// pairs than warps: 8 rows and a warp a pair.
+static WaveShapes wave_shapes(int32_t w) {
+    WaveShapes s{};
+    const int32_t g8 = g_wave_rows <= 8 ? wave_group(8, w) : 0, g16 = wave_group(16, w);
+    s.all = g8 == 8 ? 8 << 8 | 8 : 16 << 8 | g16;
+    s.tail = g8 ? 8 << 8 | g8 : 16 << 8 | g16;
+    s.few = (g8 ? 8 : 16) << 8 | 32;
+    s.force = g_wave_stream == 2;
+    s.serial = g_wave_stream == 0;
+    if (s.serial) s.all = s.tail = s.few;
+    return s;
 }
 
 int32_t sw_set_wave(int32_t key, int32_t v) {
@@ -1411,7 +1267,7 @@ static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *o
                              int32_t *err, cudaStream_t st, SwCounters *ctr) {
     int32_t status = CK_OK;
     auto kern = sw_strip_kernel<R, V, NT>;
-    const size_t smem = strip_smem<R, NT>();
+    const size_t smem = strip_smem<NT>();
     CK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     CK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
@@ -1429,8 +1285,8 @@ static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *o
     int2 *window = (int2 *)scratch(SLOT_WINDOW, (size_t)blocks * per_block, &status);
     if (!window) return status;
     kern<<<blocks, NT, smem, st>>>(in, out, order, counters, inc, window, W, ticket,
-                                              ticket + 5, fallback, fb_count, err, 1, wave_shape(in.band_width),
-                                              g_wave_stream == 2 ? 1 : 0, g_wide_key);
+                                              ticket + 5, fallback, fb_count, err, 1, wave_shapes(in.band_width),
+                                              g_wide_key);
     CK_CUDA(cudaGetLastError());
     if (ctr) ctr->launches += 1;
     return CK_OK;
@@ -1518,18 +1374,22 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
         int32_t rows = g_rows_per_strip ? g_rows_per_strip : (wmax <= 64 ? 8 : 16);
         // A call that routes every pair one warp per pair (at most
         // CK_CFG_WAVE_ALL_BELOW pairs, a band narrow enough for every pair to
-        // rotate) never runs lane-per-pair strips: the 8-row kernel's larger
-        // CTA gives its warp-per-pair phase 20 warps per SM instead of 16
-        // (search-shaped calls of 8 k and 32 k pairs: 9-18 % faster), unless
-        // the call has no more pairs than 16 warps per SM -- one pair per warp,
-        // where the 512-thread CTA's unspilled code is the faster.
+        // rotate) never runs lane-per-pair strips; its kernel is the 512-thread
+        // one, whose 128 registers hold the warp-per-pair phase unspilled (640
+        // threads at 96: 1.10 against 0.98 ms on 64 x 500 pairs at band 50).
         const bool wave_only = !g_rows_per_strip && M <= (int64_t)g_wave_all_below && in.band_width >= 1 &&
                                2 * in.band_width < 31 * 16 + 32;
         if (wave_only) rows = 8;
         int32_t nt = strip_threads(rows);
         if (wave_only && !g_strip_threads) nt = 512;
-        wave_split_kernel<<<1, 32, 0, st>>>(dk.Current(), cnt, in.band_width, g_wave_all_below,
-                                            g_wave_min_rows, g_wave_adaptive, (int64_t)sm_count() * nt);
+        // the row bound of larger calls: three quarters of the setting above
+        // band 24, where a strip of 16 rows in a group of 8 or more lanes is
+        // worth it from 384 rows on (100,000 pairs of lognormal lengths, bound
+        // 512 and 384: band 16 1.31 and 1.42 ms, 100 4.08 and 4.00, 200 7.00 and
+        // 6.78; 60,000 at band 50 2.25 and 1.69)
+        const int32_t min_rows = in.band_width > 24 ? g_wave_min_rows / 4 * 3 : g_wave_min_rows;
+        wave_split_kernel<<<1, 32, 0, st>>>(dk.Current(), cnt, in.band_width, g_wave_all_below, min_rows,
+                                            g_wave_adaptive, (int64_t)sm_count() * nt);
         CK_CUDA(cudaGetLastError());
         // profiling events bracket the alignment kernel
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -185,27 +185,28 @@ int32_t ck_sw_last_kernel_ms(float *out_ms);
  *                          skipped pairs) run every pair one warp per pair
  *                          (default 40960)
  *   CK_CFG_WAVE_MIN_ROWS   in larger calls with band_width > 0, pairs with at
- *                          least this many rows (shorter side) run one warp
- *                          per pair instead of one lane per pair (default 512)
+ *                          least this many rows (shorter side), or three
+ *                          quarters of it at bands above 24, run one warp per
+ *                          pair instead of one lane per pair (default 512)
  *   CK_CFG_WAVE_ADAPTIVE   1 (default): raise that row bound to where a pair's
  *                          one-lane time would pass the call's expected
  *                          kernel time, from the call's cell count; 0:
  *                          use CK_CFG_WAVE_MIN_ROWS as given
- *   CK_CFG_WAVE_STREAM     1 (default): when a call has more warp-per-pair
- *                          pairs than the kernel has warps, a warp streams the
- *                          row strips of consecutive pairs through its lanes;
- *                          2: always; 0: never (one pair per warp at a time)
- *   CK_CFG_WAVE_ROWS       rows per strip of that streamed schedule: 0
- *                          (default) the smallest of 4/8/16 whose strips can
- *                          rotate through the lanes at the call's band width;
- *                          4, 8 or 16: at least that many
+ *   CK_CFG_WAVE_STREAM     1 (default): the strips of consecutive pairs stream
+ *                          through groups of 8, 16 or 32 lanes of a warp, sized
+ *                          by the band, with strip heights by what bounds the
+ *                          phase; 2: always those of calls that run every pair
+ *                          one warp per pair; 0: one pair per warp at a time
+ *   CK_CFG_WAVE_ROWS       rows per strip of that schedule: 0 (default) 8 or 16
+ *                          by band and longest pair; 4, 8 or 16: at least that
  *                          (key 7, a cluster-shared-memory form of the
  *                          similar-k-mer posting walk, is retired: it
  *                          measured 2.6x slower than the L2-atomic walk)
  *   CK_CFG_STRIP_THREADS   threads of the strip kernel's one persistent CTA
  *                          per SM for strips of 8 rows: 512 (16 warps, up to
  *                          128 registers), 640 (20 warps, 96) or 768 (24, 80);
- *                          0 (default): 640.  Strips of 16 rows always run
+ *                          0 (default): 640, or 512 for calls whose pairs all
+ *                          run one warp per pair.  Strips of 16 rows always run
  *                          512 threads, of 24 or 32 rows 256.  With the
  *                          default rows per strip, a call whose pairs all run
  *                          one warp per pair runs the 8-row kernel.  (Key 8,
