@@ -119,10 +119,10 @@ __global__ void jaccard_kernel(const int32_t *__restrict__ pairs, int64_t M,
 // s = 128), and only hits search A.  A and its bitmap stay in shared memory
 // while consecutive pairs of the warp's run share their first sequence, as a
 // sorted candidate list's do; the next pair's B is loaded while one is worked
-// on.  That leaves one coalesced sketch read a pair, and about 25 instructions
-// a lane for a pair without shared values: bound by issue and by the sketch
-// rows' way from L2.  4 M pairs of 100,000 sketches at s = 128: 2.92 -> 1.39 ms (both
-// sketches staged in shared memory and every element searched, before).
+// on.  A lane works through its own hits, so a chance pair costs one binary
+// search.  Bound by issue (83 %).  4 M pairs of 100,000 sketches at s = 128:
+// 2.92 ms with both sketches staged and every element searched, 1.39 with the
+// bitmap and a search for each of a lane's elements, 1.01 now.
 constexpr int JACCARD_RUN = 32;  // pairs a warp takes at most (one per lane to load and to write)
 
 template <int E>
@@ -191,27 +191,44 @@ jaccard_bitmap_kernel(const int32_t *__restrict__ pairs, int64_t M, const uint64
             if (B[k] != MAXV && ((bm[h >> 5] >> (h & 31)) & 1u)) hit |= 1u << k;
         }
         int32_t shared = 0, total = 0;
-        if (__any_sync(FULL, hit != 0)) {
-            const uint64_t *gb = sk + (int64_t)i_b * s;
+        uint32_t paired = 0;
+        int32_t at[E];  // of a paired element: its place in A plus its copies before it in B
+        // each lane works through its own hits, so a pair costs as many
+        // searches as the lane with the most hits has (mostly one)
+        while (__any_sync(FULL, hit != 0)) {
+            if (hit) {
+                const int k = __ffs(hit) - 1;
+                hit &= hit - 1;
+                uint64_t v = B[0];
 #pragma unroll
-            for (int k = 0; k < E; ++k) {
-                const int32_t j = 32 * k + lane;
-                bool paired = false;
-                int32_t low = 0, m = 0;
-                if ((hit >> k) & 1u) {
-                    const uint64_t v = B[k];
-                    low = lower_bound_u64(A, s, v);
-                    if (low < s && A[low] == v) {
-                        while (m < j && __ldg(gb + j - m - 1) == v) ++m;
-                        paired = low + m < s && A[low + m] == v;
+                for (int i = 1; i < E; ++i)
+                    if (k == i) v = B[i];
+                int32_t low = 0;  // A is padded with MAX to 32 E, above any v here
+#pragma unroll
+                for (int step = 16 * E; step; step >>= 1)
+                    if (A[low + step - 1] < v) low += step;
+                if (A[low] == v) {
+                    const uint64_t *gb = sk + (int64_t)i_b * s;
+                    const int32_t j = 32 * k + lane;
+                    int32_t m = 0;
+                    while (m < j && __ldg(gb + j - m - 1) == v) ++m;
+                    if (low + m < s && A[low + m] == v) {
+                        paired |= 1u << k;
+#pragma unroll
+                        for (int i = 0; i < E; ++i)
+                            if (k == i) at[i] = low + m;
                     }
                 }
-                const uint32_t bal = __ballot_sync(FULL, paired);
-                if (bal) {
-                    const int32_t r = total + __popc(bal & ((1u << lane) - 1u));
-                    shared += __popc(__ballot_sync(FULL, paired && low + j - (r - m) < s));
-                    total += __popc(bal);
-                }
+            }
+        }
+        if (__any_sync(FULL, paired != 0)) {
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                const bool p = (paired >> k) & 1u;
+                const uint32_t bal = __ballot_sync(FULL, p);
+                const int32_t r = total + __popc(bal & ((1u << lane) - 1u));
+                shared += __popc(__ballot_sync(FULL, p && at[k] + 32 * k + lane - r < s));
+                total += __popc(bal);
             }
         }
         int32_t steps = s;  // a full sketch alone gives the walk its s steps
@@ -235,8 +252,8 @@ static int32_t launch_bitmap(const int32_t *pairs, int64_t M, const uint64_t *sk
                              float *sims, uint8_t *mask, int32_t *d_err, cudaStream_t st) {
     const size_t per_warp = (size_t)(32 * E + 32 * E) * sizeof(uint64_t);  // A, and 64 bits an element
     const int wpb = 8;
-    // runs short enough that a small list still fills the SMs (16 warps each)
-    const int64_t fill = (M + 16 * (int64_t)sm_count() - 1) / (16 * (int64_t)sm_count());
+    // runs short enough that a small list still fills the SMs (48 warps each)
+    const int64_t fill = (M + 48 * (int64_t)sm_count() - 1) / (48 * (int64_t)sm_count());
     const int32_t run = (int32_t)(fill < 1 ? 1 : fill > JACCARD_RUN ? JACCARD_RUN : fill);
     const int64_t blocks = ((M + run - 1) / run + wpb - 1) / wpb;
     jaccard_bitmap_kernel<E><<<(unsigned)blocks, wpb * 32, per_warp * wpb, st>>>(pairs, M, sk, N, s, run, floor, sims,
