@@ -126,40 +126,63 @@ constexpr int INC_ENTRIES = (N_CODES + 1) * N_CODES;     // 462: row code (0..21
 constexpr size_t INC_SMEM = (size_t)INC_ENTRIES * 32 * 4;  // replicated per lane
 
 // ----------------------------------------------------------------- tables
-__global__ void build_inc_kernel(const int8_t *sub, int32_t *inc) {
-    int t = threadIdx.x + blockIdx.x * blockDim.x;
-    if (t >= INC_ENTRIES) return;
-    int a = t / N_CODES, b = t % N_CODES;
-    int s = (a < 20 && b < 20) ? (int)sub[a * 20 + b] : -4;
-    inc[t] = a == (int)PAD_CODE ? PAD_INC : s * key::KU + 2 * key::PU + (a == b ? 1 : 0);
-}
-
-// Whether every residue code of sequence i is <= 20, memoised per call in
-// ok[i] (0 unknown, 1 yes, 2 no): only sequences that some pair references
-// are read, once or a few times (concurrent first readers agree).
-__device__ __forceinline__ bool seq_codes_ok(const SwIn &in, int32_t i, uint8_t *ok) {
-    const uint8_t m = ok[i];
-    if (m) return m == 1;
-    const uint8_t *s = in.flat + in.offsets[i];
-    const int32_t L = in.lengths[i];
-    // bytes up to a 16-byte boundary, then 16 per load (four compared per
-    // instruction), then the tail
-    int32_t head = (int32_t)((16u - ((uint32_t)(uintptr_t)s & 15u)) & 15u);
-    if (head > L) head = L;
-    uint32_t bad = 0;
-    for (int32_t t = 0; t < head; ++t) bad |= __ldg(s + t) > 20 ? 1u : 0u;
-    const uint4 *v = (const uint4 *)(s + head);
-    const int32_t nv = (L - head) >> 4;
-#pragma unroll 4
-    for (int32_t k = 0; k < nv; ++k) {
-        const uint4 x = __ldg(v + k);
-        bad |= __vcmpgtu4(x.x, 0x14141414u) | __vcmpgtu4(x.y, 0x14141414u) |
-               __vcmpgtu4(x.z, 0x14141414u) | __vcmpgtu4(x.w, 0x14141414u);
+// What the other kernels of a call read: the increment table and zeroed
+// counters (block 0), and ok[i] = 1 when every residue code of sequence i is
+// <= 20, else 2.  CODE_LANES lanes read a sequence, 16 bytes each at a time.
+// Items are the sequences themselves, or -- by_pair, for calls that name fewer
+// sequences than there are -- the two of each pair; an index or extent out of
+// range is left to the prep kernel to report.  (One thread read a whole
+// sequence before, on the first pair that named it, inside the prep kernel: 47 us
+// of a 500-pair call and 119 of 700,000 pairs, now 15 and 44 with prep.)
+constexpr int CODE_LANES = 8;
+__global__ void sw_tables_kernel(const int8_t *__restrict__ sub, int32_t *__restrict__ inc,
+                                 int32_t *__restrict__ counters, SwIn in, int64_t items, int32_t by_pair,
+                                 uint8_t *__restrict__ ok) {
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < 16) counters[threadIdx.x] = 0;
+        for (int t = threadIdx.x; t < INC_ENTRIES; t += blockDim.x) {
+            const int a = t / N_CODES, b = t % N_CODES;
+            const int s = (a < 20 && b < 20) ? (int)sub[a * 20 + b] : -4;
+            inc[t] = a == (int)PAD_CODE ? PAD_INC : s * key::KU + 2 * key::PU + (a == b ? 1 : 0);
+        }
     }
-    for (int32_t t = head + nv * 16; t < L; ++t) bad |= __ldg(s + t) > 20 ? 1u : 0u;
-    const bool good = bad == 0;
-    ok[i] = good ? 1 : 2;
-    return good;
+    const int gl = threadIdx.x & (CODE_LANES - 1);
+    const int64_t step = (int64_t)gridDim.x * blockDim.x / CODE_LANES;
+    for (int64_t x0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x - gl) / CODE_LANES;; x0 += step) {
+        if (!__any_sync(0xffffffffu, x0 < items)) break;
+        bool valid = x0 < items;
+        int64_t i = 0;
+        if (valid) {
+            i = by_pair ? (int64_t)__ldg(in.pairs + x0) : x0;
+            valid = i >= 0 && i < in.n_seqs;
+        }
+        uint32_t bad = 0;
+        if (valid) {
+            const int32_t L = __ldg(in.lengths + i);
+            const int64_t o = __ldg(in.offsets + i);
+            valid = L >= 0 && o >= 0 && o + L <= in.flat_len;
+            if (valid) {
+                const uint8_t *s = in.flat + o;
+                // bytes up to a 16-byte boundary, then 16 per load (four
+                // compared per instruction), then the tail
+                int32_t head = (int32_t)((16u - ((uint32_t)(uintptr_t)s & 15u)) & 15u);
+                if (head > L) head = L;
+                const int32_t nv = (L - head) >> 4;
+                const uint4 *v = (const uint4 *)(s + head);
+#pragma unroll 4
+                for (int32_t k = gl; k < nv; k += CODE_LANES) {
+                    const uint4 x = __ldg(v + k);
+                    bad |= __vcmpgtu4(x.x, 0x14141414u) | __vcmpgtu4(x.y, 0x14141414u) |
+                           __vcmpgtu4(x.z, 0x14141414u) | __vcmpgtu4(x.w, 0x14141414u);
+                }
+                for (int32_t t = gl; t < head; t += CODE_LANES) bad |= __ldg(s + t) > 20 ? 1u : 0u;
+                for (int32_t t = head + nv * 16 + gl; t < L; t += CODE_LANES) bad |= __ldg(s + t) > 20 ? 1u : 0u;
+            }
+        }
+        const uint32_t any = __ballot_sync(0xffffffffu, bad != 0);
+        const int lane = threadIdx.x & 31;
+        if (valid && gl == 0) ok[i] = ((any >> lane) & ((1u << CODE_LANES) - 1u)) ? 2 : 1;
+    }
 }
 
 // Closed-form count of the band cells of a pair (the cells clustkit's loop
@@ -196,7 +219,7 @@ __host__ __device__ inline int64_t band_cells_closed(int32_t la, int32_t lb, int
 }
 
 // ----------------------------------------------------------------- prep
-__global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, uint8_t *__restrict__ seq_ok,
+__global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, const uint8_t *__restrict__ seq_ok,
                                uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
                                int32_t *__restrict__ fallback, int32_t *__restrict__ counters,
                                unsigned long long *__restrict__ cells, int32_t *err) {
@@ -213,8 +236,7 @@ __global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, uint8_t *__restric
             write_result(out, in, p, 0, 0, g.la, g.la, g.lb);
         } else {
             local_cells += band_cells_closed(g.la, g.lb, g.w, g.h);
-            if (g.la <= key::ROWS_MAX && seq_codes_ok(in, g.a_idx, seq_ok) &&
-                seq_codes_ok(in, g.b_idx, seq_ok)) {
+            if (g.la <= key::ROWS_MAX && __ldg(seq_ok + g.a_idx) == 1 && __ldg(seq_ok + g.b_idx) == 1) {
                 int32_t cb = g.lb < key::ROWS_MAX ? g.lb : key::ROWS_MAX;
                 k = ((uint32_t)g.la << 13) | (uint32_t)cb;
                 elig++;
@@ -246,34 +268,42 @@ __global__ void sw_prep_kernel(SwIn in, SwOut out, int64_t M, uint8_t *__restric
 // pairs start first, so a pair below that bound does not set the tail).
 // Pairs at or above max(min_rows, that bound) are counted by a binary search
 // over the sorted keys.
-__global__ void wave_split_kernel(const uint32_t *__restrict__ sorted_keys, int32_t *counters,
-                                  int32_t band_width, int32_t all_below, int32_t min_rows,
-                                  int32_t adaptive, int64_t lanes) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int32_t n_elig = counters[0];
-    counters[6] = 0;
-    if (n_elig <= 0) return;
+// Every block of the alignment kernel decides it for itself (one warp, a few
+// loads; the first block records it), which spares the call a launch.
+struct WaveRoute {
+    int32_t band_width, all_below, min_rows, adaptive;
+    int64_t lanes;
+};
+__device__ __forceinline__ int32_t wave_split(const uint32_t *__restrict__ sorted_keys,
+                                              const int32_t *__restrict__ counters, const WaveRoute &r, int32_t lane) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const int32_t n_elig = counters[0], band_width = r.band_width;
     const int32_t max_rows = (int32_t)(sorted_keys[0] >> 13);
-    counters[8] = max_rows;  // the warp-per-pair phase's key form depends on it
     const bool all_capable = (band_width >= 1 && 2 * band_width < 31 * 16 + 32) || max_rows <= 512;
-    if (!all_capable) return;
-    if (n_elig <= all_below) { counters[6] = n_elig; return; }
-    if (band_width <= 0 || min_rows >= (1 << 13)) return;
+    if (!all_capable) return 0;
+    if (n_elig <= r.all_below) return n_elig;
+    if (band_width <= 0 || r.min_rows >= (1 << 13)) return 0;
     unsigned long long cells = 0;
     memcpy(&cells, counters + 4, sizeof(cells));
-    int64_t rows_thr = min_rows;
-    if (adaptive) {
-        const int64_t per_lane = (int64_t)(cells / (unsigned long long)(lanes > 0 ? lanes : 1));
-        const int64_t r = per_lane / (2 * (int64_t)band_width + 1) + 1;
-        if (r > rows_thr) rows_thr = r;
+    int64_t rows_thr = r.min_rows;
+    if (r.adaptive) {
+        const int64_t per_lane = (int64_t)(cells / (unsigned long long)(r.lanes > 0 ? r.lanes : 1));
+        const int64_t x = per_lane / (2 * (int64_t)band_width + 1) + 1;
+        if (x > rows_thr) rows_thr = x;
     }
-    // keys are (rows << 13 | cols), descending: count the prefix with rows >= rows_thr
-    int32_t lo = 0, hi = n_elig;
+    // keys are (rows << 13 | cols), descending: count the prefix with rows >=
+    // rows_thr, 32 probes a round
+    int32_t lo = 0, hi = n_elig;  // keys before lo reach it, those from hi on do not
     while (lo < hi) {
-        const int32_t mid = (lo + hi) >> 1;
-        if ((int64_t)(sorted_keys[mid] >> 13) >= rows_thr) lo = mid + 1; else hi = mid;
+        const int32_t span = hi - lo;
+        const int32_t at = lo + (int32_t)((int64_t)span * lane / 32);
+        const uint32_t bal = __ballot_sync(FULL, (int64_t)(sorted_keys[at] >> 13) >= rows_thr);
+        const int32_t n = __popc(bal);  // the first n probes reach it
+        const int32_t last = lo + (int32_t)((int64_t)span * (n - 1) / 32), next = lo + (int32_t)((int64_t)span * n / 32);
+        if (n < 32) hi = next;
+        if (n > 0) lo = last + 1;
     }
-    counters[6] = lo;
+    return lo;
 }
 
 // ----------------------------------------------------------------- strip kernel
@@ -746,7 +776,7 @@ __device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, cons
                                              int32_t *fallback_count, int32_t *err, int32_t one, int32_t compact);
 
 // Persistent alignment kernel.  Its warps first take the leading
-// counters[6] sorted pairs one warp per pair (long pairs, or every pair of a
+// pairs that wave_split picks one warp per pair (long pairs, or every pair of a
 // small call), then the rest 32 pairs per warp, one lane per pair, in
 // register strips of R rows.  Long pairs thus start first and the lane-per-
 // pair groups fill in around them.  Each warp's (or group's) first warp-per-pair
@@ -756,18 +786,26 @@ __device__ __noinline__ void wave_stream_any(int32_t shape, const SwIn &in, cons
 // band, dealt out: 0.37 -> 0.24 ms the whole call).
 template <int R, int V, int NT>
 __global__ void __launch_bounds__(NT, 1)
-sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
-                const int32_t *__restrict__ counters, const int32_t *__restrict__ inc_global,
+sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order, const uint32_t *__restrict__ sorted_keys,
+                int32_t *__restrict__ counters, const int32_t *__restrict__ inc_global, WaveRoute route,
                 int2 *__restrict__ window, int32_t W, int32_t *__restrict__ ticket,
                 int32_t *__restrict__ wave_ticket, int32_t *__restrict__ fallback,
                 int32_t *__restrict__ fallback_count, int32_t *err, int32_t one, WaveShapes wave,
                 int32_t wide_key) {
     extern __shared__ int32_t s_inc[];
+    __shared__ int32_t s_wave;
     if (counters[0] <= 0) return;
+    if (threadIdx.x < 32) {
+        const int32_t n = wave_split(sorted_keys, counters, route, threadIdx.x);
+        if (threadIdx.x == 0) {
+            s_wave = n;
+            if (blockIdx.x == 0) counters[6] = n;
+        }
+    }
     for (int t = threadIdx.x; t < INC_ENTRIES * 32; t += blockDim.x) s_inc[t] = inc_global[t >> 5];
     __syncthreads();
     const int32_t lane = threadIdx.x & 31;
-    const int32_t n_wave = counters[6];
+    const int32_t n_wave = s_wave, max_rows = (int32_t)(sorted_keys[0] >> 13);
     if (n_wave > 0) {
         char *slot_base = (char *)(s_inc + INC_ENTRIES * 32);  // behind the increment table
         WaveSlot *slots = (WaveSlot *)(slot_base + (size_t)(threadIdx.x >> 5) * WAVE_SLOTS_PER_WARP *
@@ -776,12 +814,12 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order,
         const int32_t n_warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
         const bool few = n_wave <= n_warps;
         const int32_t shape = wave.force ? wave.all
-                              : few ? wave.few : counters[8] > KeyCompact::ROWS_MAX ? wave.tail : wave.all;
+                              : few ? wave.few : max_rows > KeyCompact::ROWS_MAX ? wave.tail : wave.all;
         // the compact key when every pair of the call (so every warp-per-pair
         // pair) has at most 2047 rows
         wave_stream_any(shape, in, out, order, n_wave, !few, wave.serial, wave_ticket,
                         (const char *)s_inc, slots, lane, fallback, fallback_count, err, one,
-                        !wide_key && counters[8] <= KeyCompact::ROWS_MAX);
+                        !wide_key && max_rows <= KeyCompact::ROWS_MAX);
     }
     const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int2 *win = window + (size_t)gwarp * (size_t)W * 32 + lane;
@@ -1164,7 +1202,7 @@ static int32_t g_wave_rows = 0;
 // first).  Pairs of at most G strips never rotate: those with a longer side of
 // at most 50, whose band is the whole matrix, have at most 7 strips of 8 rows;
 // and where the band is too wide for 32 lanes of 16 rows, every pair has at most
-// 512 rows (wave_split_kernel), 32 strips.  0: none.
+// 512 rows (wave_split), 32 strips.  0: none.
 static int32_t wave_group(int32_t R, int32_t w) {
     if (w >= 1)
         for (int32_t G = 8; G <= 32; G <<= 1)
@@ -1262,7 +1300,8 @@ static int32_t strip_threads(int32_t rows) {
 
 template <int R, int V, int NT>
 static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *order,
-                             const int32_t *counters, const int32_t *inc, int32_t wmax,
+                             const uint32_t *keys, int32_t *counters, const int32_t *inc, WaveRoute route,
+                             int32_t wmax,
                              int32_t *ticket, int32_t *fallback, int32_t *fb_count,
                              int32_t *err, cudaStream_t st, SwCounters *ctr) {
     int32_t status = CK_OK;
@@ -1284,7 +1323,8 @@ static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *o
     if (blocks < 1) blocks = 1;
     int2 *window = (int2 *)scratch(SLOT_WINDOW, (size_t)blocks * per_block, &status);
     if (!window) return status;
-    kern<<<blocks, NT, smem, st>>>(in, out, order, counters, inc, window, W, ticket,
+    route.lanes = (int64_t)sm_count() * NT;
+    kern<<<blocks, NT, smem, st>>>(in, out, order, keys, counters, inc, route, window, W, ticket,
                                               ticket + 5, fallback, fb_count, err, 1, wave_shapes(in.band_width),
                                               g_wide_key);
     CK_CUDA(cudaGetLastError());
@@ -1294,14 +1334,15 @@ static int32_t launch_strips(const SwIn &in, const SwOut &out, const uint32_t *o
 
 template <int R, int NT>
 static int32_t launch_strips_m(const SwIn &in, const SwOut &out, const uint32_t *order,
-                               const int32_t *counters, const int32_t *inc, int32_t wmax,
+                               const uint32_t *keys, int32_t *counters, const int32_t *inc, WaveRoute route,
+                               int32_t wmax,
                                int32_t *ticket, int32_t *fallback, int32_t *fb_count,
                                int32_t *err, cudaStream_t st, SwCounters *ctr) {
     switch (g_variant >= 0 ? g_variant : (R <= 8 ? 3 : 1)) {
-        case 0: return launch_strips<R, 0, NT>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
-        case 2: return launch_strips<R, 2, NT>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
-        case 3: return launch_strips<R, 3, NT>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
-        default: return launch_strips<R, 1, NT>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
+        case 0: return launch_strips<R, 0, NT>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
+        case 2: return launch_strips<R, 2, NT>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
+        case 3: return launch_strips<R, 3, NT>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
+        default: return launch_strips<R, 1, NT>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
     }
 }
 
@@ -1309,19 +1350,20 @@ static int32_t launch_strips_m(const SwIn &in, const SwOut &out, const uint32_t 
 // 512 for 16, 256 for 24 and 32)
 template <int R>
 static int32_t launch_strips_v(const SwIn &in, const SwOut &out, const uint32_t *order,
-                               const int32_t *counters, const int32_t *inc, int32_t wmax,
+                               const uint32_t *keys, int32_t *counters, const int32_t *inc, WaveRoute route,
+                               int32_t wmax,
                                int32_t *ticket, int32_t *fallback, int32_t *fb_count,
                                int32_t *err, cudaStream_t st, SwCounters *ctr, int32_t nt) {
     if constexpr (R >= 24) {
-        return launch_strips_m<R, 256>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
+        return launch_strips_m<R, 256>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
     } else if constexpr (R == 8) {
         if (nt == 768)
-            return launch_strips_m<R, 768>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
+            return launch_strips_m<R, 768>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
         if (nt == 640)
-            return launch_strips_m<R, 640>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
-        return launch_strips_m<R, 512>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
+            return launch_strips_m<R, 640>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
+        return launch_strips_m<R, 512>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
     } else {
-        return launch_strips_m<R, 512>(in, out, order, counters, inc, wmax, ticket, fallback, fb_count, err, st, ctr);
+        return launch_strips_m<R, 512>(in, out, order, keys, counters, inc, route, wmax, ticket, fallback, fb_count, err, st, ctr);
     }
 }
 
@@ -1333,19 +1375,23 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
         return CK_ERR_UNSUPPORTED;
     }
     // counters: [0] eligible, [1] fallback list length, [2] ticket, [3] overflow re-runs,
-    // [4..5] cells (u64)
+    // [4..5] cells (u64), [6] pairs one warp per pair, [7] their ticket
     int32_t *cnt = (int32_t *)scratch(SLOT_COUNTERS, 256, &status);
     if (!cnt) return status;
-    CK_CUDA(cudaMemsetAsync(cnt, 0, 64, st));
     unsigned long long *cells = (unsigned long long *)(cnt + 4);
-
     uint8_t *ok = (uint8_t *)scratch(SLOT_SEQ_OK, (size_t)(in.n_seqs > 0 ? in.n_seqs : 1), &status);
     if (!ok) return status;
-    CK_CUDA(cudaMemsetAsync(ok, 0, (size_t)(in.n_seqs > 0 ? in.n_seqs : 1), st));
     int32_t *inc = (int32_t *)scratch(SLOT_INC, INC_ENTRIES * sizeof(int32_t), &status);
     if (!inc) return status;
-    build_inc_kernel<<<(INC_ENTRIES + 127) / 128, 128, 0, st>>>(d_sub, inc);
-    CK_CUDA(cudaGetLastError());
+    {
+        // residue codes of every sequence, or of the pairs' where those are fewer
+        const bool by_pair = 2 * M < in.n_seqs;
+        const int64_t items = by_pair ? 2 * M : in.n_seqs;
+        const int64_t want = (items * CODE_LANES + 255) / 256, most = 32 * (int64_t)sm_count();
+        sw_tables_kernel<<<(unsigned)(want < 1 ? 1 : want < most ? want : most), 256, 0, st>>>(d_sub, inc, cnt, in,
+                                                                                              items, by_pair, ok);
+        CK_CUDA(cudaGetLastError());
+    }
 
     const size_t n = (size_t)(M > 0 ? M : 1);
     uint32_t *k0 = (uint32_t *)scratch(SLOT_SORT_KEYS, n * 4, &status);
@@ -1388,28 +1434,25 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
         // 512 and 384: band 16 1.31 and 1.42 ms, 100 4.08 and 4.00, 200 7.00 and
         // 6.78; 60,000 at band 50 2.25 and 1.69)
         const int32_t min_rows = in.band_width > 24 ? g_wave_min_rows / 4 * 3 : g_wave_min_rows;
-        wave_split_kernel<<<1, 32, 0, st>>>(dk.Current(), cnt, in.band_width, g_wave_all_below, min_rows,
-                                            g_wave_adaptive, (int64_t)sm_count() * nt);
-        CK_CUDA(cudaGetLastError());
+        const WaveRoute route{in.band_width, g_wave_all_below, min_rows, g_wave_adaptive, 0};
         // profiling events bracket the alignment kernel
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;
         if (profile_events(&ev0, &ev1)) CK_CUDA(cudaEventRecord(ev0, st));
         switch (rows) {
             case 8:
-                CK_TRY(launch_strips_v<8>(in, out, order, cnt, inc, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
+                CK_TRY(launch_strips_v<8>(in, out, order, dk.Current(), cnt, inc, route, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
                 break;
             case 24:
-                CK_TRY(launch_strips_v<24>(in, out, order, cnt, inc, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
+                CK_TRY(launch_strips_v<24>(in, out, order, dk.Current(), cnt, inc, route, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
                 break;
             case 32:
-                CK_TRY(launch_strips_v<32>(in, out, order, cnt, inc, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
+                CK_TRY(launch_strips_v<32>(in, out, order, dk.Current(), cnt, inc, route, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
                 break;
             default:
-                CK_TRY(launch_strips_v<16>(in, out, order, cnt, inc, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
+                CK_TRY(launch_strips_v<16>(in, out, order, dk.Current(), cnt, inc, route, wmax, cnt + 2, fb, cnt + 1, d_err, st, ctr, nt));
                 break;
         }
         if (ev1) CK_CUDA(cudaEventRecord(ev1, st));
-        if (ctr) ctr->launches += 1;
     }
     // plain kernel over the fallback list (its length is read on the device)
     CK_TRY(sw_plain_launch(in, out, M, fb, cnt + 1, d_err, st, ctr));

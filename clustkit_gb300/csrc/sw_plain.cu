@@ -142,7 +142,7 @@ int32_t sw_plain_launch(const SwIn &in, const SwOut &out, int64_t M, const int32
     // Workspace budget: at most 4 GiB, at most one slot per work item.
     const int64_t budget = (int64_t)4 << 30;
     int64_t slots = budget / (stride * (int64_t)sizeof(int4));
-    const int64_t want = d_count ? (int64_t)sm_count() * 8 * 128 : M;
+    const int64_t want = d_count && M > (int64_t)sm_count() * 8 * 128 ? (int64_t)sm_count() * 8 * 128 : M;
     if (slots > want) slots = want;
     slots = (slots + 127) / 128 * 128;
     if (slots < 128) slots = 128;
