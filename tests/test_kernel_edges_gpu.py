@@ -214,3 +214,31 @@ def test_wave_group_shapes(ck, bw, hinted, long_rows):
             assert _lib.sw_counters()["wave"] > 2000
     finally:
         _lib.set_config(_lib.CFG_WAVE_STREAM, keep)
+
+
+def test_context_scratch_is_handed_on_clean(ck, small_db):
+    """A context takes over the last destroyed one's scratch: its unread errors
+    and its Phase-B bins (left by a call that ran out of them) must not show,
+    and contexts alive at the same time share nothing."""
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.search import Scoring, _Slot, search_batch
+    db, ss = small_db
+    qs = [ss.seq(i).copy() for i in (5, 300, 900)]
+    kw = dict(top_k=10, max_cands=100, kmer_score_thresh=0, min_diag_hits=2, use_c_scoring=True, use_c_sw=True)
+    hits = lambda res: [[(h.target, h.score, h.identity, h.rank) for h in q] for q in res]
+    first = hits(search_batch(db, qs, **kw))
+    slot = _Slot(db, 0, 100)
+    slot.bins_bound = lambda nq, res, sc: 3  # far too few bins: the call leaves them dirty and an error unread
+    slot.launch(qs, 2, 0, min_diag_hits=2, use_c_scoring=True, use_c_sw=True)
+    slot.event.synchronize()
+    slot.close()
+    assert hits(search_batch(db, qs, **kw)) == first
+    a, b = _Slot(db, 0, 100), _Slot(db, 0, 100)
+    try:
+        assert a.ctx != b.ctx
+        for s in (a, b):
+            assert hits(search_batch(db, qs[::-1], slot=s, **kw)) == first[::-1]
+    finally:
+        a.close()
+        b.close()
+    assert _lib.load().ck_ctx_status(a.ctx or 1 << 20, None) == _lib.CK_ERR_INVALID_ARGUMENT
