@@ -242,3 +242,19 @@ def test_context_scratch_is_handed_on_clean(ck, small_db):
         a.close()
         b.close()
     assert _lib.load().ck_ctx_status(a.ctx or 1 << 20, None) == _lib.CK_ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("n", [32, 33, 160, 1000, 1001, 1300])
+def test_lsh_large_buckets(ck, n):
+    """Buckets either side of the one-thread limit and of the cap, several at once."""
+    rng = np.random.default_rng(n)
+    sk = rng.integers(0, 2 ** 60, (2 * n + 50, 4)).astype(np.uint64)
+    sk[:n, 0] = 7
+    sk[n:2 * n, 1] = 9
+    got = lsh_candidates_device(sk, 12, 1, 3).cpu().numpy()
+    k = min(n, 1000)
+    a, b = np.triu_indices(k, 1)
+    want = np.concatenate([np.stack([a, b], 1), np.stack([a, b], 1) + n]).astype(np.int32)
+    idx, _ = band_parameters(4, 12, 1, 3)
+    assert {0, 1} <= set(idx[:, 0].tolist())
+    assert np.array_equal(got, want)
