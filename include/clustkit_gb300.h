@@ -431,7 +431,8 @@ int32_t ck_search_kmer_candidates_device(int32_t ctx, const uint8_t *d_qflat, in
  * number of entries.  ck_connected_components_device: component labels of
  * the undirected graph on the pairs, numbered in order of each component's
  * smallest node as scipy's connected_components does (clustkit/cluster.py:
- * 43-55); *out_n_components, *out_rounds (may be NULL) the union-find rounds.
+ * 43-55); *out_n_components, *out_rounds (may be NULL) the passes over the
+ * pairs (1, or 0 without pairs).
  * Both blocking. */
 int32_t ck_graph_csr_device(int32_t ctx, const int32_t *d_pairs, const float *d_sims, int64_t K, int64_t N,
                             int64_t *d_indptr, int32_t *d_indices, float *d_data, int64_t *out_nnz,

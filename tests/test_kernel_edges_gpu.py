@@ -244,6 +244,28 @@ def test_context_scratch_is_handed_on_clean(ck, small_db):
     assert _lib.load().ck_ctx_status(a.ctx or 1 << 20, None) == _lib.CK_ERR_INVALID_ARGUMENT
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 65536, 65537])
+def test_graph_key_widths(ck, n):
+    """Rows and columns packed in as many bits as n needs, n at powers of two;
+    chains, repeats and self-loops hooked in one pass."""
+    import oracle.graph_oracle as go
+    from clustkit_gb300 import graph
+    rng = np.random.default_rng(n)
+    ends = np.stack([np.arange(n), np.minimum(np.arange(n) + 1, n - 1)], 1)[rng.permutation(n)]
+    pairs = np.concatenate([ends[: 3 * n // 4 + 1], rng.integers(0, n, (n // 8 + 1, 2)), ends[:2]]).astype(np.int32)
+    w = rng.random(len(pairs)).astype(np.float32)
+    got, want = graph.build_similarity_graph(n, pairs, w), go.build_similarity_graph(n, pairs, w)
+    assert np.array_equal(got.indptr, want.indptr) and np.array_equal(got.indices, want.indices)
+    assert np.allclose(got.data, want.data, rtol=1e-6)
+    k, labels, _ = graph.connected_components_device(pairs, n)
+    ref = go.cluster_connected_components(want)
+    assert np.array_equal(labels.cpu().numpy(), ref) and k == int(ref.max()) + 1
+    with pytest.raises(Exception):
+        graph.connected_components_device(np.array([[0, n]], np.int32), n)
+    k, labels, _ = graph.connected_components_device(pairs, n)  # the error above is not seen again
+    assert np.array_equal(labels.cpu().numpy(), ref)
+
+
 @pytest.mark.parametrize("n", [32, 33, 160, 1000, 1001, 1300])
 def test_lsh_large_buckets(ck, n):
     """Buckets either side of the one-thread limit and of the cap, several at once."""
