@@ -16,11 +16,14 @@
 //
 // Layout: sketches are transposed once to [s][N] so a table's band columns are
 // read coalesced.  Tables are processed in batches (as many as fit a few GB of
-// scratch; every table at once for moderate N): a batch's bucket ids are keyed
-// (table, id) and sorted together, stably, so each bucket is one run in table
-// order with its members in ascending sequence id, and the run-length, scan,
-// pair-count and emit steps cover the whole batch in one launch each; one
-// radix sort + unique de-duplicates all tables.
+// scratch; every table at once for moderate N): a batch's bucket ids are made
+// in (table, sequence) order and sorted together, stably, so each bucket is one
+// run with its members in ascending sequence id, and the run, scan, pair-count
+// and emit steps cover the whole batch in one launch each; one radix sort +
+// unique de-duplicates all tables.  The sort moves 12 bytes an item and looks
+// at as many bits of the id as tell a table's buckets apart, and not at the
+// table (6 passes over 12.8 M items, 0.84 ms; sorted by table and all 64 bits
+// as 16-byte keys, it was 9 passes and 1.56).
 //
 // Tables that read the same columns in the same order have the same buckets,
 // whatever their seeds: the seed adds one constant (seed * mul^bands) to every
@@ -34,12 +37,12 @@
 // several, the first one's count times their number (and a quarter) sizes it,
 // and only a call that outgrows that runs its batches a second time, into a
 // buffer of the counted size.  100,000 sequences, 448 tables of one band: the
-// whole call 24.3 -> 8.2 ms (the old form hashed and sorted all 448
+// whole call 24.0 -> 6.3 ms (the old form hashed and sorted all 448
 // tables twice).
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_run_length_encode.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <cmath>
 #include <set>
@@ -72,22 +75,11 @@ __global__ void transpose_sketch_kernel(const uint64_t *__restrict__ sk, int64_t
     }
 }
 
-// A batch's sort key: the table (within the batch) above the bucket id.
-struct LshKey {
-    uint64_t h;  // bucket id in its table
-    uint32_t t;  // table, counted from the batch's first
-    uint32_t pad;
-};
-__host__ __device__ inline bool operator==(const LshKey &a, const LshKey &b) { return a.h == b.h && a.t == b.t; }
-// radix-sort view of a key: (table, bucket id), most significant first
-struct LshKeyParts {
-    __host__ __device__ ::cuda::std::tuple<uint32_t &, uint64_t &> operator()(LshKey &k) const { return {k.t, k.h}; }
-};
-
-// bucket ids of tables t0 .. t0 + tb - 1 for every sequence, table-major
+// bucket ids of tables t0 .. t0 + tb - 1 for every sequence, table-major; the
+// value is the item's number, table * n + sequence (tables from the batch's first)
 __global__ void lsh_hash_kernel(const uint64_t *__restrict__ skT, int64_t n, const int32_t *__restrict__ band,
                                 int32_t nb, const uint64_t *__restrict__ seeds, int32_t t0, int32_t tb,
-                                LshKey *__restrict__ keys, int32_t *__restrict__ vals) {
+                                uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
     const int64_t total = (int64_t)tb * n;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
          k += (int64_t)gridDim.x * blockDim.x) {
@@ -99,24 +91,46 @@ __global__ void lsh_hash_kernel(const uint64_t *__restrict__ skT, int64_t n, con
         for (int32_t b = 0; b < nb; ++b) h = h * LSH_MUL + skT[(int64_t)bt[b] * n + i];
         h = (h ^ (h >> 33)) * LSH_FMIX;
         h ^= h >> 33;
-        keys[k] = LshKey{h, (uint32_t)tl, 0u};
-        vals[k] = (int32_t)i;
+        keys[k] = h;
+        vals[k] = (uint32_t)k;
     }
 }
 
-// the batch's pair total, pair_off[runs], for the host
+// True where a bucket begins in the sorted items.  Two different buckets of a
+// table that share the sorted bits may lie mixed: that sets *mixed.
+struct LshBucketStart {
+    const uint64_t *keys;
+    const uint32_t *vals;
+    uint32_t n;
+    int32_t unsorted;  // low bits of a key that were not sorted
+    int32_t *mixed;
+    __device__ bool operator()(int32_t i) const {
+        if (i == 0) return true;
+        const uint64_t a = keys[i - 1], b = keys[i];
+        if (a >> unsorted != b >> unsorted || vals[i - 1] / n != vals[i] / n) return true;
+        if (a != b) *mixed = 1;
+        return a != b;
+    }
+};
+
+// the batch's pair total, pair_off[runs], for the host; -1 of mixed buckets
 __global__ void lsh_total_kernel(const int32_t *__restrict__ n_runs, const int64_t *__restrict__ pair_off,
-                                 int64_t *__restrict__ total) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *total = pair_off[*n_runs];
+                                 const int32_t *__restrict__ mixed, int64_t *__restrict__ total) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) *total = *mixed ? -1 : pair_off[*n_runs];
 }
 
-// pairs a bucket of `count` members contributes (first 1000 only)
-__global__ void lsh_bucket_pairs_kernel(const int32_t *__restrict__ counts, const int32_t *__restrict__ n_runs,
-                                        int64_t n, int64_t *__restrict__ npairs) {
+// members of bucket r that count (the first 1000), of the R buckets of m items
+__device__ __forceinline__ int32_t lsh_members(const int32_t *__restrict__ starts, int64_t r, int32_t R, int64_t m) {
+    return min((r + 1 < R ? starts[r + 1] : (int32_t)m) - starts[r], LSH_MAX_BUCKET);
+}
+
+// pairs a bucket contributes; zero past the last one
+__global__ void lsh_bucket_pairs_kernel(const int32_t *__restrict__ starts, const int32_t *__restrict__ n_runs,
+                                        int64_t m, int64_t *__restrict__ npairs) {
     const int32_t R = *n_runs;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= m; r += (int64_t)gridDim.x * blockDim.x) {
         if (r >= R) { npairs[r] = 0; continue; }
-        const int64_t c = counts[r] < LSH_MAX_BUCKET ? counts[r] : LSH_MAX_BUCKET;
+        const int64_t c = lsh_members(starts, r, R, m);
         npairs[r] = c >= 2 ? c * (c - 1) / 2 : 0;
     }
 }
@@ -126,25 +140,26 @@ __global__ void lsh_bucket_pairs_kernel(const int32_t *__restrict__ counts, cons
 // range), and lists larger buckets for lsh_emit_big_kernel.  The raw pairs
 // are sorted and de-duplicated afterwards, so only the set matters.
 constexpr int32_t LSH_SMALL_BUCKET = 32;
-__global__ void lsh_emit_runs_kernel(const int32_t *__restrict__ order, const int32_t *__restrict__ run_start,
-                                     const int32_t *__restrict__ counts, const int64_t *__restrict__ pair_off,
-                                     const int32_t *__restrict__ n_runs, int64_t n, uint64_t *__restrict__ out,
-                                     int32_t *__restrict__ big, int32_t *__restrict__ n_big) {
+__global__ void lsh_emit_runs_kernel(const uint32_t *__restrict__ order, const int32_t *__restrict__ run_start,
+                                     const int64_t *__restrict__ pair_off, const int32_t *__restrict__ n_runs,
+                                     int64_t m, uint32_t n, uint64_t *__restrict__ out, int32_t *__restrict__ big,
+                                     int32_t *__restrict__ n_big) {
     const int32_t R = *n_runs;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < R; r += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t c = counts[r] < LSH_MAX_BUCKET ? counts[r] : LSH_MAX_BUCKET;
+        const int32_t c = lsh_members(run_start, r, R, m);
         if (c < 2) continue;
         if (c > LSH_SMALL_BUCKET) {
             big[atomicAdd(n_big, 1)] = (int32_t)r;
             continue;
         }
         const int32_t s0 = run_start[r];
+        const uint32_t base = order[s0] / n * n;  // the table's first item
         uint64_t *o = out + pair_off[r];
         for (int32_t y = 1; y < c; ++y) {
-            const int64_t b = order[s0 + y];
+            const uint32_t b = order[s0 + y] - base;
             for (int32_t x = 0; x < y; ++x) {
-                const int64_t v = order[s0 + x];
-                *o++ = v < b ? (uint64_t)(v * n + b) : (uint64_t)(b * n + v);
+                const uint32_t v = order[s0 + x] - base;  // below b: members are in ascending order
+                *o++ = (uint64_t)v * n + b;
             }
         }
     }
@@ -154,28 +169,26 @@ __global__ void lsh_emit_runs_kernel(const int32_t *__restrict__ order, const in
 // LSH_BIG_PARTS); a bucket's members are dealt out over its blocks' warps, whose
 // lanes split each member's pairs with the members before it.  (A warp a
 // bucket left the largest, half a million pairs, to one warp: 1.08 ms of the
-// call on 100,000 sequences, now 0.15.)
+// call on 100,000 sequences, now 0.11.)
 constexpr int LSH_BIG_PARTS = 16;
-__global__ void lsh_emit_big_kernel(const int32_t *__restrict__ order, const int32_t *__restrict__ run_start,
-                                    const int32_t *__restrict__ counts, const int64_t *__restrict__ pair_off,
-                                    const int32_t *__restrict__ big, const int32_t *__restrict__ n_big, int64_t n,
-                                    uint64_t *__restrict__ out) {
+__global__ void lsh_emit_big_kernel(const uint32_t *__restrict__ order, const int32_t *__restrict__ run_start,
+                                    const int64_t *__restrict__ pair_off, const int32_t *__restrict__ n_runs,
+                                    int64_t m, const int32_t *__restrict__ big, const int32_t *__restrict__ n_big,
+                                    uint32_t n, uint64_t *__restrict__ out) {
     const int32_t lane = threadIdx.x & 31;
     const int32_t nb = *n_big;
     const int32_t warps = (int32_t)(blockDim.x >> 5) * LSH_BIG_PARTS;
     const int32_t warp = (int32_t)(blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5));
     for (int32_t w = blockIdx.x; w < nb; w += gridDim.x) {
         const int32_t r = big[w];
-        const int32_t c = counts[r] < LSH_MAX_BUCKET ? counts[r] : LSH_MAX_BUCKET;
+        const int32_t c = lsh_members(run_start, r, *n_runs, m);
         const int32_t s0 = run_start[r];
+        const uint32_t base = order[s0] / n * n;
         uint64_t *o = out + pair_off[r];
         for (int32_t y = 1 + warp; y < c; y += warps) {
-            const int64_t b = order[s0 + y];
+            const uint32_t b = order[s0 + y] - base;
             uint64_t *row = o + (int64_t)y * (y - 1) / 2;
-            for (int32_t x = lane; x < y; x += 32) {
-                const int64_t v = order[s0 + x];
-                row[x] = v < b ? (uint64_t)(v * n + b) : (uint64_t)(b * n + v);
-            }
+            for (int32_t x = lane; x < y; x += 32) row[x] = (uint64_t)(order[s0 + x] - base) * n + b;
         }
     }
 }
@@ -221,38 +234,38 @@ static int32_t lsh_impl(void *pv) {
         }
     }
     const int32_t T = (int32_t)seed_h.size();
-    // tables per batch: about 4 GB of keys, values and run data (80 B an item),
-    // and fewer than 2^31 items (the run-length encoder counts in int)
-    int64_t tb64 = ((int64_t)4 << 30) / (80 * n);
+    // tables per batch: about 4 GB of keys, values and run data (40 B an item),
+    // and fewer than 2^31 items (runs are counted in int)
+    int64_t tb64 = ((int64_t)4 << 30) / (40 * n);
     if (tb64 * n > ((int64_t)1 << 30)) tb64 = ((int64_t)1 << 30) / n;
     if (tb64 < 1) tb64 = 1;
     if (tb64 > T) tb64 = T;
     const int32_t TB = (int32_t)tb64;
     const int64_t items = (int64_t)TB * n;
-    int tbits = 1;  // bits of a table index within a batch
-    while (tbits < 31 && ((int64_t)1 << tbits) < TB) ++tbits;
+    // Sorted bits of a bucket id, from the top: as many (whole digits) as leave
+    // two buckets of a table less than one chance in 64 to share them, in all
+    // the batch's n^2 TB / 2 comparisons.  A batch where some do is sorted
+    // again by all 64.
+    int sorted = 8;
+    while (sorted < 64 && std::ldexp((double)n * (double)n * TB, 5 - sorted) > 1.0) sorted += 8;
     // band indices and seeds on the device
     int32_t *d_band = (int32_t *)scratch(SLOT_SEARCH_TMP0, band_h.size() * 4 + (size_t)T * 8 + 16, &status);
     uint64_t *skT = (uint64_t *)scratch(SLOT_SEARCH_TMP1, (size_t)n * a.s * 8, &status);
-    LshKey *k0 = (LshKey *)scratch(SLOT_SEARCH_TMP2, (size_t)items * sizeof(LshKey) * 2, &status);
-    int32_t *v0 = (int32_t *)scratch(SLOT_SEARCH_TMP3, (size_t)items * 4 * 2, &status);
-    // run data: unique keys (unused), counts, starts (int32), pair offsets
-    // (int64, items + 1), then the list of buckets of more than 32 members (at
-    // most items / 33 of them)
+    uint64_t *k0 = (uint64_t *)scratch(SLOT_SEARCH_TMP2, (size_t)items * 8 * 2, &status);
+    uint32_t *v0 = (uint32_t *)scratch(SLOT_SEARCH_TMP3, (size_t)items * 4 * 2, &status);
+    // run data: pair offsets (items + 1), starts, then the list of buckets of
+    // more than 32 members (at most items / 33 of them)
     const int64_t n_big_max = items / (LSH_SMALL_BUCKET + 1) + 1;
-    char *rle = (char *)scratch(SLOT_SEARCH_TMP4, (size_t)items * (sizeof(LshKey) + 4 + 4 + 8) + 64 + (size_t)n_big_max * 4,
-                                &status);
+    char *rle = (char *)scratch(SLOT_SEARCH_TMP4, (size_t)(items + 1) * 8 + (size_t)(items + n_big_max) * 4, &status);
     int32_t *n_runs = (int32_t *)scratch(SLOT_MAXLEN, 64, &status);
     if (!d_band || !skT || !k0 || !v0 || !rle || !n_runs) return status;
-    int32_t *n_big = n_runs + 8;
+    int32_t *n_big = n_runs + 8, *d_mixed = n_runs + 9;
     uint64_t *d_seeds = (uint64_t *)(((uintptr_t)(d_band + band_h.size()) + 15) & ~(uintptr_t)15);
-    LshKey *k1 = k0 + items;
-    int32_t *v1 = v0 + items;
-    LshKey *uniq = (LshKey *)rle;
-    int32_t *counts = (int32_t *)(uniq + items);
-    int32_t *starts = counts + items;
-    int64_t *pair_off = (int64_t *)(starts + items);  // 8-byte aligned: items * 24 bytes before
-    int32_t *big = (int32_t *)(pair_off + items + 1);
+    uint64_t *k1 = k0 + items;
+    uint32_t *v1 = v0 + items;
+    int64_t *pair_off = (int64_t *)rle;
+    int32_t *starts = (int32_t *)(pair_off + items + 1);
+    int32_t *big = starts + items;
     int64_t *d_total = (int64_t *)(n_runs + 4);
     CK_CUDA(cudaMemcpyAsync(d_band, band_h.data(), band_h.size() * 4, cudaMemcpyHostToDevice, st));
     CK_CUDA(cudaMemcpyAsync(d_seeds, seed_h.data(), (size_t)T * 8, cudaMemcpyHostToDevice, st));
@@ -262,55 +275,60 @@ static int32_t lsh_impl(void *pv) {
         CK_CUDA(cudaGetLastError());
     }
     // temp storage sizes (the largest of the calls below, at a full batch)
-    size_t t_sort = 0, t_rle = 0, t_scan = 0, t_scan2 = 0;
+    const thrust::counting_iterator<int32_t> numbers(0);
+    size_t t_sort = 0, t_select = 0, t_scan = 0;
     {
-        cub::DoubleBuffer<LshKey> dk(k0, k1);
-        cub::DoubleBuffer<int32_t> dv(v0, v1);
-        CK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t_sort, dk, dv, items, LshKeyParts{}, 0, 64 + tbits, st));
-        CK_CUDA(cub::DeviceRunLengthEncode::Encode(nullptr, t_rle, k0, uniq, counts,
-                                                   n_runs, (int)items, st));
-        CK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, counts, starts, (int)items, st));
-        CK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t_scan2, pair_off, pair_off, (int)items + 1, st));
+        cub::DoubleBuffer<uint64_t> dk(k0, k1);
+        cub::DoubleBuffer<uint32_t> dv(v0, v1);
+        CK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t_sort, dk, dv, items, 0, 64, st));
+        CK_CUDA(cub::DeviceSelect::If(nullptr, t_select, numbers, starts, n_runs, (int)items,
+                                      LshBucketStart{k0, v0, (uint32_t)n, 0, d_mixed}, st));
+        CK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, pair_off, pair_off, (int)items + 1, st));
     }
-    const size_t t_max = std::max(std::max(t_sort, t_rle), std::max(t_scan, t_scan2));
+    const size_t t_max = std::max(t_sort, std::max(t_select, t_scan));
     void *tmp = scratch(SLOT_SORT_TEMP, t_max, &status);
     if (!tmp) return status;
 
-    // one batch: bucket ids, stable sort, runs, pair offsets; *total its pair count
-    auto batch = [&](int32_t t0, int32_t tb, cub::DoubleBuffer<LshKey> &dk, cub::DoubleBuffer<int32_t> &dv,
-                     int64_t *total) -> int32_t {
+    // one batch: bucket ids, stable sort, runs, pair offsets; *total its pair
+    // count.  Items are made in (table, sequence) order, so equal sorted bits
+    // keep a table's items together and their sequences ascending.
+    auto batch = [&](int32_t t0, int32_t tb, cub::DoubleBuffer<uint32_t> &dv, int64_t *total) -> int32_t {
         const int64_t m = (int64_t)tb * n;
-        lsh_hash_kernel<<<grid_of(m, 256), 256, 0, st>>>(skT, n, d_band, a.bands, d_seeds, t0, tb, dk.Current(),
-                                                         dv.Current());
-        CK_CUDA(cudaGetLastError());
-        size_t tbytes = t_max;
-        CK_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbytes, dk, dv, m, LshKeyParts{}, 0, 64 + tbits, st));
-        tbytes = t_max;
-        CK_CUDA(cub::DeviceRunLengthEncode::Encode(tmp, tbytes, dk.Current(), uniq, counts,
-                                                   n_runs, (int)m, st));
-        tbytes = t_max;
-        CK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tbytes, counts, starts, (int)m, st));
-        lsh_bucket_pairs_kernel<<<grid_of(m + 1, 256), 256, 0, st>>>(counts, n_runs, m, pair_off);
-        CK_CUDA(cudaGetLastError());
-        tbytes = t_max;
-        CK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tbytes, pair_off, pair_off, (int)m + 1, st));
-        // pair_off[R] (R = runs) is the batch's total; runs <= m, entries past R are 0
-        lsh_total_kernel<<<1, 32, 0, st>>>(n_runs, pair_off, d_total);
-        CK_CUDA(cudaGetLastError());
-        CK_CUDA(cudaMemcpyAsync(total, d_total, 8, cudaMemcpyDeviceToHost, st));
-        CK_CUDA(cudaStreamSynchronize(st));
-        return CK_OK;
+        for (int by = sorted;; by = 64) {
+            cub::DoubleBuffer<uint64_t> dk(k0, k1);
+            dv = cub::DoubleBuffer<uint32_t>(v0, v1);
+            lsh_hash_kernel<<<grid_of(m, 256), 256, 0, st>>>(skT, n, d_band, a.bands, d_seeds, t0, tb, dk.Current(),
+                                                             dv.Current());
+            CK_CUDA(cudaGetLastError());
+            CK_CUDA(cudaMemsetAsync(d_mixed, 0, 4, st));
+            size_t tbytes = t_max;
+            CK_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbytes, dk, dv, m, 64 - by, 64, st));
+            tbytes = t_max;
+            CK_CUDA(cub::DeviceSelect::If(tmp, tbytes, numbers, starts, n_runs, (int)m,
+                                          LshBucketStart{dk.Current(), dv.Current(), (uint32_t)n, 64 - by, d_mixed},
+                                          st));
+            lsh_bucket_pairs_kernel<<<grid_of(m + 1, 256), 256, 0, st>>>(starts, n_runs, m, pair_off);
+            CK_CUDA(cudaGetLastError());
+            tbytes = t_max;
+            CK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tbytes, pair_off, pair_off, (int)m + 1, st));
+            // pair_off[R] (R = runs) is the batch's total; runs <= m, entries past R are 0
+            lsh_total_kernel<<<1, 32, 0, st>>>(n_runs, pair_off, d_mixed, d_total);
+            CK_CUDA(cudaGetLastError());
+            CK_CUDA(cudaMemcpyAsync(total, d_total, 8, cudaMemcpyDeviceToHost, st));
+            CK_CUDA(cudaStreamSynchronize(st));
+            if (*total >= 0) return CK_OK;
+        }
     };
 
     // emission of the batch just prepared, at raw pair `at` of the buffer
-    auto emit = [&](int32_t tb, cub::DoubleBuffer<int32_t> &dv, uint64_t *out) -> int32_t {
+    auto emit = [&](int32_t tb, cub::DoubleBuffer<uint32_t> &dv, uint64_t *out) -> int32_t {
         const int64_t m = (int64_t)tb * n;
         CK_CUDA(cudaMemsetAsync(n_big, 0, 4, st));
-        lsh_emit_runs_kernel<<<grid_of(m, 256), 256, 0, st>>>(dv.Current(), starts, counts, pair_off, n_runs, n, out,
-                                                              big, n_big);
+        lsh_emit_runs_kernel<<<grid_of(m, 256), 256, 0, st>>>(dv.Current(), starts, pair_off, n_runs, m, (uint32_t)n,
+                                                              out, big, n_big);
         CK_CUDA(cudaGetLastError());
-        lsh_emit_big_kernel<<<dim3((unsigned)sm_count(), LSH_BIG_PARTS), 128, 0, st>>>(dv.Current(), starts, counts,
-                                                                                      pair_off, big, n_big, n, out);
+        lsh_emit_big_kernel<<<dim3((unsigned)sm_count(), LSH_BIG_PARTS), 128, 0, st>>>(
+            dv.Current(), starts, pair_off, n_runs, m, big, n_big, (uint32_t)n, out);
         CK_CUDA(cudaGetLastError());
         return CK_OK;
     };
@@ -323,10 +341,9 @@ static int32_t lsh_impl(void *pv) {
     bool fits = true;
     for (int32_t b = 0; b < n_batches; ++b) {
         const int32_t t0 = b * TB, tb = T - t0 < TB ? T - t0 : TB;
-        cub::DoubleBuffer<LshKey> dk(k0, k1);
-        cub::DoubleBuffer<int32_t> dv(v0, v1);
+        cub::DoubleBuffer<uint32_t> dv(v0, v1);
         int64_t tot = 0;
-        CK_TRY(batch(t0, tb, dk, dv, &tot));
+        CK_TRY(batch(t0, tb, dv, &tot));
         if (b == 0) {
             room = n_batches == 1 ? tot : (tot + tot / 4) * n_batches;
             if (room > 0) rk = (uint64_t *)scratch(SLOT_FALLBACK, (size_t)room * 8 * 2, &status);
@@ -349,10 +366,9 @@ static int32_t lsh_impl(void *pv) {
         int64_t at = 0;
         for (int32_t b = 0; b < n_batches; ++b) {
             const int32_t t0 = b * TB, tb = T - t0 < TB ? T - t0 : TB;
-            cub::DoubleBuffer<LshKey> dk(k0, k1);
-            cub::DoubleBuffer<int32_t> dv(v0, v1);
+            cub::DoubleBuffer<uint32_t> dv(v0, v1);
             int64_t tot = 0;
-            CK_TRY(batch(t0, tb, dk, dv, &tot));
+            CK_TRY(batch(t0, tb, dv, &tot));
             if (tot > 0) CK_TRY(emit(tb, dv, rk + at));
             at += tot;
         }

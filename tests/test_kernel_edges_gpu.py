@@ -280,3 +280,29 @@ def test_lsh_large_buckets(ck, n):
     idx, _ = band_parameters(4, 12, 1, 3)
     assert {0, 1} <= set(idx[:, 0].tolist())
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [2, 3, 40, 1500])
+def test_lsh_ids_that_share_their_upper_bits(ck, n):
+    """Bucket ids of a table that differ in their lowest bits only, the members
+    of one between those of another; the second table's are random."""
+    rng = np.random.default_rng(n)
+    idx, seeds = band_parameters(2, 8, 1, 4)
+    col = int(idx[0, 0])
+    m64 = (1 << 64) - 1
+
+    def sketch_value(h):  # the value with bucket id h in table 0
+        h ^= h >> 33
+        h = h * pow(0xC4CEB9FE1A85EC53, -1, 1 << 64) & m64
+        h ^= h >> 33
+        return (h - int(seeds[0]) * 0x517CC1B727220A95) & m64
+
+    low = rng.integers(0, max(2, n // 9), n)
+    sk = rng.integers(0, max(2, n // 2), (n, 2)).astype(np.uint64)
+    sk[:, col] = [sketch_value((0x0123456789AB << 16) | int(x)) for x in low]
+    got = lsh_candidates_device(sk, 8, 1, 4).cpu().numpy()
+    want = lsh_candidates(sk, 8, 1, 4)
+    same = low[:, None] == low[None, :]
+    a, b = np.nonzero(np.triu(same | (sk[:, None, 1 - col] == sk[None, :, 1 - col]), 1))
+    assert set(idx[:, 0].tolist()) == {0, 1}
+    assert np.array_equal(want, np.stack([a, b], 1)) and np.array_equal(got, want)
