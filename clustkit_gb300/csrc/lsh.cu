@@ -20,7 +20,7 @@
 // in (table, sequence) order and sorted together, stably, so each bucket is one
 // run with its members in ascending sequence id, and the run, scan, pair-count
 // and emit steps cover the whole batch in one launch each; one radix sort +
-// unique de-duplicates all tables.  The sort moves 12 bytes an item and looks
+// unique de-duplicates all tables, most repeats being left out before it.  The sort moves 12 bytes an item and looks
 // at as many bits of the id as tell a table's buckets apart, and not at the
 // table (6 passes over 12.8 M items, 0.84 ms; sorted by table and all 64 bits
 // as 16-byte keys, it was 9 passes and 1.56).
@@ -37,7 +37,7 @@
 // several, the first one's count times their number (and a quarter) sizes it,
 // and only a call that outgrows that runs its batches a second time, into a
 // buffer of the counted size.  100,000 sequences, 448 tables of one band: the
-// whole call 24.0 -> 6.3 ms (the old form hashed and sorted all 448
+// whole call 24.0 -> 5.5 ms (the old form hashed and sorted all 448
 // tables twice).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -193,6 +193,144 @@ __global__ void lsh_emit_big_kernel(const uint32_t *__restrict__ order, const in
     }
 }
 
+// The same two emissions where several tables find most pairs again and again:
+// a pair goes out only if it is not in its set of `seen`, four keys in one
+// 32-byte sector (all ones at first, at most 64 MB, which stay in L2), and takes
+// a free place there.  A race or a full set lets a pair out twice; none is lost,
+// since whoever puts a key into a set also writes it.  A warp queues its pairs
+// and takes room for many at a time from *n_out.  Bound by the latency of the
+// sets' reads (25 M in 0.35 ms); four rounds ahead help the large buckets (255 ->
+// 175 us) and not the small ones, whose warps have few pairs (175 -> 336).
+// 100,000 sequences, 124 distinct tables: of 25.5 M raw pairs 6.5 M are written
+// (4.6 M are distinct), and sorting them takes 0.32 ms instead of 1.17.
+//
+// Used from 12 distinct tables and 4 M raw pairs on.  Whole call without and
+// with: 22 M pairs of 124 tables 5.83 -> 5.14 ms, 32 M of 199 4.19 -> 3.18,
+// 11 M of 448 7.48 -> 7.18, 5.4 M of 15 1.98 -> 1.87; but 1.6 M of 8 1.40 ->
+// 1.44, 1.8 M of 30 1.16 -> 1.20, 0.4 M of 124 3.76 -> 3.80.
+constexpr int32_t LSH_FILTER_TABLES = 12;
+constexpr int64_t LSH_FILTER_PAIRS = (int64_t)1 << 22;
+constexpr int LSH_AHEAD = 4, LSH_QUEUE = 256, LSH_FILTER_THREADS = 256, LSH_FILTER_PARTS = 32;
+struct LshFilter {
+    uint64_t *seen;  // sets of four keys, 32 bytes
+    uint64_t mask;   // sets - 1
+    uint64_t *out;
+    unsigned long long *n_out;
+    uint64_t *queue;  // the warp's, LSH_QUEUE + 32 LSH_AHEAD
+    int32_t held;
+
+    __device__ void flush(int lane) {
+        __syncwarp();
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(n_out, (unsigned long long)held);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (int i = lane; i < held; i += 32) out[at + i] = queue[i];
+        __syncwarp();
+        held = 0;
+    }
+    // U rounds of keys, all lanes together; ~0 where the lane has none.
+    // The sets of all are read before the first is looked at.
+    template <int U> __device__ void put(const uint64_t (&key)[U], int lane) {
+        uint64_t a[U], b[U], c[U], d[U], *set[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            set[u] = seen + 4 * ((key[u] * 0x9E3779B97F4A7C15ull) >> 32 & mask);
+            asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                         : "=l"(a[u]), "=l"(b[u]), "=l"(c[u]), "=l"(d[u]) : "l"(set[u]));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t k = key[u];
+            const bool in = k != ~0ull && a[u] != k && b[u] != k && c[u] != k && d[u] != k;
+            if (in && d[u] == ~0ull) set[u][a[u] == ~0ull ? 0 : b[u] == ~0ull ? 1 : c[u] == ~0ull ? 2 : 3] = k;
+            const uint32_t m = __ballot_sync(0xffffffffu, in);
+            if (in) queue[held + __popc(m & ((1u << lane) - 1))] = k;
+            held += __popc(m);
+        }
+        if (held >= LSH_QUEUE) flush(lane);
+    }
+};
+
+__global__ void __launch_bounds__(LSH_FILTER_THREADS)
+    lsh_filter_runs_kernel(const uint32_t *__restrict__ order, const int32_t *__restrict__ run_start,
+                           const int32_t *__restrict__ n_runs, int64_t m, uint32_t n, LshFilter f,
+                           int32_t *__restrict__ big, int32_t *__restrict__ n_big) {
+    __shared__ uint64_t queues[LSH_FILTER_THREADS / 32][LSH_QUEUE + 32 * LSH_AHEAD];
+    const int lane = threadIdx.x & 31;
+    f.queue = queues[threadIdx.x >> 5];
+    f.held = 0;
+    const int32_t R = *n_runs;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; r0 < R; r0 += step) {
+        // a lane a bucket, then the warp's pairs laid end to end
+        const int64_t r = r0 + lane;
+        int32_t c = r < R ? lsh_members(run_start, r, R, m) : 0;
+        if (c > LSH_SMALL_BUCKET) {
+            big[atomicAdd(n_big, 1)] = (int32_t)r;
+            c = 0;
+        }
+        const int32_t s0 = c >= 2 ? run_start[r] : 0;
+        const uint32_t base = c >= 2 ? order[s0] / n * n : 0;
+        int32_t end = c * (c - 1) / 2;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t v = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += v;
+        }
+        const int32_t total = __shfl_sync(0xffffffffu, end, 31);
+        for (int32_t i0 = 0; i0 < total; i0 += 32) {
+            const int32_t i = min(i0 + lane, total - 1);
+            int owner = 0;  // lanes whose pairs end at i or before
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+                if (__shfl_sync(0xffffffffu, end, owner + o - 1) <= i) owner += o;
+            const int32_t before = __shfl_sync(0xffffffffu, end, max(owner - 1, 0));
+            const int32_t p = i - (owner ? before : 0);  // pair y(y - 1)/2 + x of its bucket
+            int32_t y = (int32_t)((sqrtf((float)(8 * p + 1)) + 1.0f) * 0.5f);
+            if (y * (y - 1) / 2 > p) --y;
+            if (y * (y + 1) / 2 <= p) ++y;
+            const int32_t from = __shfl_sync(0xffffffffu, s0, owner);
+            const uint32_t b = __shfl_sync(0xffffffffu, base, owner);
+            const uint32_t hi = order[from + y] - b, lo = order[from + p - y * (y - 1) / 2] - b;
+            const uint64_t key[1] = {i0 + lane < total ? (uint64_t)lo * n + hi : ~0ull};
+            f.put(key, lane);
+        }
+    }
+    f.flush(lane);
+}
+
+__global__ void __launch_bounds__(LSH_FILTER_THREADS)
+    lsh_filter_big_kernel(const uint32_t *__restrict__ order, const int32_t *__restrict__ run_start,
+                          const int32_t *__restrict__ n_runs, int64_t m, const int32_t *__restrict__ big,
+                          const int32_t *__restrict__ n_big, uint32_t n, LshFilter f) {
+    __shared__ uint64_t queues[LSH_FILTER_THREADS / 32][LSH_QUEUE + 32 * LSH_AHEAD];
+    const int lane = threadIdx.x & 31;
+    f.queue = queues[threadIdx.x >> 5];
+    f.held = 0;
+    const int32_t nb = *n_big;
+    const int32_t warps = (int32_t)(blockDim.x >> 5) * LSH_FILTER_PARTS;
+    const int32_t warp = (int32_t)(blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5));
+    for (int32_t w = blockIdx.x; w < nb; w += gridDim.x) {
+        const int32_t r = big[w];
+        const int32_t c = lsh_members(run_start, r, *n_runs, m);
+        const int32_t s0 = run_start[r];
+        const uint32_t base = order[s0] / n * n;
+        for (int32_t y = 1 + warp; y < c; y += warps) {
+            const uint32_t b = order[s0 + y] - base;
+            for (int32_t x0 = lane; x0 - lane < y; x0 += 32 * LSH_AHEAD) {
+                uint64_t key[LSH_AHEAD];
+#pragma unroll
+                for (int u = 0; u < LSH_AHEAD; ++u) {
+                    const int32_t x = x0 + 32 * u;
+                    key[u] = x < y ? (uint64_t)(order[s0 + x] - base) * n + b : ~0ull;
+                }
+                f.put(key, lane);
+            }
+        }
+    }
+    f.flush(lane);
+}
+
 __global__ void lsh_unpack_kernel(const uint64_t *__restrict__ keys, int64_t m, int64_t n,
                                   int32_t *__restrict__ pairs) {
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
@@ -320,10 +458,29 @@ static int32_t lsh_impl(void *pv) {
         }
     };
 
-    // emission of the batch just prepared, at raw pair `at` of the buffer
+    uint64_t *rk = nullptr, *seen = nullptr;  // raw pairs; keys seen, where repeats are left out
+    uint64_t places = 0;
+    unsigned long long *d_kept = (unsigned long long *)(n_runs + 10);
+    const auto forget = [&]() -> int32_t {
+        if (!seen) return CK_OK;
+        CK_CUDA(cudaMemsetAsync(seen, 0xff, (size_t)places * 8, st));
+        CK_CUDA(cudaMemsetAsync(d_kept, 0, 8, st));
+        return CK_OK;
+    };
+    // emission of the batch just prepared, at `out` (or behind what is kept)
     auto emit = [&](int32_t tb, cub::DoubleBuffer<uint32_t> &dv, uint64_t *out) -> int32_t {
         const int64_t m = (int64_t)tb * n;
         CK_CUDA(cudaMemsetAsync(n_big, 0, 4, st));
+        if (seen) {
+            const LshFilter f{seen, places / 4 - 1, rk, d_kept, nullptr, 0};
+            lsh_filter_runs_kernel<<<8 * sm_count(), LSH_FILTER_THREADS, 0, st>>>(dv.Current(), starts, n_runs, m,
+                                                                                  (uint32_t)n, f, big, n_big);
+            CK_CUDA(cudaGetLastError());
+            lsh_filter_big_kernel<<<dim3((unsigned)sm_count(), LSH_FILTER_PARTS), LSH_FILTER_THREADS, 0, st>>>(
+                dv.Current(), starts, n_runs, m, big, n_big, (uint32_t)n, f);
+            CK_CUDA(cudaGetLastError());
+            return CK_OK;
+        }
         lsh_emit_runs_kernel<<<grid_of(m, 256), 256, 0, st>>>(dv.Current(), starts, pair_off, n_runs, m, (uint32_t)n,
                                                               out, big, n_big);
         CK_CUDA(cudaGetLastError());
@@ -336,7 +493,6 @@ static int32_t lsh_impl(void *pv) {
     // room for `room` raw pairs, twice over for the de-duplicating sort; a
     // guess that does not fit the device is no error (the counted size may)
     const int32_t n_batches = (T + TB - 1) / TB;
-    uint64_t *rk = nullptr;
     int64_t room = 0, raw = 0;
     bool fits = true;
     for (int32_t b = 0; b < n_batches; ++b) {
@@ -354,6 +510,17 @@ static int32_t lsh_impl(void *pv) {
                 status = CK_OK;
                 room = 0;
             }
+            if (T >= LSH_FILTER_TABLES && room >= LSH_FILTER_PAIRS) {
+                places = (uint64_t)1 << 16;
+                while (places < ((uint64_t)1 << 23) && places < (uint64_t)room / 4) places *= 2;
+                seen = (uint64_t *)scratch(SLOT_SORT_KEYS_ALT, (size_t)places * 8, &status);
+                if (!seen) {  // done without
+                    cudaGetLastError();
+                    reset_thread_status();
+                    status = CK_OK;
+                }
+                CK_TRY(forget());
+            }
         }
         if (tot > 0 && raw + tot <= room && fits) CK_TRY(emit(tb, dv, rk + raw));
         else if (tot > 0) fits = false;
@@ -364,6 +531,7 @@ static int32_t lsh_impl(void *pv) {
         rk = (uint64_t *)scratch(SLOT_FALLBACK, (size_t)raw * 8 * 2, &status);
         if (!rk) return status;
         int64_t at = 0;
+        CK_TRY(forget());
         for (int32_t b = 0; b < n_batches; ++b) {
             const int32_t t0 = b * TB, tb = T - t0 < TB ? T - t0 : TB;
             cub::DoubleBuffer<uint32_t> dv(v0, v1);
@@ -372,6 +540,10 @@ static int32_t lsh_impl(void *pv) {
             if (tot > 0) CK_TRY(emit(tb, dv, rk + at));
             at += tot;
         }
+    }
+    if (seen) {
+        CK_CUDA(cudaMemcpyAsync(&raw, d_kept, 8, cudaMemcpyDeviceToHost, st));
+        CK_CUDA(cudaStreamSynchronize(st));
     }
     // de-duplicate: sort packed keys (enough bits for n * n), unique
     int bits = 1;

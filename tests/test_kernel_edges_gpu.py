@@ -306,3 +306,23 @@ def test_lsh_ids_that_share_their_upper_bits(ck, n):
     a, b = np.nonzero(np.triu(same | (sk[:, None, 1 - col] == sk[None, :, 1 - col]), 1))
     assert set(idx[:, 0].tolist()) == {0, 1}
     assert np.array_equal(want, np.stack([a, b], 1)) and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("members,rest,tables", [(1000, 0, 20), (900, 2000, 20), (760, 1, 40)])
+def test_lsh_repeated_pairs(ck, members, rest, tables):
+    """Pairs that every table finds, by the million, beside buckets of each
+    small size that differ from table to table."""
+    rng = np.random.default_rng(members)
+    size = 64
+    sk = rng.integers(0, 2 ** 62, (members + rest, size)).astype(np.uint64)
+    sk[rng.permutation(members + rest)[:members]] = 5
+    idx, _ = band_parameters(size, tables, 1, 8)
+    columns = len(np.unique(idx))
+    assert columns >= 12 and members * (members - 1) // 2 * columns >= 1 << 22
+    for c in range(size if rest > 1 else 0):
+        own = np.flatnonzero(sk[:, c] != 5)
+        cut = np.sort(rng.choice(len(own), 120, replace=False))
+        for x, y in zip(cut[:-1], cut[1:]):
+            sk[own[x:y], c] = 1000 + x
+    got = lsh_candidates_device(sk, tables, 1, 8).cpu().numpy()
+    assert np.array_equal(got, lsh_candidates(sk, tables, 1, 8))
