@@ -34,36 +34,90 @@ __global__ void kmer_pos_count_kernel(const int32_t *lengths, int64_t n, int32_t
     }
 }
 
+// Occurrences in (sequence, position) order, a warp a sequence; the k-mers'
+// frequencies as well where `freqs`.  K > 0: k, at compile time.  39 M: 145 us
+// (470 MB written; 275 with the atomics and k a variable).
+template <int K>
 __global__ void kmer_emit_kernel(const uint8_t *__restrict__ flat, int64_t flat_len,
                                  const int64_t *__restrict__ offsets,
-                                 const int32_t *__restrict__ lengths, int64_t n, int32_t k,
+                                 const int32_t *__restrict__ lengths, int64_t n, int32_t any_k,
                                  int32_t alpha, const int64_t *__restrict__ pos_base,
                                  uint32_t *__restrict__ keys, int64_t *__restrict__ vals,
                                  int32_t *__restrict__ freqs, uint32_t sentinel, int32_t *err) {
+    const int32_t k = K ? K : any_k;
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += warps) {
         const int32_t L = lengths[q];
         const int64_t o = offsets[q];
         if (L < k) continue;
-        if (o < 0 || o + L > flat_len) {
-            if (lane == 0) atomicOr(err, ERRBIT_SEQ_EXTENT);
-            continue;
-        }
         const int64_t base = pos_base[q];
+        const bool bad = o < 0 || o + L > flat_len;
+        if (bad && lane == 0) atomicOr(err, ERRBIT_SEQ_EXTENT);
+        const uint8_t *s = bad ? flat : flat + o;
+#pragma unroll 2
         for (int32_t p = lane; p <= L - k; p += 32) {
             uint32_t v = 0;
-            bool ok = true;
-            for (int32_t m = 0; m < k; ++m) {
-                const uint32_t c = flat[o + p + m];
-                ok &= c < (uint32_t)alpha;
-                v = v * (uint32_t)alpha + c;
-            }
+            bool ok = !bad;
+            if (!bad)
+#pragma unroll
+                for (int32_t m = 0; m < k; ++m) {
+                    const uint32_t c = __ldg(s + p + m);
+                    ok &= c < (uint32_t)alpha;
+                    v = v * (uint32_t)alpha + c;
+                }
             keys[base + p] = ok ? v : sentinel;
             vals[base + p] = ((int64_t)q << 32) | (int64_t)p;
-            if (ok) atomicAdd(&freqs[v], 1);
+            if (freqs && ok) atomicAdd(&freqs[v], 1);
         }
     }
+}
+
+// offsets[u] = the first of the P sorted keys at or above u, u <= nk (the
+// sentinel nk sorts last): a key sets those from the key before it (exclusive)
+// to its own.  A lane takes four keys (64 us for 39 M; one key a lane 101) and a
+// long gap is written by the whole warp.  The last lane of all, behind the
+// keys, ends the offsets.
+__global__ void kmer_bounds_kernel(const uint32_t *__restrict__ keys, uint32_t P, uint32_t nk,
+                                   int64_t *__restrict__ offsets) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t groups = (P >> 2) + 1, step = gridDim.x * blockDim.x;
+    for (uint32_t g0 = blockIdx.x * blockDim.x + threadIdx.x - lane; g0 < groups; g0 += step) {
+        const uint32_t i = 4 * (g0 + lane);
+        uint32_t key[4];
+        if (i + 4 <= P) {
+            const uint4 x = *(const uint4 *)(keys + i);
+            key[0] = x.x, key[1] = x.y, key[2] = x.z, key[3] = x.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) key[j] = i + j < P ? keys[i + j] : nk;
+        }
+        uint32_t before = __shfl_up_sync(0xffffffffu, key[3], 1);
+        if (lane == 0 && i > 0) before = keys[i - 1];
+        uint32_t from = i > 0 ? before + 1 : 0;
+        uint32_t left = key[3] + 1 > from && i <= P ? key[3] + 1 - from : 0;  // offsets the lane's keys set
+        if (left > 0 && left < 64) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                for (; from <= key[j] && from <= nk; ++from) offsets[from] = i + j < P ? i + j : P;
+            left = 0;
+        }
+        for (uint32_t wide = __ballot_sync(0xffffffffu, left > 0); wide; wide &= wide - 1) {
+            const int x = __ffs(wide) - 1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t f = __shfl_sync(0xffffffffu, from, x), t = min(__shfl_sync(0xffffffffu, key[j], x), nk);
+                const uint32_t at = min(4 * (g0 + x) + j, P);
+                for (uint32_t u = f + lane; u <= t; u += 32) offsets[u] = at;
+                if (lane == x && f <= t) from = t + 1;
+            }
+        }
+    }
+}
+
+__global__ void kmer_freqs_kernel(const int64_t *__restrict__ offsets, int64_t nk, int32_t *__restrict__ freqs) {
+    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nk; u += (int64_t)gridDim.x * blockDim.x)
+        freqs[u] = (int32_t)(offsets[u + 1] - offsets[u]);
 }
 
 __global__ void widen_kernel(const int32_t *in, int64_t n, int64_t *out) {
@@ -114,17 +168,27 @@ static int32_t index_build_impl(void *pv) {
         set_error(CK_ERR_INVALID_ARGUMENT, "kmer index: entries capacity below the number of k-mer positions");
         return CK_ERR_INVALID_ARGUMENT;
     }
-    CK_CUDA(cudaMemsetAsync(a.kmer_freqs, 0, (size_t)nk * 4, a.st));
+    // Offsets and frequencies: read off the sorted keys, or counted by atomics as
+    // the occurrences are made and scanned.  39 M occurrences of 3.2 M 5-mers:
+    // 72 us for reading them off; the atomics, the scan and the widening took 143.
+    // Few k-mers meet in the atomics (20 M occurrences of 8,000 3-mers: whole
+    // build 1.33 -> 0.82 ms).  An index with an eighth as many occurrences as
+    // k-mers costs the same either way (0.19 ms), a sparser one is mostly gaps.
+    const bool dense = P > 0 && nk <= 8 * P;
+    if (!dense) CK_CUDA(cudaMemsetAsync(a.kmer_freqs, 0, (size_t)nk * 4, a.st));
     const size_t P1 = (size_t)(P > 0 ? P : 1);
     uint32_t *k0 = (uint32_t *)scratch(SLOT_SEARCH_TMP1, P1 * 4, &status);
     uint32_t *k1 = (uint32_t *)scratch(SLOT_SEARCH_TMP2, P1 * 4, &status);
     int64_t *v0 = (int64_t *)scratch(SLOT_SEARCH_TMP3, P1 * 8, &status);
     if (!k0 || !k1 || !v0) return status;
     const uint32_t sentinel = (uint32_t)nk;
+    const auto emit = a.k == 5   ? kmer_emit_kernel<5>
+                      : a.k == 4 ? kmer_emit_kernel<4>
+                      : a.k == 3 ? kmer_emit_kernel<3>
+                                 : kmer_emit_kernel<0>;
     if (a.n > 0)
-        kmer_emit_kernel<<<grid_for(a.n * 32, 256), 256, 0, a.st>>>(
-            a.flat, a.flat_len, a.offsets, a.lengths, a.n, a.k, a.alpha, cnt, k0, v0, a.kmer_freqs,
-            sentinel, err);
+        emit<<<grid_for(a.n * 32, 256), 256, 0, a.st>>>(a.flat, a.flat_len, a.offsets, a.lengths, a.n, a.k, a.alpha,
+                                                        cnt, k0, v0, dense ? nullptr : a.kmer_freqs, sentinel, err);
     CK_CUDA(cudaGetLastError());
     int bits = 1;
     while (((int64_t)1 << bits) <= (int64_t)sentinel) ++bits;
@@ -139,14 +203,23 @@ static int32_t index_build_impl(void *pv) {
         CK_CUDA(cub::DeviceRadixSort::SortPairs(stmp, sb, dk, dv, (int)P, 0, bits, a.st));
         if (dv.Current() != a.kmer_entries)
             CK_CUDA(cudaMemcpyAsync(a.kmer_entries, dv.Current(), (size_t)P * 8, cudaMemcpyDeviceToDevice, a.st));
+        if (dense) {
+            kmer_bounds_kernel<<<grid_for(P / 4 + 1, 256, 32), 256, 0, a.st>>>(dk.Current(), (uint32_t)P, (uint32_t)nk,
+                                                                                a.kmer_offsets);
+            CK_CUDA(cudaGetLastError());
+            kmer_freqs_kernel<<<grid_for(nk, 256), 256, 0, a.st>>>(a.kmer_offsets, nk, a.kmer_freqs);
+            CK_CUDA(cudaGetLastError());
+        }
     }
-    widen_kernel<<<grid_for(nk + 1, 256), 256, 0, a.st>>>(a.kmer_freqs, nk, a.kmer_offsets);
-    CK_CUDA(cudaGetLastError());
-    size_t tb2 = 0;
-    CK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, a.kmer_offsets, a.kmer_offsets, nk + 1, a.st));
-    void *tmp2 = scratch(SLOT_SEARCH_TMP4, tb2, &status);
-    if (!tmp2) return status;
-    CK_CUDA(cub::DeviceScan::ExclusiveSum(tmp2, tb2, a.kmer_offsets, a.kmer_offsets, nk + 1, a.st));
+    if (!dense) {
+        widen_kernel<<<grid_for(nk + 1, 256), 256, 0, a.st>>>(a.kmer_freqs, nk, a.kmer_offsets);
+        CK_CUDA(cudaGetLastError());
+        size_t tb2 = 0;
+        CK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, a.kmer_offsets, a.kmer_offsets, nk + 1, a.st));
+        void *tmp2 = scratch(SLOT_SEARCH_TMP4, tb2, &status);
+        if (!tmp2) return status;
+        CK_CUDA(cub::DeviceScan::ExclusiveSum(tmp2, tb2, a.kmer_offsets, a.kmer_offsets, nk + 1, a.st));
+    }
     int64_t total = 0;
     CK_CUDA(cudaMemcpyAsync(&total, a.kmer_offsets + nk, 8, cudaMemcpyDeviceToHost, a.st));
     int32_t h = 0;

@@ -326,3 +326,40 @@ def test_lsh_repeated_pairs(ck, members, rest, tables):
             sk[own[x:y], c] = 1000 + x
     got = lsh_candidates_device(sk, tables, 1, 8).cpu().numpy()
     assert np.array_equal(got, lsh_candidates(sk, tables, 1, 8))
+
+
+@pytest.mark.parametrize("n,lo,hi,k,alpha,letters", [
+    (1, 5, 5, 5, 20, 20), (1, 8, 8, 5, 20, 20), (3, 0, 9, 3, 20, 25), (40, 1, 300, 2, 6, 6), (7, 60, 61, 3, 20, 1),
+    (300, 0, 90, 4, 20, 21), (900, 30, 700, 5, 20, 22), (2500, 30, 700, 5, 20, 3), (64, 4, 130, 1, 20, 30),
+    (50, 10, 400, 7, 4, 4), (2, 3, 4, 5, 20, 20), (5, 20, 30, 2, 20, 255)])
+def test_kmer_index(ck, n, lo, hi, k, alpha, letters):
+    """Offsets and frequencies counted and read off the sorted k-mers: few and
+    many occurrences, long runs without a k-mer, residues that belong to none."""
+    torch = pytest.importorskip("torch")
+    from clustkit_gb300 import _lib
+    rng = np.random.default_rng(n + k)
+    flat, off, length = _pack([rng.integers(0, letters, rng.integers(lo, hi + 1)).astype(np.uint8) for _ in range(n)])
+    keys, entries = [], []
+    for q in range(n):
+        s = flat[off[q]:off[q] + length[q]].astype(np.int64)
+        for p in range(len(s) - k + 1):
+            w = s[p:p + k]
+            keys.append(int(w @ alpha ** np.arange(k)[::-1]) if (w < alpha).all() else alpha ** k)
+            entries.append(q << 32 | p)
+    keys, entries, nk = np.array(keys, np.int64), np.array(entries, np.int64), alpha ** k
+    want_freqs = np.bincount(keys, minlength=nk + 1)[:nk]
+    want_offsets = np.concatenate([[0], np.cumsum(want_freqs)])
+    want_entries = entries[np.argsort(keys, kind="stable")]
+    flat = np.concatenate([flat, np.zeros(1, np.uint8)])
+    d = [torch.from_numpy(x).cuda() for x in (flat, off, length)]
+    offsets = torch.full((nk + 1,), -1, dtype=torch.int64, device="cuda")
+    freqs = torch.full((nk,), -1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(max(len(keys), 1), dtype=torch.int64, device="cuda")
+    total = np.zeros(1, np.int64)
+    _lib.check(_lib.load().ck_kmer_index_build_device(
+        0, d[0].data_ptr(), d[0].numel(), d[1].data_ptr(), d[2].data_ptr(), n, k, alpha, offsets.data_ptr(),
+        out.data_ptr(), len(keys), freqs.data_ptr(), total.ctypes.data, torch.cuda.current_stream().cuda_stream))
+    assert total[0] == want_offsets[-1]
+    assert np.array_equal(offsets.cpu().numpy(), want_offsets)
+    assert np.array_equal(freqs.cpu().numpy(), want_freqs)
+    assert np.array_equal(out.cpu().numpy()[:len(keys)], want_entries)
