@@ -1074,6 +1074,9 @@ nbr_walk_kernel(const int32_t *__restrict__ n, const int32_t *__restrict__ run0,
 // order_kernel checks that (and that targets lie in the database), and a call
 // whose lists are not goes to the walk above.  Cutting and checking cost about
 // what a few queries save, so fewer than NB_RANGE_MIN_QUERIES keep that one.
+// Whole search of 1, 3, 4, 6 and 16 queries, walk above and ranges: 20,000
+// sequences 0.47 0.91 1.02 1.26 2.20 and 0.53 0.91 1.01 1.20 1.99 ms; 200,000
+// sequences 1.05 1.49 1.72 2.25 3.87 and 1.20 1.57 1.74 2.11 3.38.
 // 64 queries, 200,000 sequences: 5.3 ms, with 0.2 for the cuts and the check;
 // the walk on the count rows took 11.4 (listed triples, repeats and all).
 constexpr int32_t NB_RANGE = 56 * 1024;   // counters of a block: 224 KB of shared memory
