@@ -30,7 +30,7 @@ struct ScratchSet {
     size_t cap[SLOT_COUNT] = {};
     int32_t *err = nullptr;
     bool frozen = false;  // buffers may be baked into a captured CUDA graph: never reallocate
-    bool dirty[SLOT_COUNT] = {};  // a kept-zero buffer whose last user may not have cleaned it
+    bool dirty[SLOT_COUNT] = {};  // not known to be all zero: newly allocated, or its last user may not have cleaned it
     // resident sequence database of the submit/poll interface (ck_ctx_upload_db)
     uint8_t *db_flat = nullptr;
     int64_t *db_offsets = nullptr;
@@ -196,6 +196,7 @@ void *scratch(int slot, size_t bytes, int32_t *status) {
             return nullptr;
         }
         s->cap[slot] = want;
+        s->dirty[slot] = true;  // also at its old address, which may hold anything by now
     }
     return s->buf[slot];
 }
@@ -206,10 +207,9 @@ void *scratch(int slot, size_t bytes, int32_t *status) {
 void *scratch_zeroed(int slot, size_t bytes, cudaStream_t st, int32_t *status) {
     ScratchSet *s = current_set(status);
     if (!s) return nullptr;
-    const void *before = s->buf[slot];
     void *p = scratch(slot, bytes, status);
     if (!p) return nullptr;
-    if (p != before || s->dirty[slot]) {
+    if (s->dirty[slot]) {
         const cudaError_t e = cudaMemsetAsync(p, 0, s->cap[slot], st);
         if (e != cudaSuccess) { *status = cuda_status(e, "cudaMemsetAsync(zeroed scratch)"); return nullptr; }
         s->dirty[slot] = false;
