@@ -5,7 +5,7 @@
 // where v_i = sum_m code[i+m] * alphabet^(k-1-m) in wrapping uint64 (the
 // value clustkit's rolling update produces), padded with UINT64_MAX.
 //
-// One warp per sequence.  sketch_select_kernel (s up to about 1,900) hashes
+// One warp per sequence.  sketch_select_kernel (s up to 1,768) hashes
 // the k-mers against a threshold that a uniform hash would leave between s and
 // C of (C a power of two a few standard deviations above s), keeps those at or
 // below it in shared memory, and sorts them in registers; it is bound by
@@ -104,19 +104,31 @@ __device__ __forceinline__ uint64_t kmer_value(const uint8_t *p, int32_t k, V al
     return (uint64_t)v;
 }
 
-// Sketches by threshold: with nk > C hashes the first threshold leaves about
-// `aim` of them (s < aim < C) if they are spread evenly; a count outside
-// [s, C] moves it (first by half, then by bisection between the largest
-// threshold known to leave too few and the smallest known to leave too many).
-// When those two are neighbours, the upper one is a value with many copies:
-// everything below it is kept and copies of it fill the sketch.  The kept
-// hashes are sorted by their leading bits (as many as fit beside the slot
+// Sketches by threshold: with nk > C hashes a threshold that leaves about `aim`
+// of them (s < aim < C) if they are spread evenly.  A count outside [s, C] -- one
+// random sequence in a thousand, and many repeats, whose k-mers come in many
+// copies -- takes a second pass that needs no threshold: it sorts whenever the
+// buffer is full and goes on below the s-th smallest so far.  (Moving the
+// threshold until the count fits took up to 66 passes where one value has more
+// than C - s copies.  Going on from a full buffer in the first pass costs its
+// loop a test, 5 % of the whole.)
+// The hashes are sorted by their leading bits (as many as fit beside the slot
 // number in 32 bits: a compare-exchange is then one instruction a key, not
 // the five or six that 64-bit keys take), and the few neighbours whose leading
 // bits agree are put right in shared memory.
-// 200,000 sequences (median 300 residues), k = 5, s = 128: 3.62 -> 0.46 ms (sketch_kernel, sorting 64-bit keys in shared memory, before).
+// 200,000 sequences (median 300 residues), k = 5, s = 128: 3.62 -> 0.46 ms
+// (sketch_kernel, sorting 64-bit keys in shared memory, before).  5,000 of 2,000
+// residues: random ones 54 us, repeats of 4 with 2 % changed 106 (sketch_kernel
+// 279 and 227; by moving the threshold 54 and 2,117).
+// warps of a block: 8 while their buffers fit 48 KB, else as many as do (C <= 2048: 16 KB a warp)
+template <int NPL>
+constexpr int select_warps() { return NPL <= 16 ? 8 : 48 * 1024 / (32 * NPL * 8); }
+// resident blocks: registers for as many as the buffers leave room for (NPL >= 32), or without spills
+template <int NPL>
+constexpr int select_blocks() { return NPL >= 16 ? 4 : NPL == 8 ? 5 : 6; }
+
 template <int NPL, class V>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * select_warps<NPL>(), select_blocks<NPL>())
 sketch_select_kernel(const uint8_t *__restrict__ flat, int64_t flat_len, const int64_t *__restrict__ offsets,
                      const int32_t *__restrict__ lengths, int64_t N, int32_t k, int32_t s, int32_t aim, V alphabet,
                      uint64_t seed, uint64_t *__restrict__ out, int32_t *err) {
@@ -141,83 +153,80 @@ sketch_select_kernel(const uint8_t *__restrict__ flat, int64_t flat_len, const i
         }
         const uint8_t *seq = flat + off;
         const int32_t nk = L - k + 1;
-        // hashes at or below `tau` into buf (the first C of them); their number
-        auto gather = [&](uint64_t tau) {
-            int32_t cnt = 0;
-            __syncwarp();  // a gather before this one has been written
-            for (int32_t base = 0; base < nk; base += 32) {
-                const int32_t i = base + lane;
+        auto hash = [&](int32_t i) { return fmix64(kmer_value<V>(seq + i, k, alphabet), seed); };
+        // hashes below cap into buf (the first C of them); their number.  (One
+        // equal to MAXV may be left out: the padding stands for it.)
+        uint64_t cap = nk <= C ? MAXV : MAXV / (uint64_t)nk * (uint64_t)aim;
+        int32_t cnt = 0;
+        for (int32_t base = 0; base < nk; base += 32) {
+            const int32_t i = base + lane;
+            uint64_t hv = 0;
+            bool take = false;
+            if (i < nk) {
+                hv = hash(i);
+                take = hv < cap;
+            }
+            const uint32_t bal = __ballot_sync(FULL, take);
+            const int32_t at = cnt + __popc(bal & ((1u << lane) - 1u));
+            if (take && at < C) buf[at] = hv;
+            cnt += __popc(bal);
+        }
+        int32_t next = nk;  // the second pass's next k-mer
+        if (cnt > C || (cnt < s && nk > C)) {
+            if (cnt < s) cap = MAXV;
+            cnt = next = 0;
+        }
+        for (;;) {
+            __syncwarp();
+            while (next < nk && cnt + 32 <= C) {
+                const int32_t i = next + lane;
                 uint64_t hv = 0;
                 bool take = false;
                 if (i < nk) {
-                    hv = fmix64(kmer_value<V>(seq + i, k, alphabet), seed);
-                    take = hv <= tau;
+                    hv = hash(i);
+                    take = hv < cap;
                 }
                 const uint32_t bal = __ballot_sync(FULL, take);
-                const int32_t at = cnt + __popc(bal & ((1u << lane) - 1u));
-                if (take && at < C) buf[at] = hv;
+                if (take) buf[cnt + __popc(bal & ((1u << lane) - 1u))] = hv;
                 cnt += __popc(bal);
+                next += 32;
             }
-            return cnt;
-        };
-        uint64_t tau = MAXV;
-        int32_t cnt;
-        if (nk <= C) {
-            cnt = gather(MAXV);
-        } else {
-            uint64_t lo = 0, hi = MAXV;  // lo leaves too few (or is 0), hi leaves s or more
-            tau = MAXV / (uint64_t)nk * (uint64_t)aim;
-            for (int tries = 0;; ++tries) {
-                cnt = gather(tau);
-                if (cnt >= s && cnt <= C) break;
-                if (cnt < s) lo = tau; else hi = tau;
-                if (hi - lo <= 1) {
-                    // lo leaves fewer than s unless it is 0, untested: then hi may be 1 with zeros below it
-                    if (tau != lo) cnt = gather(lo);
-                    if (cnt >= s) { cnt = s; hi = 0; }  // s or more copies of 0
+            for (int t = cnt + lane; t < C; t += 32) buf[t] = MAXV;
+            __syncwarp();
+            // sort keys: leading bits of the hash (none is above cap), then the slot
+            const int width = 64 - __clzll((long long)cap);
+            const int shift = width > 32 - IDX_BITS ? width - (32 - IDX_BITS) : 0;
+            uint32_t v[NPL];
+#pragma unroll
+            for (int r = 0; r < NPL; ++r) {
+                const int t = r * 32 + lane;  // any order will do here: neighbouring lanes read neighbouring slots
+                v[r] = t < cnt ? ((uint32_t)(buf[t] >> shift) << IDX_BITS) | (uint32_t)t : 0xffffffffu;
+            }
+            warp_sort_keys<NPL>(v, lane);
+            // slots -> values in place (read, then written).  A pad key names slot
+            // C - 1, which holds MAXV whenever there is a pad
+            uint64_t val[NPL];
+#pragma unroll
+            for (int r = 0; r < NPL; ++r) val[r] = buf[v[r] & (C - 1)];
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < NPL; ++r) buf[lane * NPL + r] = val[r];
+            __syncwarp();
+            // neighbours with equal leading bits: exchanged until none is out of order
+            for (;;) {
+                bool moved = false;
+                for (int par = 0; par < 2; ++par) {
+                    for (int t = 2 * lane + par; t + 1 < cnt; t += 64) {
+                        const uint64_t a = buf[t], b = buf[t + 1];
+                        if (a > b) { buf[t] = b; buf[t + 1] = a; moved = true; }
+                    }
                     __syncwarp();
-                    for (int t = cnt + lane; t < s; t += 32) buf[t] = hi;
-                    cnt = s;
-                    tau = hi;
-                    break;
                 }
-                const uint64_t step = cnt < s ? tau + tau / 2 : tau - tau / 3;
-                tau = tries < 3 && step > lo && step < hi ? step : lo + (hi - lo) / 2;
+                if (!__any_sync(FULL, moved)) break;
             }
-        }
-        __syncwarp();
-        for (int t = cnt + lane; t < C; t += 32) buf[t] = MAXV;
-        __syncwarp();
-        // sort keys: leading bits of the hash (none is above tau), then the slot
-        const int width = 64 - __clzll((long long)tau);
-        const int shift = width > 32 - IDX_BITS ? width - (32 - IDX_BITS) : 0;
-        uint32_t v[NPL];
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) {
-            const int t = r * 32 + lane;  // any order will do here: neighbouring lanes read neighbouring slots
-            v[r] = t < cnt ? ((uint32_t)(buf[t] >> shift) << IDX_BITS) | (uint32_t)t : 0xffffffffu;
-        }
-        warp_sort_keys<NPL>(v, lane);
-        // slots -> values in place (read, then written).  A pad key names slot
-        // C - 1, which holds MAXV whenever there is a pad
-        uint64_t val[NPL];
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) val[r] = buf[v[r] & (C - 1)];
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < NPL; ++r) buf[lane * NPL + r] = val[r];
-        __syncwarp();
-        // neighbours with equal leading bits: exchanged until none is out of order
-        for (;;) {
-            bool moved = false;
-            for (int par = 0; par < 2; ++par) {
-                for (int t = 2 * lane + par; t + 1 < cnt; t += 64) {
-                    const uint64_t a = buf[t], b = buf[t + 1];
-                    if (a > b) { buf[t] = b; buf[t + 1] = a; moved = true; }
-                }
-                __syncwarp();
-            }
-            if (!__any_sync(FULL, moved)) break;
+            if (next >= nk) break;
+            cnt = s;  // of a full buffer (s + 32 <= C): only what is below the largest of these matters now
+            cap = buf[s - 1];
         }
         for (int t = lane; t < s; t += 32) o[t] = t < cnt ? buf[t] : MAXV;
         __syncwarp();
@@ -308,9 +317,8 @@ struct SketchCall {
 
 template <int NPL, class V>
 static int32_t launch_select_v(const SketchCall &c) {
-    // 8 warps a block while their buffers fit 48 KB, else as many as do (C <= 2048: 16 KB a warp)
     constexpr size_t per_warp = (size_t)32 * NPL * sizeof(uint64_t);
-    constexpr int warps = per_warp * 8 <= 48 * 1024 ? 8 : (int)(48 * 1024 / per_warp);
+    constexpr int warps = select_warps<NPL>();
     const int64_t want = (c.N + warps - 1) / warps, most = (int64_t)sm_count() * 64;
     sketch_select_kernel<NPL, V><<<(unsigned)(want < most ? want : most), warps * 32, per_warp * warps, c.st>>>(
         c.flat, c.flat_len, c.offsets, c.lengths, c.N, c.k, c.s, c.aim, (V)c.alphabet, c.seed, c.out, c.err);
@@ -337,7 +345,7 @@ int32_t sketch_launch(const uint8_t *flat, int64_t flat_len, const int64_t *offs
     if (N == 0) return CK_OK;
     // the threshold form's buffer: C with aim = (s + C) / 2 at least 3.2
     // standard deviations (of about sqrt(aim)) from s and from C, so that about
-    // one sequence in a thousand needs a second threshold
+    // one sequence in a thousand needs a second pass
     for (int32_t C = 64; C <= 2048; C <<= 1) {
         const double mid = 0.5 * ((double)s + C), near = s + 5.5 * sqrt((double)s) + 15.0;
         if (C <= s || 0.5 * (C - s) < 3.2 * sqrt(mid)) continue;

@@ -1,0 +1,71 @@
+"""Kernels where a rule of their dispatch changes sides, and inputs that a rule
+tuned on ordinary ones could lose on, against the oracle (bit for bit)."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _pack(seqs):
+    lengths = np.array([len(x) for x in seqs], np.int32)
+    offsets = (np.cumsum(lengths) - lengths).astype(np.int64)
+    return np.concatenate(seqs).astype(np.uint8), offsets, lengths
+
+
+def _repeat(rng, n, period, changed):
+    x = np.tile(rng.integers(0, 20, period), n // period + 1)[:n]
+    m = rng.random(n) < changed
+    x[m] = rng.integers(0, 20, int(m.sum()))
+    return x
+
+
+@pytest.mark.parametrize("s", [22, 23, 65, 66, 128, 163, 164, 377, 378, 829, 830, 1768, 1769])
+@pytest.mark.parametrize("k", [5, 3, 8])
+def test_sketch_buffer_edges(ck, s, k):
+    """The largest sketch of each buffer size and the next: ordinary sequences
+    of many lengths, and repeats of which no threshold leaves s to C hashes."""
+    from clustkit_gb300.sketch import sketch_flat
+    rng = np.random.default_rng(s * 10 + k)
+    seqs = [rng.integers(0, 20, n) for n in list(rng.integers(s // 2 + 8, 6 * s + 100, 200)) + [9000]]
+    for period in (1, 2, 4, 9, 30):
+        for changed in (0.0, 0.02, 0.1, 0.4):
+            for n in (s + 70, 2000, 7000):
+                seqs.append(_repeat(rng, n, period, changed))
+    for n in (3000, 6000):  # a repeat before and behind ordinary residues
+        seqs.append(np.concatenate([_repeat(rng, n, 4, 0.02), rng.integers(0, 20, n)]))
+        seqs.append(np.concatenate([rng.integers(0, 20, n), _repeat(rng, n, 4, 0.02)]))
+    flat, off, lens = _pack(seqs)
+    assert np.array_equal(sketch_flat(flat, off, lens, k, s), oracle.sketches(flat, off, lens, k, s, 20))
+
+
+def test_sketch_time_of_repeats(ck):
+    """A sequence takes at most two passes over its k-mers, and the second sorts
+    the buffer a few times: repeats stay within 8 times the time of as many
+    random residues (a threshold search by bisection took up to 66 passes)."""
+    import torch
+    from clustkit_gb300 import _lib
+    lib, rng, n, length = _lib.load(), np.random.default_rng(2), 4000, 2000
+    stream = torch.cuda.current_stream().cuda_stream
+    off = torch.arange(n, device="cuda") * length
+    lens = torch.full((n,), length, dtype=torch.int32, device="cuda")
+    out = torch.empty((n, 128), dtype=torch.int64, device="cuda")
+
+    def ms(period, changed):
+        flat = torch.from_numpy(np.concatenate([_repeat(rng, length, period, changed) for _ in range(n)])
+                                .astype(np.uint8)).cuda()
+        best = np.inf
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            _lib.check(lib.ck_sketch_device(flat.data_ptr(), flat.numel(), off.data_ptr(), lens.data_ptr(), n, 5, 128,
+                                            20, 42, out.data_ptr(), stream))
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    random = ms(1, 1.0)
+    for period, changed in ((4, 0.02), (4, 0.1), (9, 0.02), (9, 0.0), (30, 0.05)):
+        assert ms(period, changed) < 8 * random, (period, changed)
