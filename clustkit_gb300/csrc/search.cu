@@ -1083,16 +1083,22 @@ constexpr int32_t NB_RANGE = 56 * 1024;   // counters of a block: 224 KB of shar
 constexpr int32_t NB_MAX_RANGES = 16;     // 917,504 targets; 25.6 MB of cuts each
 constexpr int NB_RW_THREADS = 1024;
 constexpr int32_t NB_RANGE_MIN_QUERIES = 4;
+// postings the walk can number: an octet's end and the step past it stay below 2^32
+constexpr int64_t NB_MAX_POSTINGS = 0xffffff00;
 
 // Whether every list is in target order: the places where a target is below
 // the one before it, over the whole index, less those where a list starts
 // (order[0] - order[1], 0 when all are in order); order[2] counts targets
-// outside the database.
+// outside the database, and is not zero for an index too long to walk.
 __global__ void order_kernel(const int64_t *__restrict__ kmer_offsets, const int64_t *__restrict__ kmer_entries,
                              const int32_t *__restrict__ kmer_targets, int32_t n_kmers, int32_t num_db,
                              unsigned long long *__restrict__ order) {
     const int64_t total = kmer_offsets[n_kmers], step = (int64_t)gridDim.x * blockDim.x;
     const int64_t me = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (total > NB_MAX_POSTINGS) {  // left to the walk on the count rows
+        if (me == 0) order[2] = 1;
+        return;
+    }
     uint32_t falls = 0, starts = 0, outside = 0;
     for (int64_t h = me * 4; h < total; h += step * 4) {
         int32_t before = h > 0 ? entry_target(kmer_entries, kmer_targets, h - 1) : -1;
@@ -1109,7 +1115,7 @@ __global__ void order_kernel(const int64_t *__restrict__ kmer_offsets, const int
         const int64_t b = kmer_offsets[v], e = kmer_offsets[v + 1];
         if (b > 0 && b < e)
             starts += entry_target(kmer_entries, kmer_targets, b) < entry_target(kmer_entries, kmer_targets, b - 1);
-        outside += b < 0 || b > e || e > total || e > (int64_t)0xffffffff;
+        outside += b < 0 || b > e || e > total;
     }
     falls = __reduce_add_sync(0xffffffffu, falls);
     starts = __reduce_add_sync(0xffffffffu, starts);

@@ -69,3 +69,39 @@ def test_sketch_time_of_repeats(ck):
     random = ms(1, 1.0)
     for period, changed in ((4, 0.02), (4, 0.1), (9, 0.02), (9, 0.0), (30, 0.05)):
         assert ms(period, changed) < 8 * random, (period, changed)
+
+
+def test_similar_index_of_almost_2_to_32_postings(ck):
+    """The walk by target ranges numbers postings in 32 bits, eight at a time;
+    an index that ends a few short of 2^32 is left to the other walk."""
+    import torch
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.blosum import BLOSUM62
+    lib, total, nk, nq, top_k = _lib.load(), 2 ** 32 - 4, 20 ** 5, 4, 5
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 24 GB of device memory")
+    sub = np.ascontiguousarray(BLOSUM62, np.int8)
+    targets = torch.zeros(total, dtype=torch.int32, device="cuda")
+    targets[-6:] = torch.tensor([0, 0, 1, 2, 2, 2], dtype=torch.int32)
+    offsets = torch.full((nk + 1,), total - 6, dtype=torch.int64, device="cuda")
+    offsets[0], offsets[-1] = 0, total  # all but six are the first 5-mer's, the six the last one's
+    freqs = torch.zeros(nk, dtype=torch.int32, device="cuda")
+    freqs[0], freqs[-1] = 2 ** 31 - 1, 6
+    queries = [[19] * 5, [0] * 9, [19] * 6, [0] * 5]
+    lens = np.array([len(q) for q in queries], np.int32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_q, d_len = dev(np.concatenate(queries).astype(np.uint8)), dev(lens)
+    d_off = dev((np.cumsum(lens) - lens).astype(np.int64))
+    out_t = torch.zeros(nq * top_k, dtype=torch.int32, device="cuda")
+    out_s, out_n = torch.zeros_like(out_t), torch.zeros(nq, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.ck_search_phase_a_similar_device(
+        0, d_q.data_ptr(), int(lens.sum()), d_off.data_ptr(), d_len.data_ptr(), nq, int(lens.max()), sub.ctypes.data,
+        13, offsets.data_ptr(), None, targets.data_ptr(), freqs.data_ptr(), 1000, 3, 2, top_k, out_t.data_ptr(),
+        out_s.data_ptr(), out_n.data_ptr(), -1, st))
+    _lib.check(lib.ck_ctx_status(0, st))
+    w = 5 * int(sub[19, 19])
+    assert w >= 13 and 5 * int(sub[0, 19]) < 13
+    got = [list(zip(t[:n], s[:n])) for t, s, n in zip(out_t.view(nq, -1).tolist(), out_s.view(nq, -1).tolist(),
+                                                      out_n.tolist())]
+    assert got == [[(0, 2 * w), (1, w), (2, 3 * w)], [], [(0, 4 * w), (1, 2 * w), (2, 6 * w)], []]
