@@ -1072,30 +1072,45 @@ nbr_walk_kernel(const int32_t *__restrict__ n, const int32_t *__restrict__ run0,
 // the walk waiting for L2.
 // The cuts need lists in target order, as the index build leaves them;
 // order_kernel checks that (and that targets lie in the database), and a call
-// whose lists are not goes to the walk above.  Cutting and checking cost about
-// what a few queries save, so fewer than NB_RANGE_MIN_QUERIES keep that one.
-// Whole search of 1, 3, 4, 6 and 16 queries, walk above and ranges: 20,000
-// sequences 0.47 0.91 1.02 1.26 2.20 and 0.53 0.91 1.01 1.20 1.99 ms; 200,000
-// sequences 1.05 1.49 1.72 2.25 3.87 and 1.20 1.57 1.74 2.11 3.38.
+// whose lists are not goes to the walk above.  So does one whose lists are too
+// short to be cut (nbr_least_postings).
 // 64 queries, 200,000 sequences: 5.3 ms, with 0.2 for the cuts and the check;
 // the walk on the count rows took 11.4 (listed triples, repeats and all).
 constexpr int32_t NB_RANGE = 56 * 1024;   // counters of a block: 224 KB of shared memory
 constexpr int32_t NB_MAX_RANGES = 16;     // 917,504 targets; 25.6 MB of cuts each
 constexpr int NB_RW_THREADS = 1024;
 constexpr int32_t NB_RANGE_MIN_QUERIES = 4;
+
+// Postings an index needs for the cuts to pay in a call of nq queries, against
+// the walk on the count rows: a query reads its lists' cuts range by range (they
+// leave L2 as the ranges become more) and adds the counters to its row, and the
+// cutting and checking are spread over the queries.  Phase A of 300-residue
+// queries, count rows and ranges, ms: 57,000 targets of 120 residues 4 queries
+// 0.29 0.32, 64 2.07 1.80; of 350 0.45 0.41, 3.85 2.23.  460,000 (9 ranges) of
+// 120 0.70 1.16, 7.26 8.54; of 350 1.59 1.93, 17.8 12.6.  900,000 (16) of 120
+// 1.15 2.12, 12.5 15.8; of 350 2.96 3.58, 32.7 23.5.  5,000 of 350 0.24 0.26,
+// 1.51 1.34.  The line below is fitted to 300 such calls (500 to 1,500,000
+// targets, 4 to 64 queries): 0.3 % over the better walk of each, 9 % at most; by
+// ranges from 4 queries on cost 17 % and up to 2.2 times.
+static int64_t nbr_least_postings(double ranges, double targets, double nq) {
+    const double squared = ranges * ranges;
+    return (int64_t)(NB_KMERS * (0.05 * squared + 2e-5 * targets + (1.5 + 2.0 * ranges + 2.5 * squared) / nq));
+}
+
 // postings the walk can number: an octet's end and the step past it stay below 2^32
 constexpr int64_t NB_MAX_POSTINGS = 0xffffff00;
 
 // Whether every list is in target order: the places where a target is below
 // the one before it, over the whole index, less those where a list starts
 // (order[0] - order[1], 0 when all are in order); order[2] counts targets
-// outside the database, and is not zero for an index too long to walk.
+// outside the database, and is not zero for an index too short or too long for
+// the walk by ranges.
 __global__ void order_kernel(const int64_t *__restrict__ kmer_offsets, const int64_t *__restrict__ kmer_entries,
-                             const int32_t *__restrict__ kmer_targets, int32_t n_kmers, int32_t num_db,
+                             const int32_t *__restrict__ kmer_targets, int32_t n_kmers, int32_t num_db, int64_t least,
                              unsigned long long *__restrict__ order) {
     const int64_t total = kmer_offsets[n_kmers], step = (int64_t)gridDim.x * blockDim.x;
     const int64_t me = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (total > NB_MAX_POSTINGS) {  // left to the walk on the count rows
+    if (total < least || total > NB_MAX_POSTINGS) {  // left to the walk on the count rows
         if (me == 0) order[2] = 1;
         return;
     }
@@ -1491,7 +1506,7 @@ static int32_t similar_weights_and_walk(const PhaseAArgs &a, const int8_t *d_sub
     CK_CUDA(cudaGetLastError());
     if (n_ranges > 0) {
         order_kernel<<<sm_count() * 8, 256, 0, a.st>>>(a.kmer_offsets, a.kmer_entries, a.kmer_targets, NB_KMERS,
-                                                       a.num_db, order);
+                                                       a.num_db, nbr_least_postings(n_ranges, a.num_db, a.nq), order);
         CK_CUDA(cudaGetLastError());
         frag_kernel<<<(NB_KMERS + 255) / 256, 256, 0, a.st>>>(a.kmer_offsets, a.kmer_entries, a.kmer_targets,
                                                               a.kmer_freqs, a.freq_thresh, NB_KMERS, range, n_ranges,

@@ -105,3 +105,51 @@ def test_similar_index_of_almost_2_to_32_postings(ck):
     got = [list(zip(t[:n], s[:n])) for t, s, n in zip(out_t.view(nq, -1).tolist(), out_s.view(nq, -1).tolist(),
                                                       out_n.tolist())]
     assert got == [[(0, 2 * w), (1, w), (2, 3 * w)], [], [(0, 4 * w), (1, 2 * w), (2, 6 * w)], []]
+
+
+@pytest.mark.parametrize("n_db,mean,nq,shuffled,compact", [
+    (57344, 100, 64, False, True), (57344, 300, 4, False, True), (57345, 160, 70, False, True),
+    (57345, 160, 64, False, False), (57345, 160, 64, True, True), (120001, 150, 64, False, True),
+    (57345, 160, 3, False, True), (57345, 80, 64, False, True)])
+def test_similar_ranges_of_long_lists(ck, n_db, mean, nq, shuffled, compact):
+    """The walk by target ranges on indexes with enough postings for it: one
+    range that is just full, two, three, more queries than are held at a time;
+    lists out of target order, and calls either side of its rule."""
+    import torch
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.blosum import BLOSUM62
+    from clustkit_gb300.search import DeviceDatabase
+    rng = np.random.default_rng(n_db + nq)
+    lens = rng.integers(mean // 2, mean + mean // 2 + 1, n_db).astype(np.int32)
+    off = (np.cumsum(lens) - lens).astype(np.int64)
+    flat = rng.integers(0, 20, int(lens.sum())).astype(np.uint8)
+    db = DeviceDatabase(flat, off, lens, arena_queries=8, arena_residues=8 * 400)
+    koff, ent, fr = db.index_arrays()
+    ranges = -(-n_db // 57344)
+    enough = (0.05 * ranges ** 2 + 2e-5 * n_db + (1.5 + 2 * ranges + 2.5 * ranges ** 2) / nq) * 20 ** 5
+    assert (int(koff[-1]) >= enough and nq >= 4) == (mean != 80 and nq > 3)
+    if shuffled:  # each list's entries reversed
+        ent = ent[np.repeat(koff[:-1] + koff[1:] - 1, np.diff(koff)) - np.arange(len(ent))]
+    at = rng.integers(0, n_db, nq)
+    qs = [flat[off[i]:off[i] + int(rng.integers(20, 50))].copy() for i in at]
+    qs[0], qs[1] = flat[off[-1]:off[-1] + lens[-1]].copy(), np.zeros(3, np.uint8)
+    sub = np.ascontiguousarray(BLOSUM62, np.int8)
+    qlen = np.array([len(q) for q in qs], np.int32)
+    qoff = (np.cumsum(qlen) - qlen).astype(np.int64)
+    want = oracle.similar_candidates_batch(np.concatenate(qs), qoff, qlen, sub, 13, koff, ent, fr, db.freq_thresh,
+                                           n_db, 2, 300)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_q, d_off, d_len, d_ent = dev(np.concatenate(qs)), dev(qoff), dev(qlen), dev(ent)
+    d_tgt = dev((ent >> 32).astype(np.int32)) if compact else None
+    out_t = torch.zeros(nq * 300, dtype=torch.int32, device="cuda")
+    out_s, out_n = torch.zeros_like(out_t), torch.zeros(nq, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(db.lib.ck_search_phase_a_similar_device(
+        0, d_q.data_ptr(), int(qlen.sum()), d_off.data_ptr(), d_len.data_ptr(), nq, int(qlen.max()), sub.ctypes.data,
+        13, db.d_kmer_offsets.data_ptr(), d_ent.data_ptr(), d_tgt.data_ptr() if compact else None,
+        db.d_kmer_freqs.data_ptr(), db.freq_thresh, n_db, 2, 300, out_t.data_ptr(), out_s.data_ptr(),
+        out_n.data_ptr(), -1, st))
+    _lib.check(db.lib.ck_ctx_status(0, st))
+    t, s, n = out_t.cpu().numpy().reshape(nq, -1), out_s.cpu().numpy().reshape(nq, -1), out_n.cpu().numpy()
+    for q in range(nq):
+        assert np.array_equal(t[q, :n[q]], want[q][0]) and np.array_equal(s[q, :n[q]], want[q][1])
