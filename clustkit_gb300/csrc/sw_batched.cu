@@ -1184,7 +1184,8 @@ static int32_t g_wide_key = 0;
 // every pair runs one warp per pair when a call has at most this many pairs;
 // in larger calls, long pairs do: rows >= max(min rows, the adaptive bound)
 static int32_t g_wave_all_below = 40960;
-static int32_t g_wave_min_rows = 512;
+constexpr int32_t WAVE_MIN_ROWS = 512;
+static int32_t g_wave_min_rows = WAVE_MIN_ROWS;
 static int32_t g_wave_adaptive = 1;
 // warp-per-pair schedule: 1 the shape by what bounds the phase, 2 always the
 // one of calls that run every pair this way, 0 a group's next pair only after
@@ -1428,12 +1429,13 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
         if (wave_only) rows = 8;
         int32_t nt = strip_threads(rows);
         if (wave_only && !g_strip_threads) nt = 512;
-        // the row bound of larger calls: three quarters of the setting above
-        // band 24, where a strip of 16 rows in a group of 8 or more lanes is
-        // worth it from 384 rows on (100,000 pairs of lognormal lengths, bound
-        // 512 and 384: band 16 1.31 and 1.42 ms, 100 4.08 and 4.00, 200 7.00 and
-        // 6.78; 60,000 at band 50 2.25 and 1.69)
-        const int32_t min_rows = in.band_width > 24 ? g_wave_min_rows / 4 * 3 : g_wave_min_rows;
+        // the row bound of larger calls.  Its default, with the adaptive rule,
+        // stands for three quarters of it above band 24, where a strip of 16 rows
+        // in a group of 8 or more lanes is worth it from 384 rows on (100,000 pairs
+        // of lognormal lengths, bound 512 and 384: band 16 1.31 and 1.42 ms, 100
+        // 4.08 and 4.00, 200 7.00 and 6.78; 60,000 at band 50 2.25 and 1.69)
+        const bool by_band = g_wave_adaptive && g_wave_min_rows == WAVE_MIN_ROWS && in.band_width > 24;
+        const int32_t min_rows = by_band ? WAVE_MIN_ROWS / 4 * 3 : g_wave_min_rows;
         const WaveRoute route{in.band_width, g_wave_all_below, min_rows, g_wave_adaptive, 0};
         // profiling events bracket the alignment kernel
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;

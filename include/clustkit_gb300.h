@@ -185,9 +185,11 @@ int32_t ck_sw_last_kernel_ms(float *out_ms);
  *                          skipped pairs) run every pair one warp per pair
  *                          (default 40960)
  *   CK_CFG_WAVE_MIN_ROWS   in larger calls with band_width > 0, pairs with at
- *                          least this many rows (shorter side), or three
- *                          quarters of it at bands above 24, run one warp per
- *                          pair instead of one lane per pair (default 512)
+ *                          least this many rows (shorter side) run one warp
+ *                          per pair instead of one lane per pair; 8192 or
+ *                          more: none (default 512, which with
+ *                          CK_CFG_WAVE_ADAPTIVE stands for 384 at bands
+ *                          above 24)
  *   CK_CFG_WAVE_ADAPTIVE   1 (default): raise that row bound to where a pair's
  *                          one-lane time would pass the call's expected
  *                          kernel time, from the call's cell count; 0:

@@ -189,3 +189,33 @@ def test_components_of_chains_and_stars(ck):
         assert not labels.any() and seconds < 2.4 * random
     _, labels = run(two[rng.permutation(len(two))], 2)
     assert np.array_equal(labels, (np.arange(n) >= n // 2).astype(np.int32))
+
+
+@pytest.mark.parametrize("bw", [16, 50, 128])
+@pytest.mark.parametrize("setting,adaptive,routed", [
+    (450, 0, 450), (450, 1, 450), (512, 0, 512), (3, 0, 3), (8192, 0, None), (8192, 1, None), (9000, 1, None)])
+def test_wave_row_bound_is_taken_as_given(ck, bw, setting, adaptive, routed):
+    """Pairs run one warp per pair from the row bound that was set, at every
+    band; 8192 and more is never."""
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.blosum import BLOSUM62
+    from clustkit_gb300.pairwise import batch_sw
+    rng = np.random.default_rng(setting)
+    rows = np.array([2, 3, 4, 100, 337, 338, 380, 400, 449, 450, 511, 512, 600, 6200, 8000])
+    flat, off, lens = _pack([rng.integers(0, 20, n) for n in rows for _ in range(2)])
+    pairs = np.stack([np.arange(0, len(lens), 2), np.arange(1, len(lens), 2)], 1).astype(np.int32)
+    keys = {_lib.CFG_WAVE_ALL_BELOW: 0, _lib.CFG_WAVE_MIN_ROWS: setting, _lib.CFG_WAVE_ADAPTIVE: adaptive}
+    keep = {k: _lib.get_config(k) for k in keys}
+    try:
+        for k, v in keys.items():
+            _lib.set_config(k, v)
+        got = batch_sw(pairs, flat, off, lens, bw, BLOSUM62, 0.3)
+        wave = _lib.sw_counters()["wave"]
+    finally:
+        for k, v in keep.items():
+            _lib.set_config(k, v)
+    want = oracle.sw_batch(pairs, flat, off, lens, bw, BLOSUM62)
+    assert np.array_equal(got["scores"], want["scores"]) and np.array_equal(got["matches"], want["matches"])
+    # the adaptive rule may raise the bound, here never above the two longest pairs
+    at_least = int((rows >= routed).sum()) if routed else 0
+    assert wave == at_least if not adaptive or not routed else 0 < wave <= at_least
