@@ -34,7 +34,7 @@
 //
 // A batch is hashed, sorted and emitted in one go.  Its pair count is on the
 // host before the emission, so one batch sizes the raw buffer exactly; of
-// several, the first one's count times their number (and a quarter) sizes it,
+// several, the first one's count, in proportion to the tables, and a quarter sizes it,
 // and only a call that outgrows that runs its batches a second time, into a
 // buffer of the counted size.  100,000 sequences, 448 tables of one band: the
 // whole call 24.0 -> 5.5 ms (the old form hashed and sorted all 448
@@ -490,6 +490,20 @@ static int32_t lsh_impl(void *pv) {
         return CK_OK;
     };
 
+    // scratch of the sort and unique that de-duplicate m raw pairs (packed keys
+    // of enough bits for n * n)
+    int bits = 1;
+    while (bits < 64 && ((uint64_t)1 << bits) <= (uint64_t)n * (uint64_t)n) ++bits;
+    auto dedup_bytes = [&](int64_t m, size_t *bytes) -> int32_t {
+        size_t ts = 0, tu = 0;
+        uint64_t *none = nullptr;
+        cub::DoubleBuffer<uint64_t> both(none, none);
+        CK_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, ts, both, m, 0, bits, st));
+        CK_CUDA(cub::DeviceSelect::Unique(nullptr, tu, none, none, (int64_t *)nullptr, m, st));
+        *bytes = std::max(ts, tu);
+        return CK_OK;
+    };
+
     // room for `room` raw pairs, twice over for the de-duplicating sort; a
     // guess that does not fit the device is no error (the counted size may)
     const int32_t n_batches = (T + TB - 1) / TB;
@@ -501,14 +515,22 @@ static int32_t lsh_impl(void *pv) {
         int64_t tot = 0;
         CK_TRY(batch(t0, tb, dv, &tot));
         if (b == 0) {
-            room = n_batches == 1 ? tot : (tot + tot / 4) * n_batches;
-            if (room > 0) rk = (uint64_t *)scratch(SLOT_FALLBACK, (size_t)room * 8 * 2, &status);
+            room = n_batches == 1 ? tot : (int64_t)((double)(tot + tot / 4) * T / TB) + 1;
+            if (room > 0) {
+                // the de-duplicating sort's own scratch first: the guess must leave it that
+                size_t t_dedup = 0;
+                CK_TRY(dedup_bytes(room, &t_dedup));
+                tmp = scratch(SLOT_SORT_TEMP, std::max(t_max, t_dedup), &status);
+                if (tmp) rk = (uint64_t *)scratch(SLOT_FALLBACK, (size_t)room * 8 * 2, &status);
+            }
             if (!rk && room > 0) {
                 if (n_batches == 1) return status;
                 cudaGetLastError();  // the failed allocation: later launches are checked for their own errors
                 reset_thread_status();
                 status = CK_OK;
                 room = 0;
+                tmp = scratch(SLOT_SORT_TEMP, t_max, &status);
+                if (!tmp) return status;
             }
             if (T >= LSH_FILTER_TABLES && room >= LSH_FILTER_PAIRS) {
                 places = (uint64_t)1 << 16;
@@ -545,20 +567,17 @@ static int32_t lsh_impl(void *pv) {
         CK_CUDA(cudaMemcpyAsync(&raw, d_kept, 8, cudaMemcpyDeviceToHost, st));
         CK_CUDA(cudaStreamSynchronize(st));
     }
-    // de-duplicate: sort packed keys (enough bits for n * n), unique
-    int bits = 1;
-    while (bits < 64 && ((uint64_t)1 << bits) <= (uint64_t)n * (uint64_t)n) ++bits;
+    // de-duplicate: sort, unique
     cub::DoubleBuffer<uint64_t> rb(rk, rk + raw);
-    size_t ts = 0, tu = 0;
-    CK_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, ts, rb, raw, 0, bits, st));
-    uint64_t *uq = rb.Alternate();
     int64_t *n_uniq = (int64_t *)(n_runs + 2);
-    CK_CUDA(cub::DeviceSelect::Unique(nullptr, tu, rk, uq, n_uniq, raw, st));
-    void *tmp2 = scratch(SLOT_SORT_TEMP, std::max(ts, tu), &status);
-    if (!tmp2) return status;
-    CK_CUDA(cub::DeviceRadixSort::SortKeys(tmp2, ts, rb, raw, 0, bits, st));
-    size_t tu2 = std::max(ts, tu);
-    CK_CUDA(cub::DeviceSelect::Unique(tmp2, tu2, rb.Current(), rb.Alternate(), n_uniq, raw, st));
+    size_t t_dedup = 0;
+    CK_TRY(dedup_bytes(raw, &t_dedup));
+    tmp = scratch(SLOT_SORT_TEMP, t_dedup, &status);
+    if (!tmp) return status;
+    size_t tbytes = t_dedup;
+    CK_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tbytes, rb, raw, 0, bits, st));
+    tbytes = t_dedup;
+    CK_CUDA(cub::DeviceSelect::Unique(tmp, tbytes, rb.Current(), rb.Alternate(), n_uniq, raw, st));
     int64_t m = 0;
     CK_CUDA(cudaMemcpyAsync(&m, n_uniq, 8, cudaMemcpyDeviceToHost, st));
     CK_CUDA(cudaStreamSynchronize(st));

@@ -219,3 +219,42 @@ def test_wave_row_bound_is_taken_as_given(ck, bw, setting, adaptive, routed):
     # the adaptive rule may raise the bound, here never above the two longest pairs
     at_least = int((rows >= routed).sum()) if routed else 0
     assert wave == at_least if not adaptive or not routed else 0 < wave <= at_least
+
+
+def test_lsh_room_of_a_short_last_batch(ck):
+    """1,000,000 sequences are worked on in batches of 107 tables: for 124 the
+    raw pairs' room follows the tables, not two batches' worth.  In bytes: 40 an
+    item of a batch, the sketches, 16 a raw pair with a quarter and 5 % to spare,
+    the places of pairs seen, and 300 MB for the sorts."""
+    import ctypes
+
+    import torch
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.lsh import band_parameters
+    lib, n, s, tables, values = _lib.load(), 1_000_000, 16, 124, 500
+    per_batch = (4 << 30) // (40 * n)
+    idx, seeds = band_parameters(s, tables * 2, 2, 3)
+    _, first = np.unique(idx, axis=0, return_index=True)
+    idx = np.ascontiguousarray(idx[np.sort(first)[:tables]], np.int32)  # distinct ones
+    seeds = np.ascontiguousarray(seeds[:tables], np.uint64)
+    assert len(idx) == tables and tables // 2 < per_batch < tables
+    sk = torch.randint(0, values, (n, s), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    if torch.cuda.mem_get_info()[0] < 32 << 30:
+        pytest.skip("needs 32 GB of device memory")
+    ctx, count = ctypes.c_int32(), np.zeros(1, np.int64)
+    _lib.check(lib.ck_ctx_create(ctypes.byref(ctx)))
+    try:
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        status = lib.ck_lsh_candidates_device(ctx.value, sk.data_ptr(), n, s, tables, 2, idx.ctypes.data,
+                                              seeds.ctypes.data, None, 0, count.ctypes.data,
+                                              torch.cuda.current_stream().cuda_stream)
+        assert status == _lib.CK_ERR_OUT_OF_MEMORY and count[0] > 0  # no room for the output: counted
+        held = before - torch.cuda.mem_get_info()[0]
+    finally:
+        _lib.check(lib.ck_ctx_destroy(ctx.value))
+    # raw pairs: every table's n(n - 1)/2 comparisons, one in values^2 of which agree in two
+    # different columns, one in values where both bands read one column
+    same = int((idx[:, 0] == idx[:, 1]).sum())
+    raw = n * (n - 1) / 2 * ((tables - same) / values ** 2 + same / values)
+    assert held < 40 * per_batch * n + n * s * 8 + 16 * 1.25 * 1.05 * raw + (64 << 20) + (300 << 20)
