@@ -55,6 +55,7 @@ SIGNATURES = {
     "ck_sw_status_device": (_I32, [_P]),
     "ck_ctx_create": (_I32, [_P]),
     "ck_ctx_destroy": (_I32, [_I32]),
+    "ck_ctx_trim": (_I32, []),
     "ck_ctx_status": (_I32, [_I32, _P]),
     "ck_sw_batch_device_ctx": (_I32, [_I32, _P, _I64, _P, _I64, _P, _P, _I64, _I32, _P, ctypes.c_float, _P,
                                       _I32, _I32, _P, _P, _P, _P, _P, _P]),

@@ -66,11 +66,14 @@ struct DeviceState {
     // caller that makes a context per call (search_batch, search_kmer_index)
     // would otherwise allocate and free some 25 buffers, and clear those kept
     // zero, each time (a 64-query C-path call on 200,000 sequences: 5.3 -> 3.7 ms).  At
-    // most one set of at most PARK_BYTES, freed when it is replaced or when an
-    // allocation of this library fails without it.
+    // most one set, of at most PARK_BYTES and 1 / PARK_SHARE of what the device has
+    // left, since other allocators of the process cannot ask for it; freed when it
+    // is replaced, when an allocation of this library fails without it, and by
+    // ck_ctx_trim.
     ScratchSet *parked = nullptr;
 };
 constexpr size_t PARK_BYTES = (size_t)2 << 30;
+constexpr size_t PARK_SHARE = 8;
 
 std::mutex g_mutex;
 DeviceState g_dev[MAX_DEVICES];
@@ -141,14 +144,20 @@ static void free_set(ScratchSet *set) {
     delete set;
 }
 
+// Frees the current device's parked set; whether there was one.
+static bool unpark() {
+    const int d = current_device();
+    if (d < 0 || d >= MAX_DEVICES || !g_dev[d].parked) return false;
+    free_set(g_dev[d].parked);
+    g_dev[d].parked = nullptr;
+    return true;
+}
+
 // cudaMalloc, once more without the parked set when it fails for memory.
 static cudaError_t malloc_or_unpark(void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
-    const int d = current_device();
-    if (e == cudaErrorMemoryAllocation && d >= 0 && d < MAX_DEVICES && g_dev[d].parked) {
+    if (e == cudaErrorMemoryAllocation && unpark()) {
         cudaGetLastError();
-        free_set(g_dev[d].parked);
-        g_dev[d].parked = nullptr;
         e = cudaMalloc(p, bytes);
     }
     return e;
@@ -550,15 +559,23 @@ int32_t ck_ctx_destroy(int32_t handle) {
     set->pending = set->frozen = false;
     size_t held = 0;
     for (int i = 0; i < SLOT_COUNT; ++i) held += set->cap[i];
-    ScratchSet *&parked = g_dev[set->device].parked;
-    if (held <= PARK_BYTES && cudaMemset(set->err, 0, 64) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess) {
-        if (parked) free_set(parked);
-        parked = set;
+    size_t left = 0, total = 0;
+    if (held <= PARK_BYTES && cudaMemGetInfo(&left, &total) == cudaSuccess && held <= left / PARK_SHARE &&
+        cudaMemset(set->err, 0, 64) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess) {
+        unpark();
+        g_dev[set->device].parked = set;
     } else {
         free_set(set);
     }
     cudaSetDevice(prev);
     g_ctx[handle - 1] = nullptr;
+    return CK_OK;
+}
+
+int32_t ck_ctx_trim(void) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    t_status = CK_OK;
+    unpark();
     return CK_OK;
 }
 

@@ -168,3 +168,34 @@ def test_kept_zero_buffer_that_grows_in_place(rt, handed_on):
             assert rt.ck_ctx_destroy(ctx) == 0
             ctx = _create(rt)
     assert len(set(places)) == 1  # it did come back where it was
+
+
+def test_kept_scratch_is_given_back(rt):
+    """A destroyed context's scratch is kept for the next one only while it is a
+    small part of the memory left, and is freed by ck_ctx_trim, by the next set
+    kept, and when an allocation fails without it."""
+    MB = 1 << 20
+    base, ctx = rt.t_in_use(), _create(rt)  # the device's own words stay allocated
+    one = rt.t_in_use()
+    base += 0 if base else one - 256  # (made by the first call)
+    p, _ = _scratch(rt, ctx, 0, 4 * MB)
+    assert rt.ck_ctx_destroy(ctx) == 0 and rt.t_in_use() >= base + 4 * MB  # kept
+    ctx = _create(rt)
+    assert _scratch(rt, ctx, 0, 3 * MB)[0] == p  # handed on
+    assert rt.ck_ctx_destroy(ctx) == 0
+    assert rt.ck_ctx_trim() == 0 and rt.t_in_use() == base
+    assert rt.ck_ctx_trim() == 0 and rt.t_in_use() == base
+
+    # 4 MB of scratch with less than 32 MB left is freed at once
+    other = rt.t_malloc(30 * MB)
+    ctx = _create(rt)
+    _scratch(rt, ctx, 0, 4 * MB)
+    assert rt.ck_ctx_destroy(ctx) == 0 and rt.t_in_use() == base + 30 * MB
+    rt.t_free(other)
+
+    # kept, and in the way of the library's own next allocation
+    ctx, second = _create(rt), _create(rt)
+    _scratch(rt, ctx, 0, 4 * MB)
+    assert rt.ck_ctx_destroy(ctx) == 0 and rt.t_in_use() >= base + 4 * MB
+    assert _scratch(rt, second, 0, 62 * MB)[0]
+    assert rt.ck_ctx_destroy(second) == 0 and rt.t_in_use() == base
