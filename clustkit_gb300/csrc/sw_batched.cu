@@ -48,6 +48,7 @@
 #include <cstring>
 
 #include "ck_common.cuh"
+#include "sw_schedule.cuh"
 
 namespace ck {
 
@@ -103,9 +104,6 @@ struct KeyCompact {
 // warps at 96 or 80 registers) for 8-row strips, 256 (8 warps, up to 255
 // registers) for 24 or 32 rows.  One CTA per SM holds one increment table,
 // so the warps a CTA adds cost no table copy.
-// per warp, the streamed warp-per-pair phase's pair slots in shared memory
-constexpr size_t WAVE_SLOT_BYTES = 72;  // sizeof(WaveSlot), checked where it is defined
-constexpr int WAVE_SLOTS_PER_WARP = 16;
 
 // a * one + b with `one` a runtime 1: issued as an integer multiply-add on
 // the FMA pipe, which the recurrence leaves mostly idle, instead of an add on
@@ -761,10 +759,9 @@ __device__ void align_pair_strips(const SwIn &in, const SwOut &out, int64_t p, c
 // increment table + the warp-per-pair slots, for a CTA of NT threads
 template <int NT>
 __host__ __device__ constexpr size_t strip_smem() {
-    return INC_SMEM + (size_t)(NT / 32) * WAVE_SLOTS_PER_WARP * WAVE_SLOT_BYTES;
+    return INC_SMEM + (size_t)(NT / 32) * WS_SLOTS * sizeof(WaveSlot);
 }
 
-struct WaveSlot;
 // Shapes of the warp-per-pair phase, chosen in the kernel (wave_shapes).
 struct WaveShapes {
     int32_t all, tail, few;  // R << 8 | G
@@ -808,8 +805,8 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order, const ui
     const int32_t n_wave = s_wave, max_rows = (int32_t)(sorted_keys[0] >> 13);
     if (n_wave > 0) {
         char *slot_base = (char *)(s_inc + INC_ENTRIES * 32);  // behind the increment table
-        WaveSlot *slots = (WaveSlot *)(slot_base + (size_t)(threadIdx.x >> 5) * WAVE_SLOTS_PER_WARP *
-                                                       WAVE_SLOT_BYTES);
+        WaveSlot *slots = (WaveSlot *)(slot_base + (size_t)(threadIdx.x >> 5) * WS_SLOTS *
+                                                       sizeof(WaveSlot));
         // the shape by what bounds the phase (wave_shapes)
         const int32_t n_warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
         const bool few = n_wave <= n_warps;
@@ -880,35 +877,6 @@ sw_strip_kernel(SwIn in, SwOut out, const uint32_t *__restrict__ order, const ui
 // a strip a lane holds its best cell in registers: on a trigger, each column's
 // lowest row with its best score replaces it when it scores more, or as much
 // in a lower row (a later column of the same row does not).
-constexpr int WS_SLOTS = WAVE_SLOTS_PER_WARP;
-constexpr int WS_U = 2;  // columns a step
-
-struct WaveSlot {
-    unsigned long long acc;   // score << 27 | (16383 - row) << 13 | matches
-    int64_t a_off, b_off;     // residues of the row and column sequences
-    int64_t p;                // pair index
-    int32_t la, lb, w, h, c0, S, m00, T0;
-    int32_t gs;               // running best score of the pair (first-maximum trigger)
-    int32_t live;
-};
-
-static_assert(sizeof(WaveSlot) == WAVE_SLOT_BYTES, "slot layout");
-
-// steps at which strip s starts (its first column's block) and ends (its last's)
-template <int R>
-__device__ __forceinline__ int32_t strip_t0(const WaveSlot &sl, int32_t s) {
-    const int32_t lo = s * R + sl.c0;
-    return sl.T0 + s + ((lo > 1 ? lo : 1) - sl.c0) / WS_U - sl.m00;
-}
-template <int R>
-__device__ __forceinline__ int32_t strip_te(const WaveSlot &sl, int32_t s) {
-    const int32_t hi = s * R + sl.c0 + R - 1 + 2 * sl.w;
-    const int32_t J1 = hi < sl.lb ? hi : sl.lb;
-    const int32_t te = sl.T0 + s + (J1 - sl.c0) / WS_U - sl.m00;
-    const int32_t t0 = strip_t0<R>(sl, s);
-    return te > t0 ? te : t0;  // a strip whose band lies left of column 1 ends where it starts
-}
-
 template <int R, int G, class K>
 __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *order, int32_t n_wave, int32_t pack,
                             int32_t serial, int32_t *ticket, const char *s_inc, WaveSlot *warp_slots, int32_t lane,
@@ -965,26 +933,16 @@ __device__ void wave_stream(const SwIn &in, const SwOut &out, const uint32_t *or
             } else {
                 const int64_t p = (int64_t)order[q];
                 const PairGeom g = pair_geometry(in, p, err);
-                int32_t n_strips = (g.la + R - 1) / R;
-                {
-                    const int64_t lim = (int64_t)g.lb - 1 - g.h + g.w;
-                    const int64_t s_lim = lim < 0 ? 0 : lim / R + 1;
-                    if (s_lim < n_strips) n_strips = (int32_t)s_lim;
-                }
+                const int32_t n_strips = wave_strips(R, g.la, g.lb, g.w, g.h);
                 if (n_strips <= 0) {
                     if (gl == 0) write_result(out, in, p, 0, 0, g.la, g.la, g.lb);
                 } else {
                     WaveSlot &sl = slots[seq % SLOTS];
                     const int32_t c0 = 1 + g.h - g.w;
-                    const int32_t m00 = ((c0 > 1 ? c0 : 1) - c0) / U;
+                    const int32_t m00 = wave_block(R, c0, 0);
                     const int32_t m = (gl - g_next) & (G - 1);
                     const int32_t first = n_strips < G ? n_strips : G;
-                    int32_t req = T;
-                    if (m < first) {
-                        const int32_t lom = m * R + c0;
-                        const int32_t r = F + 1 - m - (((lom > 1 ? lom : 1) - c0) / U - m00);
-                        req = r > T ? r : T;
-                    }
+                    const int32_t req = m < first ? wave_earliest(R, c0, m00, m, F, T) : T;
                     const int32_t T0p = __reduce_max_sync(gmask, req);
                     if (gl == 0) {
                         sl.acc = 0;
@@ -1194,22 +1152,6 @@ static int32_t g_wave_stream = 1;
 // rows per strip of the warp-per-pair schedule: 0 = by shape, else at least
 // that many (4, 8 or 16)
 static int32_t g_wave_rows = 0;
-
-// The smallest group that strips of R rows can rotate through in a band of
-// half-width w.  A lane may start its next strip, G strips on, once its last is
-// done: that one's last column is R - 1 + 2w after its first row's first, the
-// other's first at least G R after it and G steps later, so
-// 2w <= (G - 1)(R + U) + 1 is enough (clipping at the matrix only shortens the
-// first).  Pairs of at most G strips never rotate: those with a longer side of
-// at most 50, whose band is the whole matrix, have at most 7 strips of 8 rows;
-// and where the band is too wide for 32 lanes of 16 rows, every pair has at most
-// 512 rows (wave_split), 32 strips.  0: none.
-static int32_t wave_group(int32_t R, int32_t w) {
-    if (w >= 1)
-        for (int32_t G = 8; G <= 32; G <<= 1)
-            if (2 * (int64_t)w <= (G - 1) * (R + WS_U) + 1) return G;
-    return R == 16 ? 32 : 0;
-}
 
 // The shapes of a call with band half-width w.  16 rows, for the cells a step's
 // own cost is spread over (8 where 8 lanes of them rotate: at narrow bands a

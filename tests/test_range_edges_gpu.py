@@ -258,3 +258,41 @@ def test_lsh_room_of_a_short_last_batch(ck):
     same = int((idx[:, 0] == idx[:, 1]).sum())
     raw = n * (n - 1) / 2 * ((tables - same) / values ** 2 + same / values)
     assert held < 40 * per_batch * n + n * s * 8 + 16 * 1.25 * 1.05 * raw + (64 << 20) + (300 << 20)
+
+
+@pytest.mark.parametrize("bw", [35, 36, 63, 64, 75, 76, 135, 136, 155, 156, 263])
+@pytest.mark.parametrize("hinted,long_rows", [(False, 0), (True, 0), (False, 2100), (True, 2100)])
+def test_wave_groups_at_their_band_limits(ck, bw, hinted, long_rows):
+    """The bands where strips of 8 and of 16 rows take the next larger group of
+    lanes (where a lane's next strip starts right after its last one), in calls
+    of more pairs than the kernel has warps; with a pair of more than 2,047 rows
+    the default schedule takes strips of 8 rows in each of these groups."""
+    from clustkit_gb300 import _lib
+    from clustkit_gb300.blosum import BLOSUM62
+    from clustkit_gb300.pairwise import batch_sw
+    rng = np.random.default_rng(2 * bw + long_rows + hinted)
+    lens = [1, 7, 8, 9, 16, 17, 50, 51, 52, 64, 65, 127, 128, 129, 255, 256, 257, 400, 512, 513, 700]
+    if long_rows:
+        lens += [long_rows, long_rows + 37]
+    base = rng.integers(0, 20, max(lens) + 40)
+    seqs = []
+    for n in lens:
+        for v in range(3):  # related, shifted and unrelated
+            x = base[7 * v: 7 * v + n].copy() if v < 2 else rng.integers(0, 20, n)
+            x[rng.random(n) < 0.2] = rng.integers(0, 20)
+            seqs.append(x)
+    flat, off, length = _pack(seqs)
+    pairs = rng.integers(0, len(seqs), (2900, 2)).astype(np.int32)
+    pairs = np.concatenate([pairs, np.stack([np.arange(len(seqs) - 1), np.arange(1, len(seqs))], 1).astype(np.int32)])
+    hints = rng.integers(-120, 121, len(pairs)).astype(np.int32) if hinted else None
+    want = oracle.sw_batch(pairs, flat, off, length, bw, BLOSUM62, diag_hints=hints)
+    keep = _lib.get_config(_lib.CFG_WAVE_STREAM)
+    try:
+        for stream in (1, 2, 0):
+            _lib.set_config(_lib.CFG_WAVE_STREAM, stream)
+            got = batch_sw(pairs, flat, off, length, bw, BLOSUM62, 0.3, diag_hints=hints)
+            for k in ("scores", "matches", "shorter", "sims"):
+                assert np.array_equal(got[k], want[k]), (k, stream)
+            assert _lib.sw_counters()["wave"] > 2432  # more than 16 warps on each of 152 SMs
+    finally:
+        _lib.set_config(_lib.CFG_WAVE_STREAM, keep)
