@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -262,7 +263,13 @@ static int32_t with_context(int32_t handle, F fn) {
         return CK_ERR_INVALID_ARGUMENT;
     }
     t_set = set;
-    const int32_t st = fn();
+    int32_t st;
+    try {
+        st = fn();
+    } catch (const std::exception &e) {  // host containers; the callers are C
+        st = CK_ERR_OUT_OF_MEMORY;
+        set_error(st, std::string("host memory: ") + e.what());
+    }
     t_set = nullptr;
     return st;
 }

@@ -74,6 +74,7 @@ void t_free(void *p) { cudaFree(p); }
 """
 
 REST = r"""
+#include <new>
 #include "ck_common.cuh"
 namespace ck {
 int32_t sw_plain_launch(const SwIn &, const SwOut &, int64_t, const int32_t *, const int32_t *, int32_t *, cudaStream_t, SwCounters *) { return 0; }
@@ -99,7 +100,9 @@ static int32_t ask(void *pv) {
     a.p = (char *)(a.zeroed ? ck::scratch_zeroed(a.slot, a.bytes, nullptr, &status) : ck::scratch(a.slot, a.bytes, &status));
     return status;
 }
+static int32_t no_memory(void *) { throw std::bad_alloc(); }
 extern "C" {
+int32_t t_no_memory(int32_t ctx) { return ck::run_in_context(ctx, no_memory, nullptr); }
 // The buffer of a context's slot, or null; *nonzero the bytes of it that are not zero.
 void *t_scratch(int32_t ctx, int32_t slot, int64_t bytes, int32_t zeroed, int64_t *nonzero) {
     Ask a{slot, (size_t)bytes, zeroed != 0, nullptr};
@@ -199,3 +202,15 @@ def test_kept_scratch_is_given_back(rt):
     assert rt.ck_ctx_destroy(ctx) == 0 and rt.t_in_use() >= base + 4 * MB
     assert _scratch(rt, second, 0, 62 * MB)[0]
     assert rt.ck_ctx_destroy(second) == 0 and rt.t_in_use() == base
+
+
+def test_host_allocation_that_fails_is_a_status(rt):
+    """An exception of a host container ends as a status of the call, whose
+    context is no longer the thread's."""
+    ctx = _create(rt)
+    p, _ = _scratch(rt, ctx, 0, 1000)
+    assert rt.t_no_memory(ctx) == 4  # CK_ERR_OUT_OF_MEMORY
+    rt.ck_last_error.restype = ctypes.c_char_p
+    assert b"host memory" in rt.ck_last_error()
+    assert _scratch(rt, 0, 0, 1000)[0] != p  # the default context's own
+    assert _scratch(rt, ctx, 0, 1000)[0] == p
