@@ -375,7 +375,7 @@ static int32_t read_and_clear_error(cudaStream_t st) {
         return CK_ERR_CAPACITY;
     }
     if (h & ERRBIT_LIST) {
-        set_error(CK_ERR_CAPACITY, "similar k-mer neighbour list beyond the caller's list_capacity (truncated)");
+        set_error(CK_ERR_CAPACITY, "similar k-mers: more (query position, 5-mer) pairs than the caller's list_capacity");
         return CK_ERR_CAPACITY;
     }
     if (h & ERRBIT_SCHEDULE) {

@@ -33,7 +33,7 @@ enum : int32_t {
     ERRBIT_SEQ_EXTENT = 2,     // offsets[i] + lengths[i] outside [0, flat_len]
     ERRBIT_SCHEDULE = 4,       // a streamed warp-per-pair strip missed its start step (internal)
     ERRBIT_CAPACITY = 8,       // a device-side count passed the caller's bound (Phase-B bins)
-    ERRBIT_LIST = 16,          // the similar-k-mer neighbour list passed the caller's bound
+    ERRBIT_LIST = 16,          // the similar-k-mer (position, 5-mer) pairs passed the caller's bound
 };
 
 // ---------------------------------------------------------------- SW constants
