@@ -125,7 +125,7 @@ template <int NPL>
 constexpr int select_warps() { return NPL <= 16 ? 8 : 48 * 1024 / (32 * NPL * 8); }
 // resident blocks: registers for as many as the buffers leave room for (NPL >= 32), or without spills
 template <int NPL>
-constexpr int select_blocks() { return NPL >= 16 ? 4 : NPL == 8 ? 5 : 6; }
+constexpr int select_blocks() { return NPL >= 16 ? 4 : 6; }
 
 template <int NPL, class V>
 __global__ void __launch_bounds__(32 * select_warps<NPL>(), select_blocks<NPL>())
