@@ -58,6 +58,7 @@ void free_db(ScratchSet *set) {
 struct DeviceState {
     bool init = false;
     int sms = 0;
+    size_t memory = 0;  // bytes of the device
     cudaStream_t stream = nullptr;
     ScratchSet def;
     int8_t *sub = nullptr;
@@ -68,13 +69,14 @@ struct DeviceState {
     // would otherwise allocate and free some 25 buffers, and clear those kept
     // zero, each time (a 64-query C-path call on 200,000 sequences: 5.3 -> 3.7 ms).  At
     // most one set, of at most PARK_BYTES and 1 / PARK_SHARE of what the device has
-    // left, since other allocators of the process cannot ask for it; freed when it
-    // is replaced, when an allocation of this library fails without it, and by
-    // ck_ctx_trim.
+    // left, since other allocators of the process cannot ask for it (asking costs 10
+    // to 30 us, so a set of 1 / PARK_FREELY of the device is kept without); freed
+    // when it is replaced, when an allocation of this library fails without it, and
+    // by ck_ctx_trim.
     ScratchSet *parked = nullptr;
 };
 constexpr size_t PARK_BYTES = (size_t)2 << 30;
-constexpr size_t PARK_SHARE = 8;
+constexpr size_t PARK_SHARE = 8, PARK_FREELY = 2048;
 
 std::mutex g_mutex;
 DeviceState g_dev[MAX_DEVICES];
@@ -102,6 +104,7 @@ DeviceState *state(int32_t *status) {
         e = cudaGetDeviceProperties(&prop, d);
         if (e != cudaSuccess) { *status = cuda_status(e, "cudaGetDeviceProperties"); return nullptr; }
         s.sms = prop.multiProcessorCount;
+        s.memory = prop.totalGlobalMem;
         e = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) { *status = cuda_status(e, "cudaStreamCreate"); return nullptr; }
         s.def.device = d;
@@ -567,7 +570,9 @@ int32_t ck_ctx_destroy(int32_t handle) {
     size_t held = 0;
     for (int i = 0; i < SLOT_COUNT; ++i) held += set->cap[i];
     size_t left = 0, total = 0;
-    if (held <= PARK_BYTES && cudaMemGetInfo(&left, &total) == cudaSuccess && held <= left / PARK_SHARE &&
+    const bool small = held <= g_dev[set->device].memory / PARK_FREELY;
+    if (held <= PARK_BYTES &&
+        (small || (cudaMemGetInfo(&left, &total) == cudaSuccess && held <= left / PARK_SHARE)) &&
         cudaMemset(set->err, 0, 64) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess) {
         unpark();
         g_dev[set->device].parked = set;

@@ -263,10 +263,10 @@ int32_t ck_jaccard_device(const int32_t *d_pairs, int64_t M, const uint64_t *d_s
  * bound to the device current at creation. */
 int32_t ck_ctx_create(int32_t *out_handle);
 /* Waits for the device, then ends the context.  Its scratch (one set a device,
- * up to 2 GiB and an eighth of the memory the device has left) is kept for the
- * next ck_ctx_create on the device and freed when another replaces it, when the
- * library runs out of device memory, or by ck_ctx_trim; the database of
- * ck_ctx_upload_db is freed at once. */
+ * up to 2 GiB and an eighth of the memory the device has left, or 1/2048 of its
+ * memory whatever is left) is kept for the next ck_ctx_create on the device and
+ * freed when another replaces it, when the library runs out of device memory,
+ * or by ck_ctx_trim; the database of ck_ctx_upload_db is freed at once. */
 int32_t ck_ctx_destroy(int32_t handle);
 /* Frees the scratch of the last destroyed context, if the current device still
  * keeps one. */
