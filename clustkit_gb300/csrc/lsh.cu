@@ -169,7 +169,7 @@ __global__ void lsh_emit_runs_kernel(const uint32_t *__restrict__ order, const i
 // LSH_BIG_PARTS); a bucket's members are dealt out over its blocks' warps, whose
 // lanes split each member's pairs with the members before it.  (A warp a
 // bucket left the largest, half a million pairs, to one warp: 1.08 ms of the
-// call on 100,000 sequences, now 0.11.)
+// call on 100,000 sequences, now 0.15.)
 constexpr int LSH_BIG_PARTS = 16;
 __global__ void lsh_emit_big_kernel(const uint32_t *__restrict__ order, const int32_t *__restrict__ run_start,
                                     const int64_t *__restrict__ pair_off, const int32_t *__restrict__ n_runs,
@@ -204,10 +204,17 @@ __global__ void lsh_emit_big_kernel(const uint32_t *__restrict__ order, const in
 // 100,000 sequences, 124 distinct tables: of 25.5 M raw pairs 6.5 M are written
 // (4.6 M are distinct), and sorting them takes 0.32 ms instead of 1.17.
 //
-// Used from 12 distinct tables and 4 M raw pairs on.  Whole call without and
-// with: 22 M pairs of 124 tables 5.83 -> 5.14 ms, 32 M of 199 4.19 -> 3.18,
-// 11 M of 448 7.48 -> 7.18, 5.4 M of 15 1.98 -> 1.87; but 1.6 M of 8 1.40 ->
-// 1.44, 1.8 M of 30 1.16 -> 1.20, 0.4 M of 124 3.76 -> 3.80.
+// Used from 12 distinct tables and 4 M raw pairs on: the sort of the repeats has
+// to cost more than looking every pair up, and how many there are is not known
+// before.  Whole call without and with, ms:
+//   pairs that most tables find: 22 M raw of 124 tables 5.83 5.14, 32 M of 199
+//     4.19 3.18, 11 M of 448 7.48 7.18; families of ten, 20 tables 0.78 0.75, 40
+//     1.23 1.00; the same buckets in every table, 72 M of 16 3.50 1.44, 40 M of
+//     12 2.01 1.36 (and 27 M of 8 1.43 1.21, 7 M of 2 0.57 0.64)
+//   pairs that few find: 300,000 in families, 12 tables 1.00 1.08, 40 2.40 2.47;
+//     unlike tables, 71 M of 16 3.61 4.32, 171 M of 40 8.56 10.25 (36 M of 8 1.93
+//     2.34)
+//   fewer than 4 M: 1.6 M of 8 1.40 1.44, 1.8 M of 30 1.16 1.20
 constexpr int32_t LSH_FILTER_TABLES = 12;
 constexpr int64_t LSH_FILTER_PAIRS = (int64_t)1 << 22;
 constexpr int LSH_AHEAD = 4, LSH_QUEUE = 256, LSH_FILTER_THREADS = 256, LSH_FILTER_PARTS = 32;

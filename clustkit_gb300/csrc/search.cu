@@ -1077,7 +1077,10 @@ nbr_walk_kernel(const int32_t *__restrict__ n, const int32_t *__restrict__ run0,
 // 64 queries, 200,000 sequences: 5.3 ms, with 0.2 for the cuts and the check;
 // the walk on the count rows took 11.4 (listed triples, repeats and all).
 constexpr int32_t NB_RANGE = 56 * 1024;   // counters of a block: 224 KB of shared memory
-constexpr int32_t NB_MAX_RANGES = 16;     // 917,504 targets; 25.6 MB of cuts each
+// 917,504 targets, 25.6 MB of cuts each.  Past it (1,500,000 targets, 27 ranges)
+// 64 queries take 53.2 ms on the count rows and would 39.7 by ranges at 350
+// residues a target, 19.7 and 27.2 at 120; 4 queries 4.5 and 6.3, 1.7 and 3.7
+constexpr int32_t NB_MAX_RANGES = 16;
 constexpr int NB_RW_THREADS = 1024;
 constexpr int32_t NB_RANGE_MIN_QUERIES = 4;
 

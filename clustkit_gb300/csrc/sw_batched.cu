@@ -1372,10 +1372,11 @@ int32_t sw_batched_launch(const SwIn &in, const SwOut &out, int64_t M, const int
         int32_t nt = strip_threads(rows);
         if (wave_only && !g_strip_threads) nt = 512;
         // the row bound of larger calls.  Its default, with the adaptive rule,
-        // stands for three quarters of it above band 24, where a strip of 16 rows
-        // in a group of 8 or more lanes is worth it from 384 rows on (100,000 pairs
-        // of lognormal lengths, bound 512 and 384: band 16 1.31 and 1.42 ms, 100
-        // 4.08 and 4.00, 200 7.00 and 6.78; 60,000 at band 50 2.25 and 1.69)
+        // stands for three quarters of it above band 24: 70 calls of 41,000 to
+        // 400,000 pairs at bands 26 to 200, time at 512 over time at 384: lognormal
+        // lengths 1.04 (0.91 to 1.39), Pareto 1.11 (0.93 to 1.39); it loses where
+        // medians are above 250 and bands below 128.  At bands 12 to 24 (60,000 and
+        // 100,000 pairs) 384 rows are 5 to 14 % slower
         const bool by_band = g_wave_adaptive && g_wave_min_rows == WAVE_MIN_ROWS && in.band_width > 24;
         const int32_t min_rows = by_band ? WAVE_MIN_ROWS / 4 * 3 : g_wave_min_rows;
         const WaveRoute route{in.band_width, g_wave_all_below, min_rows, g_wave_adaptive, 0};
