@@ -230,12 +230,6 @@ void *scratch_zeroed(int slot, size_t bytes, cudaStream_t st, int32_t *status) {
     return p;
 }
 
-size_t scratch_capacity(int slot) {
-    int32_t status = CK_OK;
-    ScratchSet *s = current_set(&status);
-    return s ? s->cap[slot] : 0;
-}
-
 void scratch_mark_dirty(int slot) {
     int32_t status = CK_OK;
     ScratchSet *s = current_set(&status);

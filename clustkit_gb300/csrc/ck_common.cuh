@@ -194,7 +194,6 @@ void reset_thread_status();
 // Per-device scratch: grow-only buffers owned by the library.
 void *scratch(int slot, size_t bytes, int32_t *status);
 void *scratch_zeroed(int slot, size_t bytes, cudaStream_t st, int32_t *status);
-size_t scratch_capacity(int slot);  // bytes the slot holds now (0 when unallocated)
 void scratch_mark_dirty(int slot);
 void scratch_clear_dirty(int slot);
 int32_t *device_error_word(int32_t *status);
