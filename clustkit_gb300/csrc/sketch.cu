@@ -116,7 +116,7 @@ __device__ __forceinline__ uint64_t kmer_value(const uint8_t *p, int32_t k, V al
 // number in 32 bits: a compare-exchange is then one instruction a key, not
 // the five or six that 64-bit keys take), and the few neighbours whose leading
 // bits agree are put right in shared memory.
-// 200,000 sequences (median 300 residues), k = 5, s = 128: 3.62 -> 0.46 ms
+// 200,000 sequences (median 300 residues), k = 5, s = 128: 3.62 -> 0.45 ms
 // (sketch_kernel, sorting 64-bit keys in shared memory, before).  5,000 of 2,000
 // residues: random ones 54 us, repeats of 4 with 2 % changed 106 (sketch_kernel
 // 279 and 227; by moving the threshold 54 and 2,117).
